@@ -131,7 +131,7 @@ ft_rotation_plan * make_rotation_plan(int kind, int n, double alpha, double beta
     for (long long i = 0; i < len; i++) sc[i] = make_double2(RP->s[i], RP->c[i]);
     if (!cuda_ok(cudaMalloc(&RP->d_sc, sizeof(double2) * len), "cudaMalloc(table)") ||
         !cuda_ok(cudaMemcpy(RP->d_sc, sc.data(), sizeof(double2) * len, cudaMemcpyHostToDevice), "cudaMemcpy(table)") ||
-        !cuda_ok(cudaMalloc(&RP->d_counter, sizeof(int)), "cudaMalloc(counter)") || !rotation_plan_pad(RP)) {
+        !cuda_ok(cudaMalloc(&RP->d_counter, sizeof(int)), "cudaMalloc(counter)") || !rotation_plan_skew(RP)) {
         ft_destroy_rotation_plan(RP);
         return nullptr;
     }
@@ -186,7 +186,7 @@ bool rotations(ft_rotation_plan * RP, bool hi2lo, const double * in, double * ou
     if (ntasks == 0) return true;
     static thread_local RotLaunch L;   // large parameter block; kept off the stack
     L.nfields = 1;
-    L.fields[0] = RotField{in, out, RP->d_scp, RP->n, M, RP->kind, lda, 0};
+    L.fields[0] = RotField{in, out, RP->d_skew, RP->n, M, RP->kind, lda, 0};
     L.tasks = d_tasks;
     L.ntasks = ntasks;
     L.counter = cs ? cs->counter : RP->d_counter;
@@ -739,7 +739,7 @@ int execute_batch_chunk(HarmonicPlan * const * H, bool forward, char TRANS, doub
         for (int f = 0; f < nf; f++) {
             const double * in = from_A ? A[f] : S[f];
             double * out = to_A ? A[f] : S[f];
-            L.fields[f] = RotField{in, out, H[f]->rp_arr[0]->d_scp, N[f], M[f], H[f]->kind, (long long) N[f], blk};
+            L.fields[f] = RotField{in, out, H[f]->rp_arr[0]->d_skew, N[f], M[f], H[f]->kind, (long long) N[f], blk};
             if (in != out) {
                 const int nc = untouched_cols(H[f]->kind, M[f]);
                 if (!cuda_ok(cudaMemcpy2DAsync(out, N[f] * sizeof(double), in, N[f] * sizeof(double), N[f] * sizeof(double), nc,
@@ -1151,7 +1151,7 @@ void ft_destroy_rotation_plan(ft_rotation_plan * RP) {
     }
     delete RP->mu;
     if (RP->d_sc) cudaFree(RP->d_sc);
-    if (RP->d_scp) cudaFree(RP->d_scp);
+    if (RP->d_skew) cudaFree(RP->d_skew);
     if (RP->d_counter) cudaFree(RP->d_counter);
     std::free(RP->s);
     std::free(RP->c);

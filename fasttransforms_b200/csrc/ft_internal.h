@@ -62,23 +62,39 @@ struct Geo {
     __host__ __device__ static inline long long table_len(int kind, int N) {
         return kind == DISK ? (long long) N * N : (long long) N * (N + 1) / 2;
     }
-    // Padded copy of the table, read by the rotation kernel's bulk copies: an identity row of
-    // kIdLen pairs (sin 0, cos 1), then every column j of the packed table with kPadPos chain
-    // positions of identity pairs on each side, then another identity row.  Inside a column,
-    // entry l is the packed entry where the sweep has a rotation (0 <= l / CH <= top(j, l % CH)),
-    // the identity elsewhere, so a chunk of consecutive positions that overlaps the sweep's
-    // entries can be copied without a range check (kPadPos >= the chunk length E); a chunk
-    // entirely outside them is copied from an identity row.
-    static constexpr int kPadPos = 16;
-    static constexpr int kIdLen = 64;
     __host__ __device__ static inline int table_cols(int kind, int N) { return kind == DISK ? 2 * N - 1 : N; }
-    __host__ __device__ static inline long long pad_side(int kind) { return (long long) kPadPos * chains(kind); }
-    // offset of entry l = 0 of column j in the padded table
-    __host__ __device__ static inline long long padded_col(int kind, int N, int j) {
-        return kIdLen + table_base(kind, N, j) + (2LL * j + 1) * pad_side(kind);
+    // Skewed copy of the table, read by the rotation kernel.  Per parity p of the sweeps (tri: one),
+    // block beta holds the kSkewRows sweeps j = p + step (kSkewRows beta + i), i = 0 .. kSkewRows - 1,
+    // cut into chunks as the kernel's wavefront meets them: row i of chunk kappa holds the pairs of
+    // positions kSkewLen kappa - 2 - 2 i .. + kSkewLen - 1 (every chain of a position in turn), the
+    // identity (sin 0, cos 1) where the sweep has no rotation.  The rows of a chunk lie one after
+    // the other, and so do a block's chunks, so what a stage needs of one chunk is one bulk copy.
+    // The tops fall by one per sweep, so a block has one chunk fewer than the block before; one
+    // chunk of identities follows each block's last (a copy of two chunks may start on the last).
+    static constexpr int kSkewRows = 8, kSkewLen = 8;
+    __host__ __device__ static inline int skew_parities(int kind) { return kind == TRI ? 1 : 2; }
+    __host__ __device__ static inline long long skew_chunk(int kind) { return (long long) kSkewRows * kSkewLen * chains(kind); }
+    // blocks of parity p (the sweeps with a rotation)
+    __host__ __device__ static inline int skew_blocks(int kind, int N, int p) {
+        const int t = top(kind, N, p, 0);
+        return t < 0 ? 0 : t / kSkewRows + 1;
     }
-    __host__ __device__ static inline long long padded_len(int kind, int N) {
-        return 2LL * kIdLen + table_len(kind, N) + 2LL * table_cols(kind, N) * pad_side(kind);
+    // chunks of block beta with a rotation
+    __host__ __device__ static inline int skew_chunks(int kind, int N, int p, int beta) {
+        return (top(kind, N, p, 0) + kSkewRows + 1) / kSkewLen + 1 - beta;
+    }
+    // the block's first chunk, counted from the parity's first
+    __host__ __device__ static inline long long skew_first(int kind, int N, int p, int beta) {
+        return (long long) beta * (skew_chunks(kind, N, p, 0) + 1) - (long long) beta * (beta - 1) / 2;
+    }
+    // offset (in pairs) of chunk 0 of block beta of parity p
+    __host__ __device__ static inline long long skew_at(int kind, int N, int p, int beta) {
+        const long long before = p ? skew_first(kind, N, 0, skew_blocks(kind, N, 0)) : 0;
+        return (before + skew_first(kind, N, p, beta)) * skew_chunk(kind);
+    }
+    __host__ __device__ static inline long long skew_len(int kind, int N) {
+        const int p = skew_parities(kind) - 1;
+        return skew_at(kind, N, p, skew_blocks(kind, N, p));
     }
     // number of order columns the rotation stage visits for an N x M matrix
     // sph / disk: pairs (2m-1, 2m), m = 2 .. M/2; tri: column m, m = 1 .. M-1
@@ -90,10 +106,11 @@ struct Geo {
     // jhi applies to at least one of its columns (order m runs j = jpar .. m - step; with
     // blk > 0 only its sweeps above its last whole block of blk sweeps).  Returns their number
     // (0: nothing to do).  The kernel and the host's pass schedule both use this.
+    // orders: those of the group (0: task_orders(kind)).
     // SPIN: order m runs the sph sweeps of order |m - spin|, j = (m + spin) mod 2 .. |m - spin| - 2.
     __host__ __device__ static inline int task_sweeps(int kind, int M, int mbase, int blk, int * jlo_out, int * jhi_out,
-                                                      int spin = 0) {
-        const int st = step(kind), ord = task_orders(kind), mlast = last_order(kind, M);
+                                                      int spin = 0, int orders = 0) {
+        const int st = step(kind), ord = orders > 0 ? orders : task_orders(kind), mlast = last_order(kind, M);
         int omax = mbase + st * (ord - 1);
         if (omax > mlast) omax = mbase + st * ((mlast - mbase) / st);
         if (kind == SPIN) {
@@ -129,13 +146,14 @@ struct Geo {
 struct RotTask {
     int field;   // index into the field table of the launch
     int mbase;   // lowest order of the group
+    int side;    // spin: 0 the columns of orders -m (2m - 1), 1 those of orders m (2m); else unused
 };
 
 // One coefficient matrix of a launch.
 struct RotField {
     const double * in;      // first pass reads here
     double * out;           // every pass writes here (in == out allowed)
-    const double2 * sc;     // the padded (sin, cos) table of the field's rotation plan (Geo::padded_col)
+    const double2 * sc;     // the skewed (sin, cos) table of the field's rotation plan (Geo::skew_at)
     int N, M, kind;
     long long lda;
     int blk;                // 0: all sweeps; > 0: only each column's sweeps above the last
@@ -179,8 +197,8 @@ cudaError_t launch_rotations(int kind, bool hi2lo, const RotLaunch & L, int max_
                              double * const * dead = nullptr, RotSchedule * sched = nullptr,
                              int * prog_call = nullptr, int prog_cap = 0);
 void set_rotation_config(int cfg);   // 0 .. 3 forces a configuration, -1 chooses per shape
-// (Re)builds RP->d_scp from RP->d_sc (call after every change of d_sc; synchronous)
-bool rotation_plan_pad(ft_rotation_plan * RP);
+// (Re)builds RP->d_skew from RP->d_sc (call after every change of d_sc; synchronous)
+bool rotation_plan_skew(ft_rotation_plan * RP);
 
 // Triangular multiplies (trmm.cu).  Out = op(U) * In on column classes.
 struct TrmmClass {
@@ -333,7 +351,7 @@ struct ft_rotation_plan_s {
     double alpha, beta, gamma;
     int device;
     double2 * d_sc;            // interleaved table
-    double2 * d_scp;           // the same, padded for the rotation kernel's bulk copies (Geo::padded_col)
+    double2 * d_skew;          // the same, skewed for the rotation kernel (Geo::skew_at)
     int * d_counter;           // work counter for the persistent kernel
     std::mutex * mu;
     std::map<int, std::pair<ftb::RotTask *, int>> * tasks;   // M -> device task list (longest first)

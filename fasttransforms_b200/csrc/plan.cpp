@@ -429,11 +429,11 @@ std::vector<RotTask> build_tasks(int kind, int N, int M, int field) {
     const int mfirst = Geo::first_order(kind), mlast = Geo::last_order(kind, M);
     const int span = Geo::step(kind) * Geo::task_orders(kind);
     if (kind == TRI) {
-        for (int m = mfirst; m <= mlast; m += span) t.push_back({field, m});
+        for (int m = mfirst; m <= mlast; m += span) t.push_back({field, m, 0});
     } else {
         for (int p = 0; p < 2; p++) {
             const int m0 = p == 0 ? 2 : 3;
-            for (int m = m0; m <= mlast; m += span) t.push_back({field, m});
+            for (int m = m0; m <= mlast; m += span) t.push_back({field, m, 0});
         }
     }
     return t;

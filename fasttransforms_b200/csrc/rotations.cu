@@ -4,41 +4,45 @@
 //   lo2hi: x' = fma(c, x, -(s*y)), y' = fma(c, y, s*x)
 // (src/rotations/rotations_AVX512F.c:4-15; x is row k, y is row k+d).
 //
-// Work decomposition
-// ------------------
-// A task is a group of columns that receive the same sweeps (sph: 16 orders
-// of one parity, cos and sin column each; disk: 32 orders of one parity, cos
-// and sin each; tri: 32 consecutive orders).  Orders in a group differ, so a sweep j is applied to the columns
-// whose order m satisfies j <= m - STEP and is an exact no-op (sin 0, cos 1)
-// for the others.  Tasks are pulled from a longest-first queue by persistent
-// CTAs (one per SM), which balances the triangular cost over orders.
+// Two kernels apply them, each element meeting its rotations in the same order, so that every launch
+// shape gives the same bits.
 //
-// Inside a CTA the sweeps of a task run as a wavefront.  Warp q (a "stage")
-// owns B consecutive sweeps.  Each lane owns one chain of the columns of one
-// order and keeps, per column, a window of 2B consecutive chain positions in
-// registers.  At every step the
-// window slides by one position: one element enters, B independent rotations
-// are applied (sweep b at window slots 2b, 2b+1), one element leaves.  The
-// element leaving stage q is the element entering stage q+1 at the same step,
-// passed through a shared-memory ring buffer.  All W warps share the global
-// traffic: during each iteration every warp loads its share of the next
-// chunk's column segments into registers (latency hidden behind the sweeps)
-// and writes its share of the last stage's finished chunk back, so one pass of
-// W*B sweeps reads and writes each column once.  The lanes of a warp that carry
-// the same chain use the same (sin, cos) pair at each rotation, read as a
-// broadcast 16-byte shared-memory load (two pairs per warp for two-chain kinds);
-// each sweep's pairs of a chunk arrive in shared memory by one bulk copy from a
-// padded table (identity pairs outside the sweep), issued one chunk ahead.
-// With W = 8 warps every SM sub-partition holds two warps and the register
-// budget per thread is the full 255.  In the pipelined configurations each pass
-// of a task is a work unit of its own that streams behind the previous pass.
+// rot_kernel: columns streamed from global memory
+// -----------------------------------------------
+// A task is a group of columns that receive the same sweeps (sph: 16 orders of one parity, cos and
+// sin column each; disk: 32 orders of one parity, cos and sin each; tri: 32 consecutive orders).
+// Orders in a group differ, so a sweep j is applied to the columns whose order m satisfies
+// j <= m - STEP and is an exact no-op (sin 0, cos 1) for the others.  Tasks, or single passes of
+// W x B sweeps of a task (the pass pipeline), are pulled from a queue by persistent CTAs.
 //
-// Within a CTA no thread waits on another except through __syncthreads.  The
-// one spin loop is the pass pipeline's wait on another CTA's progress word
-// (pipelined configurations only), bounded, after which the launch records a
-// device status and every later wait gives up.  Every global access is
-// bounds-checked against the field's N, M.
+// Inside a CTA the sweeps of a pass run as a wavefront.  Warp q (a "stage") owns B consecutive
+// sweeps.  Each lane owns one chain of the columns of one order and keeps, per column, a window of
+// 2B consecutive chain positions in registers.  At every step the window slides by one position:
+// one element enters, B independent rotations are applied (sweep b at window slots 2b, 2b+1), one
+// element leaves, into a ring in shared memory that the next stage reads.  A loading warp copies
+// chunks of E positions from global memory into the first ring (cp.async), a storing warp writes
+// the last ring back, so one pass reads and writes each column once.  The lanes that carry the same
+// chain use the same (sin, cos) pair at each rotation, read as a broadcast 16-byte shared-memory
+// load; a stage's pairs of a chunk are contiguous in a skewed copy of the table (Geo::skew_at) and
+// arrive by one bulk copy a few chunks ahead.
+//
+// Warps meet only through mbarriers per ring slot, and every warp goes on to the next pass or queue
+// entry by itself: the stages never drain between passes.  What bounds the kernel: the FP64 pipe
+// (4 instructions a rotation, 2 cycles each on a sub-partition; the inner step alone, without
+// global traffic, reaches 80 % of it) and, next, instruction fetch.  The unrolled steps are 21 KB
+// of code (16 steps of 8 sweeps on 2 columns), which the stages run at different places at the
+// same time: with unrolled loading and storing loops beside them (register staging, about 50 KB in
+// all) the instruction cache missed and the launch took 10.8 ms at sph degree 4095; with the
+// compact loops 8.5 ms (9.8 ms for the former kernel, whose stages met at a barrier per chunk).
+//
+// rot_resident_kernel: columns resident in shared memory
+// ------------------------------------------------------
+// For chains that fit; see there.
+//
+// Every wait is bounded, after which the launch records a device status and every later wait gives
+// up at once.  Every global access is bounds-checked against the field's N, M.
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
@@ -59,33 +63,27 @@ struct KT {
     static constexpr int CH = (KIND == SPH || KIND == SPIN || KIND == RECT) ? 2 : 1;   // chains per column
     static constexpr int STEP = KIND == TRI ? 1 : 2;      // order step between sweeps
     // sequences per order sharing the rotations: cos, sin columns (sph, disk), the column
-    // (tri, rect), or the real and imaginary parts of the columns of -m and m (spin)
-    static constexpr int NCOL = (KIND == TRI || KIND == RECT) ? 1 : (KIND == SPIN ? 4 : 2);
+    // (tri, rect), or the real and imaginary parts of the column of -m or of m (spin)
+    static constexpr int NCOL = (KIND == TRI || KIND == RECT) ? 1 : 2;
     static constexpr int ES = KIND == SPIN ? 2 : 1;       // doubles per element (interleaved complex)
     static constexpr int ORD = 32 / CH;                   // orders per task (one lane per order and chain)
-    static constexpr int COLS = ORD * NCOL;               // columns per task
+    static constexpr int COLS = ORD * NCOL;               // sequences per task
     static constexpr int CPAD = COLS + 1;                 // padded column dimension of the stage buffers
 };
 
-// Builds the padded table (Geo::padded_col): block j fills column j's padded segment, blocks
-// >= cols the identity rows at both ends.
-__global__ void pad_table_kernel(const double2 * __restrict__ sc, double2 * __restrict__ out, int kind, int N) {
-    const int cols = Geo::table_cols(kind, N), ch = Geo::chains(kind);
-    const long long side = Geo::pad_side(kind);
-    const double2 id = make_double2(0.0, 1.0);
-    const int j = blockIdx.x;
-    if (j >= cols) {   // the identity row before column 0, and the one after the last column
-        double2 * row = j == cols ? out : out + Geo::padded_col(kind, N, cols - 1) + (Geo::table_base(kind, N, cols) -
-                                                                                     Geo::table_base(kind, N, cols - 1)) + side;
-        for (int e = threadIdx.x; e < Geo::kIdLen; e += blockDim.x) row[e] = id;
-        return;
-    }
-    const long long len = Geo::table_base(kind, N, j + 1) - Geo::table_base(kind, N, j);
-    const long long base = Geo::table_base(kind, N, j);
-    double2 * col = out + Geo::padded_col(kind, N, j);
-    for (long long l = -side + threadIdx.x; l < len + side; l += blockDim.x) {
-        const bool valid = l >= 0 && l < len && (int) (l / ch) <= Geo::top(kind, N, j, (int) (l % ch));
-        col[l] = valid ? sc[base + l] : id;
+// Builds the skewed table (Geo::skew_at): CTA (beta, p) fills block beta of parity p.
+__global__ void skew_table_kernel(const double2 * __restrict__ sc, double2 * __restrict__ out, int kind, int N) {
+    const int beta = blockIdx.x, p = blockIdx.y, ch = Geo::chains(kind);
+    if (beta >= Geo::skew_blocks(kind, N, p)) return;
+    double2 * const block = out + Geo::skew_at(kind, N, p, beta);
+    const int row_len = Geo::kSkewLen * ch, chunk = Geo::kSkewRows * row_len;
+    const int total = (Geo::skew_chunks(kind, N, p, beta) + 1) * chunk;
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int kappa = e / chunk, i = (e % chunk) / row_len, jj = e % row_len;
+        const int j = p + Geo::step(kind) * (Geo::kSkewRows * beta + i);
+        const int pos = Geo::kSkewLen * kappa - 2 - 2 * i + jj / ch, c = jj % ch;
+        const bool rotates = j < Geo::table_cols(kind, N) && pos >= 0 && pos <= Geo::top(kind, N, j, c);
+        block[e] = rotates ? sc[Geo::table_base(kind, N, j) + ch * pos + c] : make_double2(0.0, 1.0);
     }
 }
 
@@ -102,17 +100,17 @@ __device__ __forceinline__ void rot_lo2hi(double & x, double & y, double s, doub
     x = xn; y = yn;
 }
 
-// Status word of the rotation kernel: nonzero once a wait of the pass pipeline ran out
-// (its output is then not valid).  Read and cleared by rotation_device_error().
+// Status word of the rotation kernel: nonzero once a bounded wait ran out (the output is then not
+// valid).  Read and cleared by rotation_device_error().
 __device__ int g_rot_status;
 
-// Progress word of a pipeline unit: hi2lo, -X where every position >= X of its columns is
-// final for the pass; lo2hi, X where every position <= X is final.  The launcher clears the
-// words to a value below any position; a finished unit publishes INT_MAX.  Thread 0 publishes
-// after a CTA barrier: the barrier orders every thread's stores of the chunk before its release,
-// and a release is cumulative, so one thread's release covers the whole CTA's stores (the
-// consumer's thread 0 acquires, then a barrier orders its CTA's loads after that).  A release
-// reduction (max: the words only rise) does not hold the thread the way a fence does.
+// Progress of a pass over its columns: hi2lo, -X where every position >= X is final for the pass;
+// lo2hi, X where every position <= X is final.  A finished pass publishes INT_MAX.
+//
+// Pipelined launches keep one word per pass in global memory (cleared by the launcher to a value
+// below any position).  The storing warp publishes after a __syncwarp: that orders all its lanes'
+// stores before lane 0's release, and a release is cumulative.  A release reduction (max: the
+// words only rise) does not hold the thread the way a fence does.
 __device__ __forceinline__ void publish_progress(int * p, int v) {
     asm volatile("red.release.gpu.global.max.s32 [%0], %1;\n" :: "l"(p), "r"(v) : "memory");
 }
@@ -127,448 +125,803 @@ __device__ __forceinline__ int wait_progress(const int * p, int need) {
         if (v >= need) return v;
         if (*(volatile int *) &g_rot_status != 0) return v;
         if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
-        __nanosleep(128);
+        __nanosleep(32);
+    }
+}
+// Whole-task launches run a task's passes one after another in one CTA, whose loading warps wait
+// for its own storing warp: one 64-bit word in shared memory holds (pass counter of the CTA,
+// progress + 2^31), which only rises.
+__device__ __forceinline__ unsigned long long local_word(unsigned seq, int v) {
+    return ((unsigned long long) seq << 32) | (unsigned) (v ^ 0x80000000);
+}
+__device__ __forceinline__ void publish_local(unsigned long long * p, unsigned long long w) {
+    asm volatile("st.release.cta.shared::cta.u64 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned long long v;
+        asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];\n" : "=l"(v) : "r"(tc::smem_addr(p)) : "memory");
+        if (v >= need) return v;
+        if (*(volatile int *) &g_rot_status != 0) return v;
+        if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
+        __nanosleep(32);
+    }
+}
+// Bounded mbarrier wait: a wait that runs out sets the status word, after which every wait of
+// the launch returns at once and the kernel runs to its end on whatever the buffers hold.
+// (The slow path is a call: the kernel's warps run different code at the same time, and what they
+// run between them has to stay small to be served from the instruction cache.)
+__device__ __noinline__ void wait_bar_slow(uint64_t * bar, uint32_t parity) {
+    if (!tc::mbar_wait(bar, parity, (volatile int *) &g_rot_status)) atomicCAS(&g_rot_status, 0, 5);
+}
+__device__ __forceinline__ void wait_bar(uint64_t * bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok) : "r"(tc::smem_addr(bar)), "r"(parity) : "memory");
+    if (!ok) wait_bar_slow(bar, parity);
+}
+
+// Asynchronous 8-byte copy global -> shared (0 bytes read, zeros written when !valid), and the
+// arrival of this thread on a barrier once its copies so far have landed.
+__device__ __forceinline__ void copy_async8(double * dst, const double * src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(tc::smem_addr(dst)), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async_arrive(uint64_t * bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" :: "r"(tc::smem_addr(bar)) : "memory");
+}
+
+// Geometry of one pass of W x B sweeps of a task, the same for every warp of the CTA.  The
+// sweeps are numbered i = (j - parity) / STEP; a pass holds i0 .. i0 + W B - 1 (the last one
+// fewer), aligned with the task's lowest sweep, so that the B sweeps of a stage are rows of one
+// block of the skewed table.  The pass moves positions 0 .. emax of every chain as a stream of
+// nchunk chunks of E positions (hi2lo: from the top down, lo2hi: from the bottom up); chunk k
+// covers positions pmin(k) .. pmin(k) + E - 1, those outside 0 .. emax read as zero and are not
+// written.  The chunks are aligned so that the pairs of a stage's chunk are whole chunks of the
+// skewed table.
+template <int KIND, bool HI2LO, int W, int B, int E>
+struct Pass {
+    int i0, stages;   // lowest sweep, stages with a sweep
+    int emax, nchunk;
+    __host__ __device__ __forceinline__ Pass(int N, int nsw, int npass, int jpar, int jlo, int r, bool copy_all) {
+        const int at = HI2LO ? npass - 1 - r : r;
+        const int left = nsw - at * W * B;
+        i0 = (jlo - jpar) / KT<KIND>::STEP + at * W * B;
+        stages = (left >= W * B ? W * B : left) / B + ((left < W * B && left % B) ? 1 : 0);
+        const int top = Geo::top(KIND, N, jpar + KT<KIND>::STEP * i0, 0), last = Geo::chain_len(KIND, N, 0) - 1;
+        emax = top + 1;
+        if (copy_all || emax > last) emax = last;
+        if (emax < 0) emax = 0;
+        nchunk = HI2LO ? emax / E + 1 : (emax + 1) / E + 1;
+    }
+    __host__ __device__ __forceinline__ int pmin(int k) const { return HI2LO ? (nchunk - 1 - k) * E : k * E - 1; }
+    // lowest sweep of stage q
+    __host__ __device__ __forceinline__ int stage_sweep(int q) const { return i0 + (HI2LO ? stages - 1 - q : q) * B; }
+    // chunk of the skewed table (in units of E positions) that a stage meets at its chunk k
+    __host__ __device__ __forceinline__ int kappa(int k) const { return HI2LO ? nchunk - 1 + 2 * B / E - k : k; }
+};
+
+// A task's sweeps and passes.
+template <int KIND, int W, int B>
+struct TaskGeo {
+    int N, M, mbase, mlast, jpar, nsw, jlo, jhi, npass;
+    __host__ __device__ __forceinline__ TaskGeo(const RotField & F, const RotTask & t) {
+        N = F.N; M = F.M; mbase = t.mbase;
+        mlast = Geo::last_order(KIND, M);
+        // lowest sweep of every column (spin: the parity of the effective orders |m - s|)
+        jpar = KIND == TRI ? 0 : (KIND == SPIN ? ((mbase + F.spin) & 1) : (mbase & 1));
+        nsw = Geo::task_sweeps(KIND, M, mbase, F.blk, &jlo, &jhi, F.spin);
+        npass = (nsw + W * B - 1) / (W * B);
+    }
+};
+
+// The elements of one chunk as a warp moves them between global memory and a ring slot: element v
+// of a lane is double rr(v) of the contiguous E * CH * ES doubles of column segment seg(v).
+template <int KIND, bool HI2LO, int E>
+struct Mover {
+    using T = KT<KIND>;
+    static constexpr int RPC = E * T::CH * T::ES;                  // doubles of a segment
+    static constexpr int SEGS = T::COLS / T::ES;                   // segments (columns) of a task
+    static constexpr int PER = T::COLS * E * T::CH / 32;           // elements of a lane
+    static constexpr int RB = RPC >= 32 ? RPC / 32 : 1;            // instructions per segment
+    static constexpr int SP = RPC >= 32 ? 1 : 32 / RPC;            // segments per instruction
+    static_assert(RPC % 32 == 0 || 32 % RPC == 0, "a segment must split evenly over the lanes");
+    long long base;     // double offset of this lane's element 0 at chain position 0
+    long long lda2;     // doubles between columns
+    int nseg;           // valid segments of the task, less this lane's own
+    int seg0;           // first valid one, less this lane's own (spin: order 0 has one column)
+    int N, lane;
+    __host__ __device__ __forceinline__ static int lane_seg(int lane) { return RPC < 32 ? lane / RPC : 0; }
+    __host__ __device__ __forceinline__ static int rr(int v, int lane) { return RPC >= 32 ? (v % RB) * 32 + lane : lane % RPC; }
+    // columns from segment s's column to the task's first column
+    __host__ __device__ __forceinline__ static constexpr int col_of(int s) {
+        return KIND == TRI ? s : KIND == RECT ? 2 * s : KIND == SPIN ? 4 * s : 4 * (s >> 1) + (s & 1);
+    }
+    __host__ __device__ __forceinline__ Mover(const RotField & F, const RotTask & t, int mlast, int lane_) : lane(lane_) {
+        N = F.N;
+        lda2 = (long long) T::ES * F.lda;
+        const int orders = t.mbase > mlast ? 0 : min(T::ORD, (mlast - t.mbase) / T::STEP + 1);
+        const int ls = lane_seg(lane);
+        nseg = orders * (SEGS / T::ORD) - ls;
+        seg0 = 0;
+        long long col0;
+        if (KIND == TRI || KIND == RECT) col0 = t.mbase;
+        else if (KIND == SPIN) {
+            col0 = 2LL * t.mbase - (t.side ? 0 : 1);    // side 0: order -m in column 2m - 1; 1: order m in 2m
+            if (col0 < 0) seg0 = 1 - ls;
+            // the matrix may end before the last order's column
+            const long long most = (F.M - 1 - col0) / 4 + 1;
+            if (nseg + ls > most) nseg = (int) most - ls;
+        } else col0 = 2LL * t.mbase - 1;
+        // SP > 1 with paired columns: a lane's segments differ from its first by whole orders
+        base = (col0 + col_of(ls)) * lda2;
+    }
+    __host__ __device__ __forceinline__ bool seg_ok(int v) const { const int s = (v / RB) * SP; return s < nseg && s >= seg0; }
+    __host__ __device__ __forceinline__ bool row_ok(int v, int pmin, int emax) const {
+        const int r = rr(v, lane), p = pmin + r / (T::ES * T::CH);
+        return p >= 0 && p <= emax && T::CH * p + (r / T::ES) % T::CH < N;
+    }
+    // double offset of element v of the chunk that starts at position pmin
+    __host__ __device__ __forceinline__ long long at(int v, int pmin) const {
+        return base + (long long) col_of((v / RB) * SP) * lda2 + (long long) T::ES * T::CH * pmin + rr(v, lane);
+    }
+    // its place in a ring slot
+    __host__ __device__ __forceinline__ int slot_at(int v) const {
+        const int r = rr(v, lane), pos = r / (T::ES * T::CH), c = (r / T::ES) % T::CH, part = r % T::ES;
+        const int u = HI2LO ? E - 1 - pos : pos;
+        return (u * T::CH + c) * T::CPAD + ((v / RB) * SP + lane_seg(lane)) * T::ES + part;
+    }
+};
+
+// E steps of a stage.  The window is circular: at step u, window position x lives in register
+// slot (u - x) mod 2B.  The element leaving (position 2B - 1 of the previous step) sits in slot
+// u mod 2B, which the entering element (position 0) takes over.  OFF: step number of the chunk's
+// first step mod 2B.
+template <int KIND, bool HI2LO, int B, int E, int OFF>
+__device__ __forceinline__ void stage_steps(double (&win)[KT<KIND>::NCOL][2 * B], const double * bin, double * bout,
+                                            bool has_out, const double2 * const (&sc)[B]) {
+    using T = KT<KIND>;
+    constexpr int W2 = 2 * B;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int u = OFF + e, pn = u % W2;
+#pragma unroll
+        for (int h = 0; h < T::NCOL; ++h) {
+            const double in = bin[e * T::CH * T::CPAD + h];
+            if (has_out) bout[e * T::CH * T::CPAD + h] = win[h][pn];
+            win[h][pn] = in;
+        }
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            constexpr int RL = Geo::kSkewLen * T::CH;
+            const int pos = HI2LO ? E - 1 - e : e;
+            const double2 p = sc[b][(pos / Geo::kSkewLen) * Geo::kSkewRows * RL + (pos % Geo::kSkewLen) * T::CH];
+            const int xl = (u - 2 * b + 2 * W2) % W2;       // window position 2b
+            const int xu = (u - 2 * b - 1 + 2 * W2) % W2;   // window position 2b+1
+#pragma unroll
+            for (int h = 0; h < T::NCOL; ++h) {
+                if (HI2LO) rot_hi2lo(win[h][xl], win[h][xu], p.x, p.y);
+                else       rot_lo2hi(win[h][xu], win[h][xl], p.x, p.y);
+            }
+        }
+    }
+}
+// The same without rotations: every element leaves the stage as it entered.
+template <int KIND, int B, int E, int OFF>
+__device__ __forceinline__ void shift_steps(double (&win)[KT<KIND>::NCOL][2 * B], const double * bin, double * bout, bool has_out) {
+    using T = KT<KIND>;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int pn = (OFF + e) % (2 * B);
+#pragma unroll
+        for (int h = 0; h < T::NCOL; ++h) {
+            const double in = bin[e * T::CH * T::CPAD + h];
+            if (has_out) bout[e * T::CH * T::CPAD + h] = win[h][pn];
+            win[h][pn] = in;
+        }
     }
 }
 
-// Lane layout: lane = o * CH + c owns chain c of the NCOL columns of order
-// mbase + STEP * o (sph: cos and sin columns 2m-1, 2m; disk: the same pair;
-// tri: column m; spin: the real and imaginary parts of the complex columns of
-// orders -m and m, which share the sph sweeps of order |m - s|).  The NCOL columns
-// of a lane share every (sin, cos) pair, so one shared-memory load feeds NCOL
-// rotations.
-template <int KIND, bool HI2LO, int W, int B, int E>
-__global__ void __launch_bounds__(W * 32, W <= 4 ? 2 : 1)
+// Progress of a warp of the resident kernel, in shared memory (it only rises).
+__device__ __forceinline__ void publish_word(int * p, int v) {
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "r"(v) : "memory");
+}
+__device__ __noinline__ int wait_word_slow(const int * p, int need) {
+    const long long t0 = clock64();
+    for (;;) {
+        int v;
+        asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
+        if (v >= need || *(volatile int *) &g_rot_status != 0) return v;
+        if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
+    }
+}
+__device__ __forceinline__ int wait_word(const int * p, int need) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
+    return v >= need ? v : wait_word_slow(p, need);
+}
+
+// E steps of one sequence of the resident kernel (stage_steps with the columns in place); ROTATE
+// false: the window only shifts.
+template <bool HI2LO, int CH, int B, int E, int OFF, int ROW, bool ROTATE>
+__device__ __forceinline__ void resident_steps(double (&win)[2 * B], const double * bin, double * bout, bool has_in, bool has_out,
+                                               const double2 * const (&sc)[B]) {
+    constexpr int W2 = 2 * B;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int u = OFF + e, pn = u % W2, at = HI2LO ? -e * ROW : e * ROW;
+        const double in = has_in ? bin[at] : 0.0;
+        if (has_out) bout[at] = win[pn];
+        win[pn] = in;
+        if (ROTATE) {
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const double2 p = sc[b][(HI2LO ? E - 1 - e : e) * CH];
+                const int xl = (u - 2 * b + 2 * W2) % W2, xu = (u - 2 * b - 1 + 2 * W2) % W2;
+                if (HI2LO) rot_hi2lo(win[xl], win[xu], p.x, p.y);
+                else       rot_lo2hi(win[xu], win[xl], p.x, p.y);
+            }
+        }
+    }
+}
+
+// Compile-time layout of a launch shape.
+template <int KIND, int W, int B, int E>
+struct Shape {
+    using T = KT<KIND>;
+    static constexpr int D = 2 * B / E;                  // chunks an element spends in a stage's window
+    static constexpr int SL = 2;                         // slots of a ring
+    static constexpr int SCS = E >= 16 ? 2 : 3;          // staged (sin, cos) chunks of a stage
+    static constexpr int NL = 1;                         // loading warps
+    static constexpr int WARPS = W + NL + 1;
+    static constexpr int SLOT = E * T::CH * T::CPAD;     // doubles of a ring slot
+    static constexpr int SCLEN = B * E * T::CH;          // pairs of a stage's chunk
+    static constexpr int IDLEN = (E / Geo::kSkewLen - 1) * Geo::kSkewRows * Geo::kSkewLen * T::CH + Geo::kSkewLen * T::CH;   // a row's span in one
+    static constexpr int UR = 4;                         // queue entries in flight in a CTA
+    static constexpr size_t doubles = (size_t) (W + 1) * SL * SLOT + SLOT;
+    static constexpr size_t pairs = (size_t) W * SCS * SCLEN + IDLEN;
+    static constexpr size_t bytes = (doubles * sizeof(double) + 15) / 16 * 16 + pairs * sizeof(double2);
+    static_assert(D >= 1 && D * E == 2 * B, "a window must hold whole chunks");
+    static_assert(E % Geo::kSkewLen == 0, "a chunk must be whole chunks of the skewed table");
+    static_assert(B == Geo::kSkewRows || (Geo::kSkewRows % B == 0 && E == Geo::kSkewLen && 2 * B % E == 0),
+                  "a stage's rows must lie one after the other in the skewed table");
+};
+
+template <int KIND, bool HI2LO, int W, int B, int E, int MINB>
+__global__ void __launch_bounds__(Shape<KIND, W, B, E>::WARPS * 32, MINB)
 rot_kernel(const __grid_constant__ RotLaunch L) {
     using T = KT<KIND>;
-    constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, ORD = T::ORD, COLS = T::COLS, CPAD = T::CPAD, ES = T::ES;
-    constexpr int WB = W * B;
-    static_assert(E % (2 * B) == 0, "chunk must be a multiple of the window");
-    static_assert((B * E * CH) % 32 == 0, "a chunk's (sin, cos) entries must split evenly over the lanes");
-    extern __shared__ double smem[];
-    // buffer q (0..W): input of stage q (q = W: output of the last stage), 2 slots,
-    // element (step u, chain c, task column cl)
-    auto buf = [&](int q, int slot, int u, int c) -> double * {
-        return smem + ((((q * 2 + slot) * E + u) * CH + c) * CPAD);
-    };
-    // (sin, cos) pairs of the chunk a stage works on, staged one iteration ahead
-    double2 * const sc_stage_base = reinterpret_cast<double2 *>(smem + (W + 1) * 2 * E * CH * CPAD);
-    auto sc_stage = [&](int q, int slot) -> double2 * { return sc_stage_base + ((q * 2 + slot) * B) * (E * CH); };
-    static_assert(E <= Geo::kPadPos, "the padded table must cover a chunk's overhang");
-    static_assert(E * CH <= Geo::kIdLen, "the identity row must cover a chunk");
-    __shared__ int s_task;
-    __shared__ __align__(8) uint64_t s_mbar[W * 2];   // per stage and slot: its (sin, cos) staged
+    using SH = Shape<KIND, W, B, E>;
+    using MV = Mover<KIND, HI2LO, E>;
+    constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, D = SH::D, SL = SH::SL, SCS = SH::SCS, NL = SH::NL, SLOT = SH::SLOT,
+                  SCLEN = SH::SCLEN, UR = SH::UR;
+    extern __shared__ __align__(16) double smem[];
+    double * const rings = smem;                                  // ring q: input of stage q; ring W: output of the last stage
+    double * const zeros = smem + (size_t) (W + 1) * SL * SLOT;   // what a stage reads past the stream's end
+    double2 * const pairs = reinterpret_cast<double2 *>(reinterpret_cast<unsigned char *>(smem) + (SH::doubles * sizeof(double) + 15) / 16 * 16);
+    double2 * const ident = pairs + (size_t) W * SCS * SCLEN; // identity pairs, for sweeps a lane's order does not have
+    __shared__ __align__(8) uint64_t full[(W + 1) * SL], empt[(W + 1) * SL], scbar[W * SCS], ufull[UR], uempt[UR];
+    __shared__ unsigned long long s_local;
+    __shared__ int s_unit[UR];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = warp;                       // stage index
-    const int o_lane = lane / CH, c_lane = lane % CH;
+    for (int i = threadIdx.x; i < SLOT; i += blockDim.x) zeros[i] = 0.0;
+    for (int i = threadIdx.x; i < SH::IDLEN; i += blockDim.x) ident[i] = make_double2(0.0, 1.0);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < W * 2; ++i) tc::mbar_init(&s_mbar[i], 1);
+        for (int i = 0; i < (W + 1) * SL; ++i) { tc::mbar_init(&full[i], i < SL ? 32 : 1); tc::mbar_init(&empt[i], 1); }
+        for (int i = 0; i < W * SCS; ++i) tc::mbar_init(&scbar[i], 1);
+        for (int i = 0; i < UR; ++i) { tc::mbar_init(&ufull[i], 1); tc::mbar_init(&uempt[i], SH::WARPS - 1); }
+        s_local = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    uint32_t sc_phase = 0u;                   // bit s: parity of the next phase of this stage's mbarrier s
-    uint32_t sc_live = 0u;                    // bit s: the chunk staged for slot s has a rotation (warp-uniform)
 
     const bool pipe = L.chains != nullptr;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = atomicAdd(L.counter, 1);
-        __syncthreads();
-        const int tid = s_task;
-        __syncthreads();
-        if (tid >= (pipe ? L.nchains : L.ntasks)) break;
-        // passes first, first + stride, .. of a task (pipeline), or all of its passes
-        const RotChain chain = pipe ? L.chains[tid] : RotChain{tid, 0, 0, 1};
-        const RotTask task = L.tasks[chain.task];
-        const RotField & F = L.fields[task.field];
-        const int N = F.N;
-        const long long lda = F.lda;
-        const int mlast = Geo::last_order(KIND, F.M);
-        const int mbase = task.mbase;
-        // lowest sweep of every column (spin: the parity of the effective orders |m - s|)
-        const int jpar = KIND == TRI ? 0 : (KIND == SPIN ? ((mbase + F.spin) & 1) : (mbase & 1));
-        // With F.blk > 0 a column of order m runs only its sweeps j >= jcut(m): the
-        // (m - jpar)/STEP mod blk sweeps above its last whole block of blk sweeps.
-        auto jcut = [&](int m) -> int {
-            return F.blk > 0 ? m - STEP * (((m - jpar) / STEP) % F.blk) : jpar;
-        };
-        int jlo, jhi;
-        const int nsw = Geo::task_sweeps(KIND, F.M, mbase, F.blk, &jlo, &jhi, F.spin);
-        if (nsw == 0) continue;   // nothing to do for this task (uniform)
-        const int npass = (nsw + WB - 1) / WB;
-        if (chain.first >= npass || chain.stride < 1) {   // a schedule that does not match this launch shape
-            if (threadIdx.x == 0) atomicExch(&g_rot_status, 4);
-            continue;
+    const int nwork = pipe ? L.nchains : L.ntasks;
+    unsigned nunit = 0;        // queue entries taken so far
+    unsigned seq = 0;          // passes begun so far
+    // The first loading warp takes an entry from the queue and hands it to the other warps, which
+    // take it up as they finish the one before: nothing in the CTA stands still between entries.
+    auto next_unit = [&]() -> int {
+        const int slot = nunit % UR;
+        const uint32_t ph = (nunit / UR) & 1;
+        ++nunit;
+        int id = 0;
+        if (warp == W) {
+            wait_bar(&uempt[slot], ph ^ 1);
+            if (lane == 0) {
+                id = atomicAdd(L.counter, 1);
+                if (id >= nwork) id = -1;
+                s_unit[slot] = id;
+                tc::mbar_arrive(&ufull[slot]);
+            }
+            id = __shfl_sync(0xffffffffu, id, 0);
+        } else {
+            wait_bar(&ufull[slot], ph);
+            id = *(volatile int *) &s_unit[slot];
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&uempt[slot]);
         }
-        const int m_lane = mbase + STEP * o_lane;
-        const int jcut_lane = jcut(m_lane);
-        // the order whose sweeps a lane runs: its own, or |m - s| for spin; emin: the least
-        // over the task's orders (every sweep below emin - STEP applies to all lanes)
-        const int me_lane = KIND == SPIN ? abs(m_lane - F.spin) : m_lane;
-        int emin = mbase;
-        if (KIND == SPIN) {
-            emin = abs(mbase - F.spin);
-            for (int o = 1; o < ORD; ++o) {
-                const int m = mbase + STEP * o;
-                if (m <= mlast) emin = min(emin, abs(m - F.spin));
+        return id;
+    };
+
+    if (warp < W) {
+        // ---------------- a stage: B consecutive sweeps of each pass ----------------
+        const int q = warp;
+        const int o_lane = lane / CH, c_lane = lane % CH;
+        const int lane_off = c_lane * T::CPAD + o_lane * NCOL;
+        uint64_t * const in_full = full + q * SL, * const in_empty = empt + q * SL;
+        uint64_t * const out_full = full + (q + 1) * SL, * const out_empty = empt + (q + 1) * SL;
+        double * const in_ring = rings + (size_t) q * SL * SLOT, * const out_ring = in_ring + (size_t) SL * SLOT;
+        double2 * const sc_ring = pairs + (size_t) q * SCS * SCLEN;
+        unsigned nin = 0, nout = 0;           // chunks taken and passed on
+        unsigned sc_issued = 0, sc_used = 0;  // (sin, cos) chunks staged and used
+        double win[NCOL][2 * B];
+        for (;;) {
+            const int id = next_unit();
+            if (id < 0) break;
+            const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
+            const RotTask task = L.tasks[chain.task];
+            const RotField & F = L.fields[task.field];
+            const TaskGeo<KIND, W, B> G(F, task);
+            const int N = G.N;
+            const int jpar = G.jpar;
+            // the order whose sweeps this lane runs (spin: |m - s|), and its lowest sweep: with
+            // F.blk > 0 a column of order m runs only the (m - jpar)/STEP mod blk sweeps above its
+            // last whole block of blk sweeps
+            const int m_lane = G.mbase + STEP * o_lane;
+            const int me_lane = KIND == SPIN ? abs(m_lane - F.spin) : m_lane;
+            const int jcut = F.blk > 0 ? m_lane - STEP * (((m_lane - jpar) / STEP) % F.blk) : jpar;
+            for (int r = chain.first; r < G.npass; r += chain.stride) {
+                const Pass<KIND, HI2LO, W, B, E> P(N, G.nsw, G.npass, G.jpar, G.jlo, r, r == 0 && F.in != F.out);
+                if (q >= P.stages) {
+                    // no sweep of the pass: hand the chunks on
+                    for (int k = 0; k < P.nchunk; ++k) {
+                        wait_bar(&in_full[nin % SL], (nin / SL) & 1);
+                        wait_bar(&out_empty[nout % SL], ((nout / SL) & 1) ^ 1);
+                        const double * const bin = in_ring + (nin % SL) * SLOT + lane_off;
+                        double * const bout = out_ring + (nout % SL) * SLOT + lane_off;
+#pragma unroll
+                        for (int e = 0; e < E; ++e)
+#pragma unroll
+                            for (int h = 0; h < NCOL; ++h) bout[e * CH * T::CPAD + h] = bin[e * CH * T::CPAD + h];
+                        __syncwarp();
+                        if (lane == 0) { tc::mbar_arrive(&in_empty[nin % SL]); tc::mbar_arrive(&out_full[nout % SL]); }
+                        ++nin; ++nout;
+                    }
+                    continue;
+                }
+                const int i0 = P.stage_sweep(q);
+                unsigned lane_mask = 0;   // sweeps this lane's order has (hi2lo applies the highest first)
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    const int j = jpar + STEP * (HI2LO ? i0 + B - 1 - b : i0 + b);
+                    if (j <= me_lane - STEP && j >= jcut) lane_mask |= 1u << b;
+                }
+                // The (sin, cos) pairs of chunk k: one bulk copy of the stage's rows (B = 4: one half
+                // of a block's) of the skewed table's chunk, whose entries are the identity where a
+                // sweep has no rotation, so every chunk runs the same straight-line code and those
+                // rotations are exact no-ops.  Returns false, staging nothing, when no sweep of the
+                // stage rotates in the chunk.
+                const int K = P.nchunk + D;
+                const int beta = i0 / Geo::kSkewRows, half = (i0 % Geo::kSkewRows) / B;
+                const int nk = beta < Geo::skew_blocks(KIND, N, jpar) ? Geo::skew_chunks(KIND, N, jpar, beta) : 0;
+                const double2 * const rows = F.sc + Geo::skew_at(KIND, N, jpar, beta) + half * B * Geo::kSkewLen * CH;
+                auto stage_sc = [&](int k) -> bool {
+                    // a stage of rows half B .. runs 2 half B positions ahead of the block's own grid
+                    const int kappa = P.kappa(k) * (E / Geo::kSkewLen) + half * 2 * B / Geo::kSkewLen;
+                    if (k >= K || kappa >= nk) return false;
+                    if (lane == 0) {
+                        const int slot = sc_issued % SCS;
+                        uint64_t * const bar = &scbar[q * SCS + slot];
+                        tc::mbar_arrive_expect_tx(bar, (uint32_t) (SCLEN * sizeof(double2)));
+                        tc::bulk_g2s(sc_ring + slot * SCLEN, rows + kappa * Geo::skew_chunk(KIND), (uint32_t) (SCLEN * sizeof(double2)), bar);
+                    }
+                    ++sc_issued;
+                    return true;
+                };
+                unsigned live = 0;        // bit i: chunk k + i is staged
+#pragma unroll
+                for (int i = 0; i + 1 < SCS; ++i) live |= stage_sc(i) ? 1u << i : 0u;
+#pragma unroll
+                for (int h = 0; h < NCOL; ++h)
+#pragma unroll
+                    for (int x = 0; x < 2 * B; ++x) win[h][x] = 0.0;
+                // element entering at chunk k leaves at chunk k + D
+                for (int k = 0; k < K; ++k) {
+                    live |= stage_sc(k + SCS - 1) ? 1u << (SCS - 1) : 0u;
+                    const bool has_in = k < P.nchunk, has_out = k >= D;
+                    const int is = nin % SL, os = nout % SL;
+                    if (has_in) wait_bar(&in_full[is], (nin / SL) & 1);
+                    if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1);
+                    const double * const bin = (has_in ? in_ring + is * SLOT : zeros) + lane_off;
+                    double * const bout = out_ring + os * SLOT + lane_off;   // written once elements leave (has_out)
+                    const bool odd = D > 1 && (k & 1);   // the chunk starts halfway round the window
+                    if (live & 1u) {
+                        const int slot = sc_used % SCS;
+                        wait_bar(&scbar[q * SCS + slot], (sc_used / SCS) & 1);
+                        ++sc_used;
+                        const double2 * sc[B];
+#pragma unroll
+                        for (int b = 0; b < B; ++b)
+                            sc[b] = ((lane_mask >> b) & 1u ? sc_ring + slot * SCLEN + (HI2LO ? B - 1 - b : b) * Geo::kSkewLen * CH : ident) + c_lane;
+                        if (odd) stage_steps<KIND, HI2LO, B, E, E % (2 * B)>(win, bin, bout, has_out, sc);
+                        else     stage_steps<KIND, HI2LO, B, E, 0>(win, bin, bout, has_out, sc);
+                    } else {
+                        if (odd) shift_steps<KIND, B, E, E % (2 * B)>(win, bin, bout, has_out);
+                        else     shift_steps<KIND, B, E, 0>(win, bin, bout, has_out);
+                    }
+                    live >>= 1;
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (has_in) tc::mbar_arrive(&in_empty[is]);
+                        if (has_out) tc::mbar_arrive(&out_full[os]);
+                    }
+                    nin += has_in; nout += has_out;
+                }
             }
         }
-        int jlo_all_max = jpar;   // highest first sweep over the task's columns
-        if (F.blk > 0)
-            for (int o = 0; o < ORD; ++o) {
-                const int m = mbase + STEP * o;
-                if (m <= mlast) jlo_all_max = max(jlo_all_max, jcut(m));
-            }
-        const int L0 = Geo::chain_len(KIND, N, 0);
-
-        for (int r = chain.first; r < npass; r += chain.stride) {
-            const double * src = r == 0 ? F.in : F.out;
-            double * dst = F.out;
-            const bool copy_all = r == 0 && F.in != F.out;
-            // Passes of W*B sweeps; the one partial pass is the one with the shortest
-            // sweeps (the first in hi2lo order, the last in lo2hi order), and only its
-            // first WA stages run, so its cost scales with its sweeps.
-            const int rem = nsw - (npass - 1) * WB;   // sweeps of the partial pass (1..WB)
-            const int s0 = HI2LO ? (r == 0 ? 0 : rem + (r - 1) * WB) : r * WB;
-            const int S = HI2LO ? (r == 0 ? rem : WB) : min(WB, nsw - s0);
-            const int WA = (S + B - 1) / B;            // active stages
-            const int WAB = WA * B;
-            const int jfirst = HI2LO ? jhi - STEP * s0 : jlo + STEP * s0;
-            int topc[CH];
-#pragma unroll
-            for (int c = 0; c < CH; ++c) topc[c] = Geo::top(KIND, N, jfirst, c);
-            const int ref = HI2LO ? topc[0] : 0;
-            int emax = HI2LO ? ref + S : topc[0] + 1;
-            if (copy_all || emax > L0 - 1) emax = L0 - 1;
-            if (emax < 0) emax = 0;
-            const int tstart = HI2LO ? ref - emax : -1;
-            const int tend = HI2LO ? ref + 2 * WAB : emax + 2 * WAB - 1;
-            const int K = (tend - tstart + 1 + E - 1) / E;
-            // pass pipeline: the previous pass's progress word and this pass's own
-            const int * const prev_prog = (pipe && r > 0) ? L.prog + chain.prog0 + r - 1 : nullptr;
-            int * const my_prog = pipe ? L.prog + chain.prog0 + r : nullptr;
-            int seen = -0x7fffffff - 1;   // (thread 0) the predecessor's progress as last read
-
-            // ---- stage state: per column a window of 2B chain positions ----
-            double win[NCOL][2 * B];
-#pragma unroll
-            for (int h = 0; h < NCOL; ++h)
-#pragma unroll
-                for (int x = 0; x < 2 * B; ++x) win[h][x] = 0.0;
-            // lane b < B: the padded-table column of sweep q*B + b and its last entry with a
-            // rotation, or -1 where the sweep has none (beyond the pass, or a column with no
-            // positions): the identity row
-            long long my_col = -1;
-            int my_lmax = -1;
-            if (lane < B) {
-                const int s = q * B + lane;
-                const int j = HI2LO ? jfirst - STEP * s : jfirst + STEP * s;
-                if (s < S && j >= 0 && j < Geo::table_cols(KIND, N)) {
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) {
-                        const int tc = Geo::top(KIND, N, j, c);
-                        if (tc >= 0) my_lmax = max(my_lmax, CH * tc + c);
+        // every staged copy was waited for above unless a wait ran out: then wait (bounded) here
+        for (; sc_used != sc_issued; ++sc_used) {
+            const long long t0 = clock64();
+            while (!tc::mbar_try_wait(&scbar[q * SCS + sc_used % SCS], (sc_used / SCS) & 1) && clock64() - t0 < (1LL << 24)) {}
+        }
+    } else if (warp < W + NL) {
+        // ---------------- loading warps: chunk i of a pass by warp i mod NL ----------------
+        const int w = warp - W;
+        unsigned n0 = 0;           // chunks of earlier passes
+        for (;;) {
+            const int id = next_unit();
+            if (id < 0) break;
+            const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
+            const RotTask task = L.tasks[chain.task];
+            const RotField & F = L.fields[task.field];
+            const TaskGeo<KIND, W, B> G(F, task);
+            if (w == 0 && lane == 0 && G.nsw > 0 && (chain.first >= G.npass || chain.stride < 1))
+                atomicExch(&g_rot_status, 4);   // a schedule that does not match this launch shape
+            const MV mv(F, task, G.mlast, lane);
+            for (int r = chain.first; r < G.npass; r += chain.stride) {
+                const Pass<KIND, HI2LO, W, B, E> P(G.N, G.nsw, G.npass, G.jpar, G.jlo, r, r == 0 && F.in != F.out);
+                const double * const src = r == 0 ? F.in : F.out;
+                const int * const prev = (pipe && r > 0) ? L.prog + chain.prog0 + r - 1 : nullptr;
+                const bool prev_local = !pipe && r > 0;
+                ++seq;
+                int seen = -0x7fffffff - 1;          // the predecessor's progress as last read
+                unsigned long long seen_local = 0;
+                // wait until the predecessor has finished the positions chunk i loads
+                auto wait_chunk = [&](int i) {
+                    if (!prev && !prev_local) return;
+                    const int pmin = P.pmin(i), pmax = pmin + E - 1;
+                    const int need = HI2LO ? -max(pmin, 0) : min(pmax, P.emax);
+                    if (prev) {
+                        if (seen < need) { if (lane == 0) seen = wait_progress(prev, need); seen = __shfl_sync(0xffffffffu, seen, 0); }
+                    } else {
+                        const unsigned long long want = local_word(seq - 1, need);
+                        if (seen_local < want) { if (lane == 0) seen_local = wait_local(&s_local, want); seen_local = __shfl_sync(0xffffffffu, seen_local, 0); }
                     }
-                    if (my_lmax >= 0) my_col = Geo::padded_col(KIND, N, j);
-                }
-            }
-            const int jmax = HI2LO ? jfirst - STEP * (q * B) : jfirst + STEP * (q * B + B - 1);
-            const int jmin = HI2LO ? jfirst - STEP * (q * B + B - 1) : jfirst + STEP * (q * B);
-            // every sweep of this stage applies to every order of the task
-            const bool full_lanes = jmax <= emin - STEP && (F.blk == 0 || jmin >= jlo_all_max);
-            unsigned lane_mask = 0;                          // sweeps that apply to this lane's order
-#pragma unroll
-            for (int b = 0; b < B; ++b) {
-                const int sg = q * B + b;
-                const int j = HI2LO ? jfirst - STEP * sg : jfirst + STEP * sg;
-                if (j <= me_lane - STEP && j >= jcut_lane) lane_mask |= 1u << b;
-            }
-
-            // Stage the (sin, cos) pairs of a chunk: entry (b, jj) is the pair sweep b uses at step
-            // u of the chunk on chain c (jj = CH u + c, u reversed in hi2lo), i.e. the CH E
-            // consecutive entries of its padded column starting at chain position ibase, where the
-            // padding holds the identity (sin 0, cos 1) wherever the sweep has no rotation at that
-            // step: every chunk runs the same straight-line code and those rotations are exact
-            // no-ops.  One bulk copy per sweep (lanes 0 .. B-1) completes on the stage's mbarrier
-            // for the slot.  A chunk in which none of the stage's sweeps has a rotation is not
-            // staged at all: the stage passes its elements through unrotated (sc_live).
-            auto prefetch_sc = [&](int kp) {
-                const int t0p = tstart + kp * E;
-                const int slot = kp & 1;
-                double2 * const d = sc_stage(q, slot);
-                uint64_t * const bar = &s_mbar[q * 2 + slot];
-                int lo = 0;
-                bool overlaps = false;
-                if (lane < B) {
-                    const int sg = q * B + lane;
-                    lo = CH * (HI2LO ? ref + 2 * sg - t0p - E + 1 : t0p - 2 * sg);   // first entry
-                    // a chunk overlapping the sweep's entries reaches at most E positions past
-                    // them, into the padding; one outside them reads the identity row
-                    overlaps = my_col >= 0 && lo <= my_lmax && lo + CH * E > 0;
-                }
-                const bool live = __ballot_sync(0xffffffffu, overlaps) != 0u;
-                sc_live = live ? (sc_live | (1u << slot)) : (sc_live & ~(1u << slot));
-                if (!live) return;
-                if (lane == 0) tc::mbar_arrive_expect_tx(bar, (uint32_t) (B * E * CH * sizeof(double2)));
-                __syncwarp();
-                if (lane < B) {
-                    const double2 * src = overlaps ? F.sc + my_col + lo : F.sc;
-                    tc::bulk_g2s(d + lane * (E * CH), src, (uint32_t) (E * CH * sizeof(double2)), bar);
-                }
-            };
-            // wait until the stage's (sin, cos) of chunk k have landed (bounded: a wait that runs out
-            // sets the status word, and every later wait of the launch gives up at once)
-            auto wait_sc = [&](int k) {
-                const int slot = k & 1;
-                if (!tc::mbar_wait(&s_mbar[q * 2 + slot], (sc_phase >> slot) & 1u, (volatile int *) &g_rot_status)) {
-                    if (lane == 0) atomicCAS(&g_rot_status, 0, 5);
-                }
-                sc_phase ^= 1u << slot;
-            };
-
-            // ---- global traffic, shared by all warps: warp w moves elements
-            //      v in [w*PER_W, (w+1)*PER_W) of each chunk (f = v*32 + lane) ----
-            constexpr int RPC = E * CH;                // rows of one column segment per chunk
-            constexpr int PER = COLS * RPC / 32;       // elements per lane per chunk (all warps)
-            constexpr int PER_W = PER / W;             // this warp's share
-            static_assert(PER % W == 0, "chunk must split evenly over the warps");
-            double pre[PER_W];
-            // Element v of this lane's share: task column cl and row offset rr inside
-            // the chunk's contiguous row range (row = CH * pmin + rr).  Everything but
-            // pmin is fixed for the pass, so it is computed once here.
-            const double * gsrc[PER_W];
-            double * gdst[PER_W];
-            int ioff[PER_W];     // rr >> (CH - 1): position offset from pmin
-            int rro[PER_W];      // rr: row offset from CH * pmin
-            int soff[PER_W];     // shared-memory offset inside a slot
-            bool colok[PER_W];
-#pragma unroll
-            for (int v = 0; v < PER_W; ++v) {
-                const int f = (q * PER_W + v) * 32 + lane;
-                const int cl = f / RPC, rr = f % RPC;
-                const int o = cl / NCOL, h = cl % NCOL;
-                const int mcl = mbase + STEP * o;
-                long long coff;
-                if constexpr (KIND == SPIN) {
-                    // h: real / imaginary part (h & 1) of the column of -m (h < 2: 2m - 1, or 0
-                    // for m = 0) or of m (2m)
-                    const long long colc = h < 2 ? (mcl == 0 ? 0 : 2 * mcl - 1) : 2 * mcl;
-                    colok[v] = mcl <= mlast && !(mcl == 0 && h >= 2) && colc < F.M;
-                    coff = colok[v] ? ES * (colc * lda + rr) + (h & 1) : 0;
-                } else {
-                    const long long colc = (KIND == TRI || KIND == RECT) ? mcl : 2 * mcl - 1 + h;
-                    colok[v] = mcl <= mlast;
-                    coff = colok[v] ? colc * lda + rr : 0;
-                }
-                gsrc[v] = src + coff;
-                gdst[v] = dst + coff;
-                ioff[v] = CH == 2 ? (rr >> 1) : rr;
-                rro[v] = rr;
-                const int c = CH == 2 ? (rr & 1) : 0;
-                const int u = HI2LO ? E - 1 - ioff[v] : ioff[v];
-                soff[v] = (u * CH + c) * CPAD + cl;
-            }
-            // lowest chain position of chunk k entering stage 0 (storer: leaving stage W-1)
-            auto pmin_of = [&](int k, bool storer) -> int {
-                const int t0 = tstart + k * E;
-                return HI2LO ? ref - t0 - E + 1 + (storer ? 2 * WAB : 0) : t0 + 1 - (storer ? 2 * WAB : 0);
-            };
-            auto row_ok = [&](int pmin, int v) -> bool {
-                const int p = pmin + ioff[v];
-                const int row = CH * pmin + rro[v];
-                return colok[v] && p >= 0 && p <= emax && row < N;
-            };
-            // (thread 0) wait until the predecessor has finished the positions chunk k loads
-            auto wait_chunk = [&](int k) {
-                if (!prev_prog || k >= K) return;
-                const int pmin = pmin_of(k, false), pmax = pmin + E - 1;
-                if (pmax < 0 || pmin > emax) return;                 // nothing of the chunk is loaded
-                // the predecessor publishes every few chunks and runs ahead: one acquire covers the
-                // chunks up to the progress it read, which the words only ever raise
-                const int need = HI2LO ? -max(pmin, 0) : min(pmax, emax);
-                if (seen < need) seen = wait_progress(prev_prog, need);
-            };
-            auto load_chunk = [&](int k) {
-                const int pmin = pmin_of(k, false);
-#pragma unroll
-                for (int v = 0; v < PER_W; ++v)
-                    pre[v] = (k < K && row_ok(pmin, v)) ? __ldcg(gsrc[v] + (long long) ES * CH * pmin) : 0.0;
-            };
-            auto stash_chunk = [&](int k) {
-                double * const b0 = buf(0, k & 1, 0, 0);
-#pragma unroll
-                for (int v = 0; v < PER_W; ++v) b0[soff[v]] = pre[v];
-            };
-            // the pass pipeline publishes progress every stored chunk for short columns, every
-            // fourth for long ones (and after the last): a successor trailing by a few chunks more
-            // loses little of a long pass, while a publish costs its CTA a fence and a release
-            auto publishes = [&](int k) {
-                const int m = F.N >= 2048 ? 3 : 0;
-                return (k & m) == m || k == K - 1;
-            };
-            auto store_chunk = [&](int k) {
-                const int pmin = pmin_of(k, true);
-                const double * const bw = buf(WA, k & 1, 0, 0);
-#pragma unroll
-                for (int v = 0; v < PER_W; ++v)
-                    if (row_ok(pmin, v)) __stcg(gdst[v] + (long long) ES * CH * pmin, bw[soff[v]]);
-            };
-            if (pipe) {
-                if (threadIdx.x == 0) {
-                    wait_chunk(0);
-                    wait_chunk(1);
-                    // hi2lo: positions above this pass's range are final once the predecessor
-                    // has finished the first chunk's (they belong to earlier passes only)
-                    publish_progress(my_prog, HI2LO ? -(emax + 1) : -1);
-                }
-                __syncthreads();
-            }
-            load_chunk(0);
-            stash_chunk(0);
-            if (q == 0) prefetch_sc(0);
-            __syncthreads();
-
-            for (int it = 0; it < K + WA; ++it) {
-                // chunk it+1: loads in flight while the stages work on their chunks
-                if (it + 1 < K) load_chunk(it + 1);
-                // the last active stage finished chunk it-WA in the previous iteration
-                if (it - WA >= 0 && it - WA < K) store_chunk(it - WA);
-                // (sin, cos) of the chunk this stage works on next iteration
-                if (q < WA && it + 1 - q >= 0 && it + 1 - q < K) prefetch_sc(it + 1 - q);
-                const int k = it - q;
-                if (q < WA && k >= 0 && k < K && !((sc_live >> (k & 1)) & 1u)) {
-                    // no rotation of this stage in the chunk: the window only shifts, every element
-                    // leaves the stage as it entered (the sequential loops do not touch them either)
-                    const int slot = k & 1;
-#pragma unroll
-                    for (int u = 0; u < E; ++u) {
-                        const int pn = u % (2 * B);
-                        const double * bin = buf(q, slot, u, c_lane) + o_lane * NCOL;
-                        double * bout = buf(q + 1, slot, u, c_lane) + o_lane * NCOL;
-#pragma unroll
-                        for (int h = 0; h < NCOL; ++h) {
-                            const double in = bin[h];
-                            bout[h] = win[h][pn];
-                            win[h][pn] = in;
-                        }
+                    __syncwarp();
+                };
+                // the copies land in the slot by themselves: up to SL chunks are on their way
+                auto fetch = [&](int i) {
+                    const unsigned n = n0 + i;
+                    const int pmin = P.pmin(i);
+                    wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1);
+                    double * const slot = rings + (size_t) (n % SL) * SLOT;
+#pragma unroll 4
+                    for (int v = 0; v < MV::PER; ++v) {
+                        const bool valid = mv.seg_ok(v) && mv.row_ok(v, pmin, P.emax);
+                        copy_async8(slot + mv.slot_at(v), valid ? src + mv.at(v, pmin) : src, valid);
                     }
-                } else if (q < WA && k >= 0 && k < K) {
-                    const int slot = k & 1;
-                    wait_sc(k);
-                    const double2 * const scb = sc_stage(q, slot);
-                    const bool masked = !full_lanes;
-                    // two copies of the step loop: all sweeps apply to all lanes, or per-lane masks
-                    auto run = [&](auto masked_tag) {
-                        constexpr bool MASKED = decltype(masked_tag)::value;
-#pragma unroll
-                        for (int u = 0; u < E; ++u) {
-                            // The window is circular: at step u, window position x lives in
-                            // register slot (u - x) mod 2B.  The element leaving (position
-                            // 2B-1 of the previous step) sits in slot u mod 2B, which the
-                            // entering element (position 0) takes over.  E is a multiple of
-                            // 2B, so the mapping is the same at every chunk boundary.
-                            constexpr int W2 = 2 * B;
-                            const int pn = u % W2;
-                            const double * bin = buf(q, slot, u, c_lane) + o_lane * NCOL;
-                            double * bout = buf(q + 1, slot, u, c_lane) + o_lane * NCOL;
-#pragma unroll
-                            for (int h = 0; h < NCOL; ++h) {
-                                const double in = bin[h];
-                                bout[h] = win[h][pn];
-                                win[h][pn] = in;
-                            }
-                            const int obase = HI2LO ? (CH == 2 ? 2 * (E - 1 - u) : E - 1 - u) : (CH == 2 ? 2 * u : u);
-#pragma unroll
-                            for (int b = 0; b < B; ++b) {
-                                const double2 sc = scb[b * (E * CH) + obase + (CH == 2 ? c_lane : 0)];
-                                double sn = sc.x, cs = sc.y;
-                                if (MASKED) {
-                                    const bool on = (lane_mask >> b) & 1u;
-                                    sn = on ? sn : 0.0;
-                                    cs = on ? cs : 1.0;
-                                }
-                                const int xl = (u - 2 * b + 2 * W2) % W2;       // window position 2b
-                                const int xu = (u - 2 * b - 1 + 2 * W2) % W2;   // window position 2b+1
-#pragma unroll
-                                for (int h = 0; h < NCOL; ++h) {
-                                    if (HI2LO) rot_hi2lo(win[h][xl], win[h][xu], sn, cs);
-                                    else       rot_lo2hi(win[h][xu], win[h][xl], sn, cs);
-                                }
-                            }
-                        }
-                    };
-                    if (masked) run(std::true_type{});
-                    else        run(std::false_type{});
-                }
-                if (it + 1 < K) stash_chunk(it + 1);
-                if (pipe && threadIdx.x == 0) wait_chunk(it + 2);   // loaded next iteration
-                __syncthreads();
-                // the chunks stored up to this iteration are final: publish them
-                if (pipe && threadIdx.x == 0 && it - WA >= 0 && it - WA < K && publishes(it - WA)) {
-                    const int pmin = pmin_of(it - WA, true);
-                    publish_progress(my_prog, HI2LO ? -pmin : pmin + E - 1);
+                    copy_async_arrive(&full[n % SL]);
+                };
+                wait_chunk(0);
+                // hi2lo: the positions above this pass's range are final once the predecessor has
+                // finished the first chunk's (they belong to earlier passes only)
+                if (pipe && w == 0 && lane == 0) publish_progress(L.prog + chain.prog0 + r, HI2LO ? -(P.emax + 1) : -1);
+                for (int i = w; i < P.nchunk; i += NL) { wait_chunk(i); fetch(i); }
+                n0 += P.nchunk;
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+    } else {
+        // ---------------- storing warp ----------------
+        unsigned n = 0;
+        uint64_t * const bfull = full + W * SL, * const bempt = empt + W * SL;
+        const double * const ring = rings + (size_t) W * SL * SLOT;
+        for (;;) {
+            const int id = next_unit();
+            if (id < 0) break;
+            const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
+            const RotTask task = L.tasks[chain.task];
+            const RotField & F = L.fields[task.field];
+            const TaskGeo<KIND, W, B> G(F, task);
+            const MV mv(F, task, G.mlast, lane);
+            // publish every 16 positions for short columns, every 64 for long ones (and at the end): a
+            // successor trailing by a little more loses little of a long pass
+            const int every = max(1, (F.N >= 2048 ? 64 : 16) / E);
+            for (int r = chain.first; r < G.npass; r += chain.stride) {
+                const Pass<KIND, HI2LO, W, B, E> P(G.N, G.nsw, G.npass, G.jpar, G.jlo, r, r == 0 && F.in != F.out);
+                ++seq;
+                int since = 0;
+                for (int i = 0; i < P.nchunk; ++i, ++n) {
+                    const int pmin = P.pmin(i);
+                    wait_bar(&bfull[n % SL], (n / SL) & 1);
+                    const double * const slot = ring + (n % SL) * SLOT;
+#pragma unroll 4
+                    for (int v = 0; v < MV::PER; ++v)
+                        if (mv.seg_ok(v) && mv.row_ok(v, pmin, P.emax)) __stcg(F.out + mv.at(v, pmin), slot[mv.slot_at(v)]);
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&bempt[n % SL]);
+                    if (++since < every && i + 1 < P.nchunk) continue;
+                    since = 0;
+                    __syncwarp();
+                    if (lane == 0) {
+                        const int v = i + 1 == P.nchunk ? 0x7fffffff : HI2LO ? -pmin : pmin + E - 1;
+                        if (pipe) publish_progress(L.prog + chain.prog0 + r, v);
+                        else      publish_local(&s_local, local_word(seq, v));
+                    }
                 }
             }
-            if (pipe && threadIdx.x == 0) publish_progress(my_prog, 0x7fffffff);
         }
     }
 }
 
-template <int KIND, bool HI2LO, int W, int B, int E>
-cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, cudaStream_t st) {
-    constexpr int CH = KT<KIND>::CH, CPAD = KT<KIND>::CPAD;
-    const size_t shm = sizeof(double) * (size_t) (W + 1) * 2 * E * CH * CPAD + sizeof(double2) * (size_t) W * 2 * B * E * CH;
-    auto kern = rot_kernel<KIND, HI2LO, W, B, E>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
+template <int KIND, bool HI2LO, int W, int B, int E, int MINB>
+cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaStream_t st) {
+    using SH = Shape<KIND, W, B, E>;
+    auto kern = rot_kernel<KIND, HI2LO, W, B, E, MINB>;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm = 1;   // resident CTAs per SM (two for the four-warp shapes)
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, W * 32, shm) != cudaSuccess || per_sm < 1) per_sm = 1;
-    int ctas = sms * per_sm;
+    // resident CTAs of the whole device, asked for once per device
+    static std::atomic<int> resident[16] = {};   // SMs x 256 + CTAs per SM
+    int room = dev < 16 ? resident[dev].load(std::memory_order_acquire) : 0;
+    if (room == 0) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SH::bytes);
+        if (e != cudaSuccess) return e;
+        int sms = 0, per_sm = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SH::WARPS * 32, SH::bytes) != cudaSuccess || per_sm < 1) per_sm = 1;
+        room = sms * 256 + per_sm;
+        if (dev < 16) resident[dev].store(room, std::memory_order_release);
+    }
+    int ctas = (room >> 8) * (per_sm_most > 0 ? std::min(per_sm_most, room & 255) : room & 255);
     if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
     const int work = L.chains ? L.nchains : L.ntasks;   // queue entries: pipeline entries or tasks
     if (ctas > work) ctas = work;
     if (ctas <= 0) return cudaSuccess;
     e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    kern<<<ctas, W * 32, shm, st>>>(L);
+    kern<<<ctas, SH::WARPS * 32, SH::bytes, st>>>(L);
     count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         cudaFuncAttributes fa{};
         cudaFuncGetAttributes(&fa, kern);
         std::fprintf(stderr, "rot_kernel launch failed (%s): regs %d, static smem %zu, dyn smem %zu, max threads %d, params %zu B\n",
-                     cudaGetErrorString(e), fa.numRegs, fa.sharedSizeBytes, shm, fa.maxThreadsPerBlock, sizeof(RotLaunch));
+                     cudaGetErrorString(e), fa.numRegs, fa.sharedSizeBytes, SH::bytes, fa.maxThreadsPerBlock, sizeof(RotLaunch));
     }
     return e;
 }
 
+// ---------------------------------------------------------------------------
+// The same sweeps with the columns of a task resident in shared memory, for chains short enough
+// to fit.  One CTA per group of orders, one lane per sequence (order, column, chain); the warps
+// take the task's blocks of B sweeps in turn and run down the columns in place, warp g + 1 behind
+// warp g.  Nothing is streamed between stages or passes, so a column's sweeps follow each other at
+// a distance of 2B + E positions whatever their number, and the loop is short enough for the
+// instruction cache.  Each (sin, cos) load feeds one sequence instead of two, so a chip full of
+// tasks runs faster in rot_kernel (launch_rotations has the rule).
+// ---------------------------------------------------------------------------
+template <int KIND>
+struct RT {
+    static constexpr int CH = KT<KIND>::CH, STEP = KT<KIND>::STEP, ES = KT<KIND>::ES, NC = KT<KIND>::NCOL;
+    static constexpr int ORD = 32 / (CH * NC);                  // orders of a CTA
+    static constexpr int SPLIT = KT<KIND>::ORD / ORD;           // CTAs of a task of the list
+    static constexpr int W = 8, B = 8, E = 8, D = 2 * B / E, SCS = 3;
+    static constexpr int ROW = 33;                              // doubles of a position: 32 lanes and a pad
+    static constexpr int SCLEN = B * E * CH, IDLEN = E * CH;
+    static constexpr size_t pair_bytes = sizeof(double2) * ((size_t) W * SCS * SCLEN + IDLEN);
+    // positions -1 .. chain_len rounded up to whole chunks
+    __host__ __device__ static int rows(int N) { return (Geo::chain_len(KIND, N, 0) + E - 1) / E * E + E; }
+    __host__ __device__ static size_t bytes(int N) { return pair_bytes + sizeof(double) * (size_t) rows(N) * ROW; }
+};
+
+template <int KIND, bool HI2LO>
+__global__ void __launch_bounds__(RT<KIND>::W * 32, 2)
+rot_resident_kernel(const __grid_constant__ RotLaunch L) {
+    using R = RT<KIND>;
+    constexpr int CH = R::CH, STEP = R::STEP, ES = R::ES, NC = R::NC, ORD = R::ORD, W = R::W, B = R::B, E = R::E, D = R::D,
+                  SCS = R::SCS, ROW = R::ROW, SCLEN = R::SCLEN;
+    extern __shared__ __align__(16) double smem[];
+    double2 * const pairs = reinterpret_cast<double2 *>(smem);
+    double2 * const ident = pairs + W * SCS * SCLEN;
+    double * const col = reinterpret_cast<double *>(ident + R::IDLEN) + ROW;   // position p of lane l at col[p * ROW + l]
+    __shared__ __align__(8) uint64_t scbar[W * SCS];
+    __shared__ int prog[W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    const RotTask task = L.tasks[blockIdx.x / R::SPLIT];
+    const RotField & F = L.fields[task.field];
+    const int N = F.N, mlast = Geo::last_order(KIND, F.M);
+    const int mbase = task.mbase + STEP * ORD * (R::SPLIT - 1 - (int) (blockIdx.x % R::SPLIT));
+    if (mbase > mlast) return;
+    int jlo, jhi;
+    const int nsw = Geo::task_sweeps(KIND, F.M, mbase, F.blk, &jlo, &jhi, F.spin, ORD);
+    const int jpar = KIND == TRI ? 0 : (KIND == SPIN ? ((mbase + F.spin) & 1) : (mbase & 1));
+    if (nsw == 0 && F.in == F.out) return;
+
+    if (threadIdx.x < W) prog[threadIdx.x] = -1;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < W * SCS; ++i) tc::mbar_init(&scbar[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < R::IDLEN; i += blockDim.x) ident[i] = make_double2(0.0, 1.0);
+    // columns in: segment s is a column (order s / SEGC), its doubles in memory order
+    constexpr int SEGC = NC / ES;                 // columns of an order
+    const int rowsN = R::rows(N), len = N * ES;
+    // positions outside the chains (and the second chain's last one of an odd column): zero
+    for (int i = threadIdx.x; i < ROW; i += blockDim.x) col[i - ROW] = 0.0;
+    for (int i = N / CH * ROW + threadIdx.x; i < (rowsN - 1) * ROW; i += blockDim.x) col[i] = 0.0;
+    __syncthreads();
+    auto column_at = [&](int s, long long * at) -> bool {
+        const int o = s / SEGC, m = mbase + STEP * o;
+        long long c;
+        if (KIND == TRI || KIND == RECT) c = m;
+        else if (KIND == SPIN) c = 2LL * m - (task.side ? 0 : 1);
+        else c = 2LL * m - 1 + s % SEGC;
+        *at = c * ES * F.lda;
+        return m <= mlast && c >= 0 && c < F.M;
+    };
+    auto place = [&](int s, int x) -> int {       // double x of segment s
+        const int row = x / ES, h = ES == 2 ? x % 2 : s % SEGC;
+        return row / CH * ROW + (s / SEGC * NC + h) * CH + row % CH;
+    };
+    for (int s = warp; s < ORD * SEGC; s += W) {
+        long long at;
+        const bool there = column_at(s, &at);
+#pragma unroll 4
+        for (int x = lane; x < len; x += 32) col[place(s, x)] = there ? __ldcg(F.in + at + x) : 0.0;
+    }
+    __syncthreads();
+
+    const int nblk = (nsw + B - 1) / B;
+    const int c_lane = lane % CH, m_lane = mbase + STEP * (lane / (CH * NC));
+    const int me_lane = KIND == SPIN ? abs(m_lane - F.spin) : m_lane;
+    const int jcut = F.blk > 0 ? m_lane - STEP * (((m_lane - jpar) / STEP) % F.blk) : jpar;
+    double2 * const sc_ring = pairs + warp * SCS * SCLEN;
+    uint64_t * const bars = scbar + warp * SCS;
+    unsigned sc_issued = 0, sc_used = 0;
+    for (int g = warp; g < nblk; g += W) {
+        const int i0 = (jlo - jpar) / STEP + (HI2LO ? nblk - 1 - g : g) * B;
+        // chunk c covers positions cE .. cE + E - 1 (hi2lo, from the highest with a rotation down)
+        // or cE - 1 .. cE + E - 2 (lo2hi, from 0 up), aligned as the skewed table is
+        const int last = Geo::chain_len(KIND, N, 0) - 1;
+        const int emax = max(0, min(last, Geo::top(KIND, N, jpar + STEP * i0, 0) + 1));
+        const int chi = HI2LO ? emax / E : (emax + 1) / E;
+        const int K = chi + 1 + D;
+        const int beta = i0 / Geo::kSkewRows;
+        const int nk = beta < Geo::skew_blocks(KIND, N, jpar) ? Geo::skew_chunks(KIND, N, jpar, beta) : 0;
+        const double2 * const rows = F.sc + Geo::skew_at(KIND, N, jpar, beta);
+        auto stage_sc = [&](int k) -> bool {
+            const int kappa = HI2LO ? chi + D - k : k;
+            if (k >= K || kappa >= nk) return false;
+            if (lane == 0) {
+                uint64_t * const bar = &bars[sc_issued % SCS];
+                tc::mbar_arrive_expect_tx(bar, (uint32_t) (SCLEN * sizeof(double2)));
+                tc::bulk_g2s(sc_ring + (sc_issued % SCS) * SCLEN, rows + kappa * Geo::skew_chunk(KIND), (uint32_t) (SCLEN * sizeof(double2)), bar);
+            }
+            ++sc_issued;
+            return true;
+        };
+        unsigned live = 0;
+#pragma unroll
+        for (int i = 0; i + 1 < SCS; ++i) live |= stage_sc(i) ? 1u << i : 0u;
+        unsigned lane_mask = 0;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int j = jpar + STEP * (HI2LO ? i0 + B - 1 - b : i0 + b);
+            if (j <= me_lane - STEP && j >= jcut) lane_mask |= 1u << b;
+        }
+        double win[2 * B];
+#pragma unroll
+        for (int x = 0; x < 2 * B; ++x) win[x] = 0.0;
+        // The warp's word: block g, and how far down the columns it is final (hi2lo: every chunk >= c
+        // as 2048 - c, lo2hi: every chunk <= c as c + 1).  Chunks above a block's own in hi2lo order
+        // have not been touched by the blocks before it either.
+        volatile int * const mine = &prog[warp];
+        const int * const before = &prog[(warp + W - 1) % W];
+        if (lane == 0) *mine = g * 4096 + (HI2LO ? 2048 - (chi + 1) : 0);
+        int seen = -2;
+        for (int k = 0; k < K; ++k) {
+            live |= stage_sc(k + SCS - 1) ? 1u << (SCS - 1) : 0u;
+            const bool has_in = k <= chi, has_out = k >= D;
+            const int cin = HI2LO ? chi - k : k, cout = HI2LO ? cin + D : cin - D;
+            if (has_in && g > 0) {
+                const int need = (g - 1) * 4096 + (HI2LO ? 2048 - cin : cin + 1);
+                if (seen < need) seen = wait_word(before, need);
+            }
+            // position of the chunk's first step, and the way the steps go
+            const double * const bin = col + (HI2LO ? cin * E + E - 1 : cin * E - 1) * ROW + lane;
+            double * const bout = col + (HI2LO ? cout * E + E - 1 : cout * E - 1) * ROW + lane;
+            const bool odd = D > 1 && (k & 1);
+            if (live & 1u) {
+                const int slot = sc_used % SCS;
+                wait_bar(&bars[slot], (sc_used / SCS) & 1);
+                ++sc_used;
+                const double2 * sc[B];
+#pragma unroll
+                for (int b = 0; b < B; ++b)
+                    sc[b] = ((lane_mask >> b) & 1u ? sc_ring + slot * SCLEN + (HI2LO ? B - 1 - b : b) * E * CH : ident) + c_lane;
+                if (odd) resident_steps<HI2LO, CH, B, E, E % (2 * B), ROW, true>(win, bin, bout, has_in, has_out, sc);
+                else     resident_steps<HI2LO, CH, B, E, 0, ROW, true>(win, bin, bout, has_in, has_out, sc);
+            } else {
+                const double2 * const none[B] = {};
+                if (odd) resident_steps<HI2LO, CH, B, E, E % (2 * B), ROW, false>(win, bin, bout, has_in, has_out, none);
+                else     resident_steps<HI2LO, CH, B, E, 0, ROW, false>(win, bin, bout, has_in, has_out, none);
+            }
+            live >>= 1;
+            __syncwarp();
+            if (lane == 0 && has_out) publish_word(&prog[warp], g * 4096 + (k + 1 == K ? 4095 : HI2LO ? 2048 - cout : cout + 1));
+        }
+    }
+    for (; sc_used != sc_issued; ++sc_used) {     // only after a wait that ran out: no copy may outlive the CTA
+        const long long t0 = clock64();
+        while (!tc::mbar_try_wait(&bars[sc_used % SCS], (sc_used / SCS) & 1) && clock64() - t0 < (1LL << 24)) {}
+    }
+    __syncthreads();
+    for (int s = warp; s < ORD * SEGC; s += W) {
+        long long at;
+        if (!column_at(s, &at)) continue;
+#pragma unroll 4
+        for (int x = lane; x < len; x += 32) __stcg(F.out + at + x, col[place(s, x)]);
+    }
+}
+
+// Resident CTAs cover a field's whole columns, so they take it when its chains fit.
+template <int KIND>
+bool resident_fits(const RotLaunch & L) {
+    for (int f = 0; f < L.nfields; ++f)
+        if (RT<KIND>::bytes(L.fields[f].N) + 1024 > 232448 || Geo::chain_len(KIND, L.fields[f].N, 0) / RT<KIND>::E > 2000) return false;
+    return true;
+}
+
+template <int KIND, bool HI2LO>
+cudaError_t launch_resident(const RotLaunch & L, cudaStream_t st) {
+    using R = RT<KIND>;
+    auto kern = rot_resident_kernel<KIND, HI2LO>;
+    int nmax = 0;
+    for (int f = 0; f < L.nfields; ++f) nmax = std::max(nmax, L.fields[f].N);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    static std::atomic<bool> ready[16] = {};
+    if (dev >= 16 || !ready[dev].load(std::memory_order_acquire)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024);
+        if (e != cudaSuccess) return e;
+        if (dev < 16) ready[dev].store(true, std::memory_order_release);
+    }
+    kern<<<L.ntasks * R::SPLIT, R::W * 32, R::bytes(nmax), st>>>(L);
+    count_launch();
+    return cudaGetLastError();
+}
+
 }  // namespace
 
-// Configurations: W stage warps x B sweeps per warp, chunk E.
-//   0: W = 8,  B = 8, E = 16 (255 registers, two warps per sub-partition)
-//   1: W = 16, B = 4, E = 8  (128 registers, four warps per sub-partition)
-//   2: W = 8,  B = 4, E = 8  (fewer sweeps per warp: lighter register pressure)
-//   3: W = 8,  B = 4, E = 16
-//   4: W = 4,  B = 4, E = 16 (two CTAs per SM)
-//   5: W = 4,  B = 8, E = 16 (two CTAs per SM where shared memory allows: tri, disk)
+// Launch shapes: 0 .. 4 rot_kernel with W stage warps x B sweeps per warp, chunk E, CTAs per SM
+// (0: as many as fit); 5 rot_resident_kernel.
+//   0: 8 x 8 x 16    1: 8 x 8 x 8    2: 4 x 8 x 8, one CTA per SM    3: 8 x 4 x 8    4: 4 x 8 x 8
 template <int KIND, bool HI2LO>
 cudaError_t launch_kind(int cfg, const RotLaunch & L, int max_ctas, cudaStream_t st) {
-    if constexpr (KIND == SPIN) {
-        (void) cfg;   // four sequences per lane: only 8 x 4 x 8 fits the stage buffers
-        return launch_cfg<KIND, HI2LO, 8, 4, 8>(L, max_ctas, st);
-    } else {
-        if constexpr (KIND != TRI && KIND != RECT) {   // one sequence per lane: too few rows per warp
-            if (cfg == 1) return launch_cfg<KIND, HI2LO, 16, 4, 8>(L, max_ctas, st);
-        }
-        if (cfg == 2) return launch_cfg<KIND, HI2LO, 8, 4, 8>(L, max_ctas, st);
-        if (cfg == 3) return launch_cfg<KIND, HI2LO, 8, 4, 16>(L, max_ctas, st);
-        if (cfg == 4) return launch_cfg<KIND, HI2LO, 4, 4, 16>(L, max_ctas, st);
-        if (cfg == 5) return launch_cfg<KIND, HI2LO, 4, 8, 16>(L, max_ctas, st);
-        return launch_cfg<KIND, HI2LO, 8, 8, 16>(L, max_ctas, st);
-    }
+    if (cfg == 5 && resident_fits<KIND>(L)) return launch_resident<KIND, HI2LO>(L, st);
+    if (cfg == 1) return launch_cfg<KIND, HI2LO, 8, 8, 8, 1>(L, max_ctas, 0, st);
+    if (cfg == 2) return launch_cfg<KIND, HI2LO, 4, 8, 8, 2>(L, max_ctas, 1, st);
+    if (cfg == 3) return launch_cfg<KIND, HI2LO, 8, 4, 8, 1>(L, max_ctas, 0, st);
+    if (cfg == 4) return launch_cfg<KIND, HI2LO, 4, 8, 8, 2>(L, max_ctas, 0, st);
+    return launch_cfg<KIND, HI2LO, 8, 8, 16, 1>(L, max_ctas, 0, st);
 }
 
 int g_rot_cfg = -2;
@@ -609,21 +962,22 @@ void rot_schedule_free(RotSchedule * s) {
     delete s;
 }
 
-bool rotation_plan_pad(ft_rotation_plan * RP) {
-    if (RP->d_scp) { cudaFree(RP->d_scp); RP->d_scp = nullptr; }
-    const long long len = Geo::padded_len(RP->kind, RP->n);
-    cudaError_t e = cudaMalloc(&RP->d_scp, sizeof(double2) * len);
+bool rotation_plan_skew(ft_rotation_plan * RP) {
+    if (RP->d_skew) { cudaFree(RP->d_skew); RP->d_skew = nullptr; }
+    const long long len = std::max(1LL, Geo::skew_len(RP->kind, RP->n));
+    cudaError_t e = cudaMalloc(&RP->d_skew, sizeof(double2) * len);
     if (e != cudaSuccess) {
-        RP->d_scp = nullptr;
-        set_error(e == cudaErrorMemoryAllocation ? FT_B200_ENOMEM : FT_B200_ECUDA, std::string("cudaMalloc(padded table): ") + cudaGetErrorString(e));
+        RP->d_skew = nullptr;
+        set_error(e == cudaErrorMemoryAllocation ? FT_B200_ENOMEM : FT_B200_ECUDA, std::string("cudaMalloc(skewed table): ") + cudaGetErrorString(e));
         return false;
     }
-    pad_table_kernel<<<Geo::table_cols(RP->kind, RP->n) + 2, 256>>>(RP->d_sc, RP->d_scp, RP->kind, RP->n);
+    const dim3 grid((unsigned) std::max(1, Geo::skew_blocks(RP->kind, RP->n, 0)), (unsigned) Geo::skew_parities(RP->kind));
+    skew_table_kernel<<<grid, 256>>>(RP->d_sc, RP->d_skew, RP->kind, RP->n);
     count_launch();
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
-        set_error(FT_B200_ECUDA, std::string("pad_table_kernel: ") + cudaGetErrorString(e));
+        set_error(FT_B200_ECUDA, std::string("skew_table_kernel: ") + cudaGetErrorString(e));
         return false;
     }
     return true;
@@ -643,7 +997,7 @@ namespace {
 
 // Sweeps per pass (W x B) of each launch shape.
 int shape_pass(int cfg) {
-    static const int wb[6] = {64, 64, 32, 32, 16, 32};
+    static const int wb[6] = {64, 64, 32, 32, 32, 64};
     return (cfg >= 0 && cfg < 6) ? wb[cfg] : 64;
 }
 
@@ -688,7 +1042,7 @@ const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotL
         int dev = 0, l2 = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-        const int seqs = (kind == TRI || kind == RECT) ? 1 : (kind == SPIN ? 4 : 2);   // doubles per order and row
+        const int seqs = (kind == TRI || kind == RECT) ? 1 : 2;   // doubles per order and row
         const long long cols = (long long) Geo::task_orders(kind) * seqs;
         const long long foot = cols * (long long) L.fields[0].N * (long long) sizeof(double);
         npipe = (int) std::min<long long>(nt, std::max<long long>(1, (l2 / 2) / std::max<long long>(foot, 1)));
@@ -746,10 +1100,27 @@ cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int
     return launch_with(kind, hi2lo, shape, P, max_ctas, st);
 }
 
-// Configuration without measurements: launches that run only the heads above whole
-// blocks (blk > 0: fewer than blk sweeps per column, 2 blk - 2 per task at most) keep more
-// stages busy with 4 sweeps per warp; full sweeps use 8 per warp.
-int default_config(const RotLaunch & L) { return (L.nfields > 0 && L.fields[0].blk > 0) ? 3 : 0; }
+// Configuration without measurements (in-place launches, capturing streams, the first launches of
+// the spin and tetrahedral sweeps).  Measured per launch in us, one field in place, resident /
+// 4 x 8 x 8 on one CTA per SM / 8 x 8 x 16, the last two through the pass pipeline:
+//   sph 301 60 / 100 / 107, 767 210 / 245 / 294, 1024 328 / 348 / 403, 1500 - / 798 / 668
+//   disk 301 138 / 185 / 219, 512 318 / 320 / 397, 1501 - / 2730 / 2000
+//   tri 301 133 / 134 / 138, 512 310 / 224 / 249, 1001 - / 470 / 509, 2048 - / 2510 / 1650
+//   rect 301 58 / 72 / 73, 1024 319 / 248 / 258
+// The resident kernel wins until its CTAs' own work, which grows with the cube of n on a number of
+// SMs that grows with n, passes what the pipeline spreads over the whole chip: chains of 512
+// positions for two columns an order, 300 for one (half the CTAs for the same work).  Past that,
+// few passes leave the SMs to single warps per sub-partition, which run a pass's steps twice as
+// fast (the launch is then bound by the longest task's passes in turn); from about two passes of
+// 64 sweeps per SM on, throughput counts.
+int default_config(int kind, const RotLaunch & L, RotSchedule * sched, cudaStream_t st) {
+    const bool pair = kind != TRI && kind != RECT;
+    int len = 0;
+    for (int f = 0; f < L.nfields; ++f) len = std::max(len, Geo::chain_len(kind, L.fields[f].N, 0));
+    const RotSchedule::Units * const U = sched && len > (pair ? 512 : 300) ? schedule_passes(sched, kind, L, shape_pass(0), 1, st) : nullptr;
+    if (!U) return 5;             // whole tasks: resident where they fit, else 8 x 8 x 16
+    return 8 + (U->n <= 300 ? 2 : 0);
+}
 
 // The autotuner's choices, by launch shape: family, direction, heads only or all sweeps,
 // fields, tasks, and the first field's N and M (the tasks of a shape are the same).
@@ -793,7 +1164,7 @@ int tune(int kind, bool hi2lo, const RotLaunch & L, double * const * dead, int m
     // spreads a task's passes over SMs: worth it when there are few tasks, not when the
     // columns would leave L2 between passes)
     for (int cfg = 0; cfg < 8 * kPipeModes; ++cfg) {
-        if ((cfg & 7) > 5 || ((kind == TRI || kind == RECT) && (cfg & 7) == 1)) continue;   // tri, rect: shape 1 not built
+        if ((cfg & 7) > 5) continue;
         if ((cfg >> 3) && !sched) continue;
         if (launch_shape(kind, hi2lo, cfg, S, max_ctas, st, sched, prog_call, prog_cap) != cudaSuccess) { best = -1; break; }
         if (cudaEventRecord(e0, st) != cudaSuccess) { best = -1; break; }
@@ -815,7 +1186,7 @@ cudaError_t launch_rotations(int kind, bool hi2lo, const RotLaunch & L, int max_
     if (L.ntasks <= 0) return cudaSuccess;
     int cfg = rotation_config();
     if (cfg < 0) {
-        cfg = default_config(L);
+        cfg = -1;
         if (autotune_enabled() && L.nfields > 0) {
             const std::string key = shape_key(kind, hi2lo, L);
             int known = -1;
@@ -837,6 +1208,7 @@ cudaError_t launch_rotations(int kind, bool hi2lo, const RotLaunch & L, int max_
             }
         }
     }
+    if (cfg < 0) cfg = default_config(kind, L, sched, st);
     return launch_shape(kind, hi2lo, cfg, L, max_ctas, st, sched, prog_call, prog_cap);
 }
 

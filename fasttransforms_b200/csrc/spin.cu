@@ -42,6 +42,7 @@ struct ft_spin_rotation_plan_s {
     double2 * d_sc2 = nullptr;      // (s2, c2) pairs, (l, j, m) at l + j n + m |s| n (src/rotations.c:458-468)
     int * d_counter = nullptr;
     std::map<int, std::pair<ftb::RotTask *, int>> tasks;   // M -> stage-2 tasks, longest first
+    std::map<int, ftb::RotSchedule *> sched;               // M -> pass schedule of that list
     double * d_stage = nullptr;     // host-pointer calls
     size_t stage_elems = 0;
     cudaStream_t stream = nullptr;
@@ -173,6 +174,7 @@ SpinHarmonicPlan * as_sp(const ft_spin_harmonic_plan * P) {
 void destroy_srp(SpinRotPlan * P) {
     if (!P) return;
     for (auto & kv : P->tasks) cudaFree(kv.second.first);
+    for (auto & kv : P->sched) rot_schedule_free(kv.second);
     cudaFree(P->d_sc2);
     cudaFree(P->d_counter);
     cudaFree(P->d_stage);
@@ -212,18 +214,20 @@ SpinRotPlan * make_srp(int n, int s) {
     return P;
 }
 
-// stage-2 tasks for M columns: 16 orders of one parity each, longest first
-bool spin_tasks(SpinRotPlan * P, int M, RotTask ** d, int * nt) {
+// stage-2 tasks for M columns: the columns of orders -m or of orders m of 16 orders of one parity
+// each, longest first
+bool spin_tasks(SpinRotPlan * P, int M, RotTask ** d, int * nt, RotSchedule ** sched) {
     std::lock_guard<std::mutex> lk(P->task_mu);
     auto it = P->tasks.find(M);
-    if (it != P->tasks.end()) { *d = it->second.first; *nt = it->second.second; return true; }
+    if (it != P->tasks.end()) { *d = it->second.first; *nt = it->second.second; *sched = P->sched[M]; return true; }
     const int mlast = Geo::last_order(SPIN, M), as = std::abs(P->s);
     std::vector<std::pair<long long, RotTask>> v;
     for (int p = 0; p < 2; p++)
         for (int mb = p; mb <= mlast; mb += 2 * Geo::task_orders(SPIN)) {
             int jlo, jhi;
             const int nsw = Geo::task_sweeps(SPIN, M, mb, 0, &jlo, &jhi, as);
-            if (nsw > 0) v.push_back({(long long) nsw * (P->n - jlo), RotTask{0, mb}});
+            if (nsw > 0)
+                for (int side = 0; side < 2; side++) v.push_back({(long long) nsw * (P->n - jlo), RotTask{0, mb, side}});
         }
     std::stable_sort(v.begin(), v.end(), [](const auto & a, const auto & b) { return a.first > b.first; });
     std::vector<RotTask> t;
@@ -233,8 +237,10 @@ bool spin_tasks(SpinRotPlan * P, int M, RotTask ** d, int * nt) {
                        !ok(cudaMemcpy(dt, t.data(), sizeof(RotTask) * t.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tasks)")))
         return false;
     P->tasks[M] = {dt, (int) t.size()};
+    P->sched[M] = rot_schedule_new(t);
     *d = dt;
     *nt = (int) t.size();
+    *sched = P->sched[M];
     return true;
 }
 
@@ -248,19 +254,20 @@ bool stage1(SpinRotPlan * P, bool hi2lo, double * A, int M, cudaStream_t st) {
 bool stage2(SpinRotPlan * P, bool hi2lo, double * A, int M, cudaStream_t st) {
     RotTask * dt = nullptr;
     int nt = 0;
-    if (!spin_tasks(P, M, &dt, &nt)) return false;
+    RotSchedule * sched = nullptr;
+    if (!spin_tasks(P, M, &dt, &nt, &sched)) return false;
     if (nt == 0) return true;
     static thread_local RotLaunch L;   // large parameter block; kept off the stack
     L.nfields = 1;
-    L.fields[0] = RotField{A, A, P->sph->d_scp, P->n, M, SPIN, (long long) P->n, 0, std::abs(P->s)};
+    L.fields[0] = RotField{A, A, P->sph->d_skew, P->n, M, SPIN, (long long) P->n, 0, std::abs(P->s)};
     L.tasks = dt;
     L.ntasks = nt;
     L.counter = P->d_counter;
-    L.chains = nullptr;   // no pass pipeline
+    L.chains = nullptr;
     L.nchains = 0;
     L.prog = nullptr;
     prof_begin(FAM_ROT, st);
-    const cudaError_t e = launch_rotations(SPIN, hi2lo, L, 0, st);
+    const cudaError_t e = launch_rotations(SPIN, hi2lo, L, 0, st, nullptr, sched);
     prof_end(st);
     return ok(e, "spin rotation kernel");
 }

@@ -146,7 +146,7 @@ bool build_tri_stage(int N, int L, int M, TriStage * T) {
             const int m = m0 + f;
             for (int mb = std::max(m, 1); mb <= L - 1; mb += 32) {
                 const int omax = std::min(mb + 31, L - 1);
-                v.push_back({(long long) omax * N, RotTask{f, mb}});
+                v.push_back({(long long) omax * N, RotTask{f, mb, 0}});
             }
         }
         std::stable_sort(v.begin(), v.end(), [](const auto & a, const auto & b) { return a.first > b.first; });
@@ -175,7 +175,7 @@ bool tri_sweeps(const ft_rotation_plan * RP1, const TriStage & T, bool hi2lo, do
             const int m = g.m0 + f;
             // column index = order: column l of slab m (order l + m) at base + (l + m) N
             double * base = A + (long long) N * L * m - (long long) N * m;
-            Lr.fields[f] = RotField{base, base, RP1->d_scp, N, L, TRI, (long long) N, 0, 0};
+            Lr.fields[f] = RotField{base, base, RP1->d_skew, N, L, TRI, (long long) N, 0, 0};
         }
         Lr.tasks = g.d_tasks;
         Lr.ntasks = g.ntasks;
