@@ -572,7 +572,8 @@ void rotations_sphv_host(const ft_rotation_plan * RPc, bool hi2lo, double * A, i
 struct TrmmSet {
     TrmmBatchClass * d_classes = nullptr;
     TrmmTile * d_tiles[4] = {nullptr, nullptr, nullptr, nullptr};   // tile order per multiply mode
-    int ntiles = 0;
+    int ntiles[4] = {0, 0, 0, 0};
+    int shape[4] = {0, 0, 0, 0};                   // and their tile shape
 };
 struct BatchCtx {
     RotTask * d_tasks = nullptr;
@@ -611,26 +612,28 @@ bool upload(BatchCtx * B, const std::vector<T> & v, T ** d) {
 
 // tiles of every class, ordered longest K first for each multiply mode
 bool build_trmm_set(BatchCtx * B, const std::vector<TrmmBatchClass> & cls, TrmmSet * T) {
-    const int bm = trmm_tile_rows(), bn = trmm_tile_cols();
-    std::vector<std::pair<long long, TrmmTile>> t[4];
-    for (int c = 0; c < (int) cls.size(); c++) {
-        const TrmmBatchClass & k = cls[c];
-        for (int tm = 0; tm * bm < k.mrows; tm++)
-            for (int tn = 0; tn * bn < k.ncols; tn++) {
-                const TrmmTile x{c, tm, tn};
-                t[0].push_back({(long long) (k.n - tm * bm), x});
-                t[1].push_back({(long long) std::min(k.n, (tm + 1) * bm), x});
-                t[2].push_back({(long long) std::min(k.n, (tn + 1) * bn), x});
-                t[3].push_back({(long long) (k.n - tn * bn), x});
-            }
-    }
     if (!upload(B, cls, &T->d_classes)) return false;
     for (int m = 0; m < 4; m++) {
-        std::stable_sort(t[m].begin(), t[m].end(), [](const auto & a, const auto & b) { return a.first > b.first; });
+        std::vector<TrmmExtent> x;
+        for (const TrmmBatchClass & k : cls) x.push_back({k.mrows, k.ncols, k.n, m});
+        T->shape[m] = trmm_shape(x);
+        int bm, bn;
+        trmm_tile(T->shape[m], &bm, &bn);
+        std::vector<std::pair<int, TrmmTile>> t;
+        for (int c = 0; c < (int) cls.size(); c++) {
+            const TrmmBatchClass & k = cls[c];
+            for (int tm = 0; tm * bm < k.mrows; tm++)
+                for (int tn = 0; tn * bn < k.ncols; tn++) {
+                    const int len = m == 0 ? k.n - tm * bm : m == 1 ? std::min(k.n, (tm + 1) * bm)
+                                  : m == 2 ? std::min(k.n, (tn + 1) * bn) : k.n - tn * bn;
+                    t.push_back({len, TrmmTile{c, tm, tn}});
+                }
+        }
+        std::stable_sort(t.begin(), t.end(), [](const auto & a, const auto & b) { return a.first > b.first; });
         std::vector<TrmmTile> o;
-        for (auto & x : t[m]) o.push_back(x.second);
+        for (auto & e : t) o.push_back(e.second);
         if (!upload(B, o, &T->d_tiles[m])) return false;
-        T->ntiles = (int) o.size();
+        T->ntiles[m] = (int) o.size();
     }
     return true;
 }
@@ -797,7 +800,7 @@ int execute_batch_chunk(HarmonicPlan * const * H, bool forward, char TRANS, doub
         P.classes = T.d_classes;
         P.tiles = T.d_tiles[mode];
         prof_begin(FAM_TRMM, st);
-        const cudaError_t e = launch_trmm_batched(P, T.ntiles, vec, mode, st);
+        const cudaError_t e = launch_trmm_batched(P, T.ntiles[mode], vec, mode, T.shape[mode], st);
         prof_end(st);
         return cuda_ok(e, "trmm kernel");
     };

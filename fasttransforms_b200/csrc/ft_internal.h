@@ -235,9 +235,12 @@ struct TrmmBatch {
     const TrmmTile * tiles;           // device, longest K first
 };
 // mode 0 / 1: Out = U In / U^T In; mode 2 / 3: Out = In U / In U^T
-cudaError_t launch_trmm_batched(const TrmmBatch & P, int ntiles, bool vec16, int mode, cudaStream_t st);
-int trmm_tile_rows();
-int trmm_tile_cols();
+// (shape: the tile shape that the tile list was built for)
+cudaError_t launch_trmm_batched(const TrmmBatch & P, int ntiles, bool vec16, int mode, int shape, cudaStream_t st);
+// Tile shape for the products of one launch, and its size.
+struct TrmmExtent { int mrows, ncols, n, mode; };
+int trmm_shape(const std::vector<TrmmExtent> & x);
+void trmm_tile(int shape, int * rows, int * cols);
 // Right multiply for tri: Out = In * op(U) (rows of In are independent).
 cudaError_t launch_trmm_right(const double * U, const double * in, double * out, int n, int nrows,
                               long long ld, bool trans, cudaStream_t st);

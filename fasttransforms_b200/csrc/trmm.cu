@@ -7,26 +7,81 @@
 // visits the nonzero triangle.  Up to four column classes (the stride-4N
 // classes of sph / disk, each with its own U) share one launch.
 //
-// Tile: 128 x 64 outputs per CTA, 8 warps of 32 x 32, K slabs of 16 staged in
-// shared memory by a 3-deep cp.async pipeline.  Shared layouts are padded so
-// every fragment load is conflict-free.
+// Three tile shapes (TileShape), chosen per launch by trmm_shape: 128 x 64 outputs with 8 warps of
+// 32 x 32 where the tiles fill the chip several times over, 64 x 64 with 4 such warps where they do
+// not, 32 x 32 with 4 warps of 16 x 16 for the smallest.  K slabs of 16 are staged in shared memory
+// by a cp.async pipeline; the layouts are padded so every fragment load is conflict-free.
 //
-// Summation: the accumulators sum one chunk of 256 consecutive k at a time;
-// at the end of each chunk a thread adds them into its outputs in C (which it
-// alone writes) and starts the next chunk from zero.  A single accumulation
-// over all n terms lets the rounding error grow with n; chunked sums, like a
-// BLAS's K panels, keep it near that of 256 terms plus n / 256 additions (the
-// reference's round trips, which amplify this error in the ill-conditioned
-// triangle transforms, then match its BLAS build).  C must not alias the
-// inputs (every caller multiplies out of place).
+// Summation: the accumulators sum one chunk of 256 consecutive k (k / 256 equal) at a time; at the
+// end of each chunk a thread adds them into its outputs in C (which it alone writes) and starts the
+// next chunk from zero.  A single accumulation over all n terms lets the rounding error grow with
+// n; chunked sums, like a BLAS's K panels, keep it near that of 256 terms plus n / 256 additions (the
+// reference's round trips, which amplify this error in the ill-conditioned triangle transforms,
+// then match its BLAS build).  The chunks do not depend on the tile, so every shape gives the same
+// bits.  C must not alias the inputs (every caller multiplies out of place).
+
+#include <algorithm>
+#include <atomic>
+#include <vector>
 
 #include "ft_internal.h"
 
 namespace ftb {
+
+void trmm_tile(int shape, int * rows, int * cols) {
+    static const int r[3] = {128, 64, 32}, c[3] = {64, 64, 32};
+    *rows = r[shape];
+    *cols = c[shape];
+}
+
+// A launch takes about its slabs' time over the SMs plus the tail in which the longest tiles run
+// alone, which is where the smaller tiles win: they are more and shorter, but load more per flop.
+// Per slab of 16 k, in us: with the chip full, 1.30, 0.67 and 0.18 (128 x 64, 64 x 64, 32 x 32: 29.0,
+// 28.3 and 26.0 TFLOP/s at sph degree 4095); of the longest tile, 0.75, 0.55 and 0.4.  Measured per
+// launch (us; 128 x 64 / 64 x 64 / 32 x 32): sph 64 13 / 11 / 8, 301 50 / 39 / 18, 512 56 / 39 / 24,
+// 1024 135 / 114 / 95, 1501 347 / 317 / 348, 2048 633 / 630 / 673, 4096 4752 / 4837 / 5250; tri 1001
+// 132 / 106 / 69, 2048 349 / 332 / 339.
+int trmm_shape(const std::vector<TrmmExtent> & x) {
+    static const double full[3] = {1.30, 0.67, 0.184}, tail[3] = {0.75, 0.55, 0.4};
+    int best = 0;
+    double least = 0.0;
+    for (int s = 0; s < 3; ++s) {
+        int bm, bn;
+        trmm_tile(s, &bm, &bn);
+        double slabs = 0.0, longest = 0.0;
+        for (const TrmmExtent & e : x) {
+            const int tm = (e.mrows + bm - 1) / bm, tn = (e.ncols + bn - 1) / bn;
+            // a tile's K runs from its place on the diagonal to the matrix's end: half of it on average
+            slabs += 0.5 * tm * tn * (e.n + (e.mode < 2 ? bm : bn)) / 16.0;
+            longest = std::max(longest, e.n / 16.0);
+        }
+        const double t = slabs * full[s] / 148.0 + longest * tail[s];
+        if (s == 0 || t < least) { least = t; best = s; }
+    }
+    return best;
+}
+
 namespace {
 
-constexpr int BM = 128, BN = 64, BK = 16, NSTAGE = 3, NTHREADS = 256;
-constexpr int KCHUNK_SLABS = 16;   // slabs of BK summed before a partial sum is added into C
+constexpr int BK = 16;
+constexpr int KCHUNK = 256;   // consecutive k summed before a partial sum is added into C
+
+template <int S> struct TileShape;
+template <> struct TileShape<0> { static constexpr int BM = 128, BN = 64, WM = 32, WN = 32, STAGES = 3, CTAS = 2; };
+template <> struct TileShape<1> { static constexpr int BM = 64, BN = 64, WM = 32, WN = 32, STAGES = 3, CTAS = 3; };
+template <> struct TileShape<2> { static constexpr int BM = 32, BN = 32, WM = 16, WN = 16, STAGES = 4, CTAS = 5; };
+
+template <int S, bool A_MC, bool B_KC>
+struct TileLayout : TileShape<S> {
+    using T = TileShape<S>;
+    static constexpr int THREADS = 32 * (T::BM / T::WM) * (T::BN / T::WN);
+    static constexpr int FA = T::WM / 8, FB = T::WN / 8;             // fragments of a warp
+    static constexpr int LDA = A_MC ? T::BM + 4 : BK + 4;            // [k][m] or [m][k]
+    static constexpr int LDB = B_KC ? BK + 4 : T::BN + 4;            // [n][k] or [k][n]
+    static constexpr int ASZ = A_MC ? BK * LDA : T::BM * LDA;
+    static constexpr int BSZ = B_KC ? T::BN * LDB : BK * LDB;
+    static constexpr size_t bytes = sizeof(double) * T::STAGES * (ASZ + BSZ);
+};
 
 __device__ __forceinline__ void cp_async16(void * smem, const void * gmem, bool valid) {
     unsigned sa = (unsigned) __cvta_generic_to_shared(smem);
@@ -63,17 +118,18 @@ struct GemmParams {
     int mode;           // 0: left N (k >= i), 1: left T (k <= i), 2: right N (k <= j), 3: right T (k >= j)
 };
 
-// A thread's 32 accumulators (rows m0 + 8a, columns n0 + 8b + {0, 1}) into C:
+// A thread's accumulators (rows m0 + 8a, columns n0 + 8b + {0, 1}) into C:
 // C = acc (first chunk) or C + acc, then acc = 0 when more chunks follow.  All
 // loads are issued before any store, so they are in flight together.
-__device__ __forceinline__ void flush_partial(const GemmClass & C, const int m0, const int n0, double (&acc)[4][4][2],
+template <int FA, int FB>
+__device__ __forceinline__ void flush_partial(const GemmClass & C, const int m0, const int n0, double (&acc)[FA][FB][2],
                                               const bool add, const bool restart) {
     if (add) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < FA; ++a) {
             const int m = m0 + a * 8;
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
+            for (int b = 0; b < FB; ++b) {
                 const int nn = n0 + b * 8;
                 if (m < C.mrows && nn < C.ncols) acc[a][b][0] += C.c[(long long) nn * C.c_ld + m];
                 if (m < C.mrows && nn + 1 < C.ncols) acc[a][b][1] += C.c[(long long) (nn + 1) * C.c_ld + m];
@@ -81,10 +137,10 @@ __device__ __forceinline__ void flush_partial(const GemmClass & C, const int m0,
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+    for (int a = 0; a < FA; ++a) {
         const int m = m0 + a * 8;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < FB; ++b) {
             const int nn = n0 + b * 8;
             if (m < C.mrows && nn < C.ncols) C.c[(long long) nn * C.c_ld + m] = acc[a][b][0];
             if (m < C.mrows && nn + 1 < C.ncols) C.c[(long long) (nn + 1) * C.c_ld + m] = acc[a][b][1];
@@ -93,13 +149,12 @@ __device__ __forceinline__ void flush_partial(const GemmClass & C, const int m0,
     }
 }
 
-// One 128 x 64 output tile of class C: rows [tm*BM, ...), columns [tn*BN, ...).
-template <bool A_MC, bool B_KC, bool VEC16>
+// One output tile of class C: rows [tm*BM, ...), columns [tn*BN, ...).
+template <int S, bool A_MC, bool B_KC, bool VEC16>
 __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const int mode, const int tm, const int tn) {
-    constexpr int LDA = A_MC ? BM + 4 : BK + 4;   // [k][m] or [m][k]
-    constexpr int LDB = B_KC ? BK + 4 : BN + 4;   // [n][k] or [k][n]
-    constexpr int ASZ = A_MC ? BK * LDA : BM * LDA;
-    constexpr int BSZ = B_KC ? BN * LDB : BK * LDB;
+    using T = TileLayout<S, A_MC, B_KC>;
+    constexpr int BM = T::BM, BN = T::BN, NSTAGE = T::STAGES, NTHREADS = T::THREADS, FA = T::FA, FB = T::FB, LDA = T::LDA, LDB = T::LDB,
+                  ASZ = T::ASZ, BSZ = T::BSZ;
     extern __shared__ double sm[];
     double * As = sm;
     double * Bs = sm + NSTAGE * ASZ;
@@ -114,7 +169,7 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
     const int nslab = (khi - klo + BK - 1) / BK;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = warp / (BN / T::WN) * T::WM, wn = warp % (BN / T::WN) * T::WN;
 
     auto load_slab = [&](int slab, int stage) {
         const int k0 = klo + slab * BK;
@@ -174,11 +229,11 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
         }
     };
 
-    double acc[4][4][2];
+    double acc[FA][FB][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < FA; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+        for (int b = 0; b < FB; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
     bool flushed = false;   // C holds the sum of the chunks before the current one
 
 #pragma unroll
@@ -199,23 +254,23 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
         const double * bs = Bs + (slab % NSTAGE) * BSZ;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 4) {
-            double af[4], bf[4];
+            double af[FA], bf[FB];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
+            for (int a = 0; a < FA; ++a) {
                 const int m = wm + a * 8 + fr, k = kk + fc;
                 af[a] = A_MC ? as[k * LDA + m] : as[m * LDA + k];
             }
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
+            for (int b = 0; b < FB; ++b) {
                 const int nn = wn + b * 8 + fr, k = kk + fc;
                 bf[b] = B_KC ? bs[nn * LDB + k] : bs[k * LDB + nn];
             }
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < FA; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
+                for (int b = 0; b < FB; ++b) dmma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
         }
-        if ((slab + 1) % KCHUNK_SLABS == 0 && slab + 1 < nslab) {   // end of a chunk: into C, restart from zero
+        if ((klo + (slab + 1) * BK) % KCHUNK == 0 && slab + 1 < nslab) {   // end of a chunk: into C, restart from zero
             flush_partial(C, i0 + wm + fr, j0 + wn + fc * 2, acc, flushed, true);
             flushed = true;
         }
@@ -226,27 +281,23 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
     flush_partial(C, i0 + wm + fr, j0 + wn + fc * 2, acc, flushed, false);
 }
 
-template <bool A_MC, bool B_KC, bool VEC16>
-__global__ void __launch_bounds__(NTHREADS, 2)
+template <int S, bool A_MC, bool B_KC, bool VEC16>
+__global__ void __launch_bounds__(TileLayout<S, A_MC, B_KC>::THREADS, TileShape<S>::CTAS)
 gemm_tri_kernel(const __grid_constant__ GemmParams P) {
-    // block -> (class, tile m, tile n); tiles with the most K work first
-    int bid = blockIdx.x;
-    const int per_class = P.tiles_m * P.tiles_n;
-    const int cl = bid / per_class;
-    bid -= cl * per_class;
-    int tm, tn;
-    if (P.mode == 0)      { tm = bid / P.tiles_n; tn = bid % P.tiles_n; }                 // small i: long K
-    else if (P.mode == 1) { tm = P.tiles_m - 1 - bid / P.tiles_n; tn = bid % P.tiles_n; } // large i: long K
-    else if (P.mode == 2) { tn = P.tiles_n - 1 - bid / P.tiles_m; tm = bid % P.tiles_m; } // large j
-    else                  { tn = bid / P.tiles_m; tm = bid % P.tiles_m; }                 // small j
-    tri_tile<A_MC, B_KC, VEC16>(P.cls[cl], P.n, P.mode, tm, tn);
+    // block -> (tile along the triangle, class, other tile): tiles with the most K work first,
+    // whatever their class
+    const int along = P.mode < 2 ? P.tiles_m : P.tiles_n, across = P.mode < 2 ? P.tiles_n : P.tiles_m;
+    int t = blockIdx.x / (P.nclasses * across);
+    const int rest = blockIdx.x % (P.nclasses * across), cl = rest / across, x = rest % across;
+    if (P.mode == 1 || P.mode == 2) t = along - 1 - t;   // long K at large i (j); else at small i (j)
+    tri_tile<S, A_MC, B_KC, VEC16>(P.cls[cl], P.n, P.mode, P.mode < 2 ? t : x, P.mode < 2 ? x : t);
 }
 
 // Batched multiplies over many fields: the tile list (longest K first) and the
 // pointer-free class table live in device memory; pointers come by value.
 // MODE 0/1: left, op(U) = U / U^T; MODE 2/3: right, op(U) = U / U^T.
-template <int MODE, bool VEC16>
-__global__ void __launch_bounds__(NTHREADS, 2)
+template <int S, int MODE, bool VEC16>
+__global__ void __launch_bounds__(TileLayout<S, MODE != 1, MODE != 3>::THREADS, TileShape<S>::CTAS)
 gemm_tri_batched_kernel(const __grid_constant__ TrmmBatch P) {
     const TrmmTile t = P.tiles[blockIdx.x];
     const TrmmBatchClass c = P.classes[t.cls];
@@ -259,59 +310,57 @@ gemm_tri_batched_kernel(const __grid_constant__ TrmmBatch P) {
     C.ncols = c.ncols;
     if (MODE < 2) { C.a = U; C.a_ld = c.n; C.b = X; C.b_ld = c.ld; }
     else          { C.a = X; C.a_ld = c.ld; C.b = U; C.b_ld = c.n; }
-    constexpr bool A_MC = MODE != 1;
-    constexpr bool B_KC = MODE != 3;
-    tri_tile<A_MC, B_KC, VEC16>(C, c.n, MODE, t.tm, t.tn);
+    tri_tile<S, MODE != 1, MODE != 3, VEC16>(C, c.n, MODE, t.tm, t.tn);
 }
 
-template <int MODE>
-cudaError_t run_batched(const TrmmBatch & P, int ntiles, bool vec16, cudaStream_t st) {
-    constexpr bool A_MC = MODE != 1;
-    constexpr bool B_KC = MODE != 3;
-    constexpr int LDA = A_MC ? BM + 4 : BK + 4;
-    constexpr int LDB = B_KC ? BK + 4 : BN + 4;
-    constexpr int ASZ = A_MC ? BK * LDA : BM * LDA;
-    constexpr int BSZ = B_KC ? BN * LDB : BK * LDB;
-    const size_t shm = sizeof(double) * NSTAGE * (ASZ + BSZ);
-    cudaError_t e;
-    if (vec16) {
-        auto k = gemm_tri_batched_kernel<MODE, true>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
+// One launch; the kernel's shared-memory limit is raised once per device.
+template <class K, class P>
+cudaError_t launch_tiles(K kern, const P & p, int blocks, int threads, size_t shm, std::atomic<unsigned> & ready, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned bit = dev < 32 ? 1u << dev : 0u;
+    if (!(ready.load(std::memory_order_acquire) & bit)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
         if (e != cudaSuccess) return e;
-        k<<<ntiles, NTHREADS, shm, st>>>(P);
-    } else {
-        auto k = gemm_tri_batched_kernel<MODE, false>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
-        if (e != cudaSuccess) return e;
-        k<<<ntiles, NTHREADS, shm, st>>>(P);
+        ready.fetch_or(bit, std::memory_order_release);
     }
+    kern<<<blocks, threads, shm, st>>>(p);
     count_launch();
     return cudaGetLastError();
 }
 
-template <bool A_MC, bool B_KC>
-cudaError_t run_gemm(const GemmParams & P, bool vec16, cudaStream_t st) {
-    constexpr int LDA = A_MC ? BM + 4 : BK + 4;
-    constexpr int LDB = B_KC ? BK + 4 : BN + 4;
-    constexpr int ASZ = A_MC ? BK * LDA : BM * LDA;
-    constexpr int BSZ = B_KC ? BN * LDB : BK * LDB;
-    const size_t shm = sizeof(double) * NSTAGE * (ASZ + BSZ);
+template <int S, int MODE, bool VEC16>
+cudaError_t run_batched(const TrmmBatch & P, int ntiles, cudaStream_t st) {
+    using T = TileLayout<S, MODE != 1, MODE != 3>;
+    static std::atomic<unsigned> ready{0};
+    return launch_tiles(gemm_tri_batched_kernel<S, MODE, VEC16>, P, ntiles, T::THREADS, T::bytes, ready, st);
+}
+template <int MODE>
+cudaError_t run_batched(const TrmmBatch & P, int ntiles, bool vec16, int shape, cudaStream_t st) {
+    if (shape == 0) return vec16 ? run_batched<0, MODE, true>(P, ntiles, st) : run_batched<0, MODE, false>(P, ntiles, st);
+    if (shape == 1) return vec16 ? run_batched<1, MODE, true>(P, ntiles, st) : run_batched<1, MODE, false>(P, ntiles, st);
+    return vec16 ? run_batched<2, MODE, true>(P, ntiles, st) : run_batched<2, MODE, false>(P, ntiles, st);
+}
+
+template <int S, bool A_MC, bool B_KC, bool VEC16>
+cudaError_t run_gemm(GemmParams P, int rows, int cols, cudaStream_t st) {
+    using T = TileLayout<S, A_MC, B_KC>;
+    P.tiles_m = (rows + T::BM - 1) / T::BM;
+    P.tiles_n = (cols + T::BN - 1) / T::BN;
     const int blocks = P.nclasses * P.tiles_m * P.tiles_n;
     if (blocks == 0) return cudaSuccess;
-    cudaError_t e;
-    if (vec16) {
-        auto k = gemm_tri_kernel<A_MC, B_KC, true>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
-        if (e != cudaSuccess) return e;
-        k<<<blocks, NTHREADS, shm, st>>>(P);
-    } else {
-        auto k = gemm_tri_kernel<A_MC, B_KC, false>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
-        if (e != cudaSuccess) return e;
-        k<<<blocks, NTHREADS, shm, st>>>(P);
-    }
-    count_launch();
-    return cudaGetLastError();
+    static std::atomic<unsigned> ready{0};
+    return launch_tiles(gemm_tri_kernel<S, A_MC, B_KC, VEC16>, P, blocks, T::THREADS, T::bytes, ready, st);
+}
+template <bool A_MC, bool B_KC>
+cudaError_t run_gemm(const GemmParams & P, int rows, int cols, bool vec16, cudaStream_t st) {
+    std::vector<TrmmExtent> x;
+    for (int c = 0; c < P.nclasses; ++c) x.push_back({P.cls[c].mrows, P.cls[c].ncols, P.n, P.mode});
+    const int shape = trmm_shape(x);
+    if (shape == 0) return vec16 ? run_gemm<0, A_MC, B_KC, true>(P, rows, cols, st) : run_gemm<0, A_MC, B_KC, false>(P, rows, cols, st);
+    if (shape == 1) return vec16 ? run_gemm<1, A_MC, B_KC, true>(P, rows, cols, st) : run_gemm<1, A_MC, B_KC, false>(P, rows, cols, st);
+    return vec16 ? run_gemm<2, A_MC, B_KC, true>(P, rows, cols, st) : run_gemm<2, A_MC, B_KC, false>(P, rows, cols, st);
 }
 
 inline bool aligned16(const void * p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -344,25 +393,21 @@ cudaError_t launch_trmm(const TrmmLaunch & L, cudaStream_t st) {
         maxcols = std::max(maxcols, g.ncols);
         vec = vec && aligned16(g.a) && aligned16(g.b);
     }
-    P.tiles_m = (L.n + BM - 1) / BM;
-    P.tiles_n = (maxcols + BN - 1) / BN;
     P.mode = L.trans ? 1 : 0;
-    return L.trans ? run_gemm<false, true>(P, vec, st) : run_gemm<true, true>(P, vec, st);
+    return L.trans ? run_gemm<false, true>(P, L.n, maxcols, vec, st) : run_gemm<true, true>(P, L.n, maxcols, vec, st);
 }
 
-cudaError_t launch_trmm_batched(const TrmmBatch & P, int ntiles, bool vec16, int mode, cudaStream_t st) {
+cudaError_t launch_trmm_batched(const TrmmBatch & P, int ntiles, bool vec16, int mode, int shape, cudaStream_t st) {
     if (ntiles == 0) return cudaSuccess;
     switch (mode) {
-        case 0: return run_batched<0>(P, ntiles, vec16, st);
-        case 1: return run_batched<1>(P, ntiles, vec16, st);
-        case 2: return run_batched<2>(P, ntiles, vec16, st);
-        case 3: return run_batched<3>(P, ntiles, vec16, st);
+        case 0: return run_batched<0>(P, ntiles, vec16, shape, st);
+        case 1: return run_batched<1>(P, ntiles, vec16, shape, st);
+        case 2: return run_batched<2>(P, ntiles, vec16, shape, st);
+        case 3: return run_batched<3>(P, ntiles, vec16, shape, st);
     }
     return cudaErrorInvalidValue;
 }
 
-int trmm_tile_rows() { return BM; }
-int trmm_tile_cols() { return BN; }
 
 cudaError_t launch_trmm_right(const double * U, const double * in, double * out, int n, int nrows,
                               long long ld, bool trans, cudaStream_t st) {
@@ -374,12 +419,10 @@ cudaError_t launch_trmm_right(const double * U, const double * in, double * out,
     g.a = in; g.b = U; g.c = out;
     g.a_ld = ld; g.b_ld = n; g.c_ld = ld;
     g.mrows = nrows; g.ncols = n;
-    P.tiles_m = (nrows + BM - 1) / BM;
-    P.tiles_n = (n + BN - 1) / BN;
     P.mode = trans ? 3 : 2;
     const bool vec = (n % 2 == 0) && (ld % 2 == 0) && aligned16(in) && aligned16(U);
     // op(U) = U: B(k, j) = U[k + j n] contiguous in k; op(U) = U^T: B(k, j) = U[j + k n] contiguous in j
-    return trans ? run_gemm<true, false>(P, vec, st) : run_gemm<true, true>(P, vec, st);
+    return trans ? run_gemm<true, false>(P, nrows, n, vec, st) : run_gemm<true, true>(P, nrows, n, vec, st);
 }
 
 cudaError_t launch_cheb_normalize(double * A, int N, int M, long long lda, bool transposed, cudaStream_t st) {
