@@ -167,8 +167,8 @@ __device__ __forceinline__ void wait_bar(uint64_t * bar, uint32_t parity) {
 
 // Asynchronous 8-byte copy global -> shared (0 bytes read, zeros written when !valid), and the
 // arrival of this thread on a barrier once its copies so far have landed.
-__device__ __forceinline__ void copy_async8(double * dst, const double * src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(tc::smem_addr(dst)), "l"(src), "r"(valid ? 8 : 0) : "memory");
+__device__ __forceinline__ void copy_async8(uint32_t dst, const double * src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
 __device__ __forceinline__ void copy_async_arrive(uint64_t * bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" :: "r"(tc::smem_addr(bar)) : "memory");
@@ -218,8 +218,9 @@ struct TaskGeo {
     }
 };
 
-// The elements of one chunk as a warp moves them between global memory and a ring slot: element v
-// of a lane is double rr(v) of the contiguous E * CH * ES doubles of column segment seg(v).
+// The elements of one chunk as a warp moves them between global memory and a ring slot.  A column's
+// part of a chunk is a segment of E * CH * ES consecutive doubles; a lane takes, in each of PH
+// phases, the same double of every SSTEP-th segment, so that its addresses advance by constants.
 template <int KIND, bool HI2LO, int E>
 struct Mover {
     using T = KT<KIND>;
@@ -228,15 +229,21 @@ struct Mover {
     static constexpr int PER = T::COLS * E * T::CH / 32;           // elements of a lane
     static constexpr int RB = RPC >= 32 ? RPC / 32 : 1;            // instructions per segment
     static constexpr int SP = RPC >= 32 ? 1 : 32 / RPC;            // segments per instruction
+    static constexpr bool PAIRED = KIND == SPH || KIND == DISK;    // two columns an order, side by side
+    static constexpr int PH = RB > 1 ? RB : (PAIRED && SP == 1) ? 2 : 1;
+    static constexpr int NV = PER / PH;                            // elements of a lane in a phase
+    static constexpr int SSTEP = RB > 1 ? 1 : SP * PH;
+    static constexpr int SLOT_STEP = SSTEP * T::ES;                // ring slot doubles between them
     static_assert(RPC % 32 == 0 || 32 % RPC == 0, "a segment must split evenly over the lanes");
-    long long base;     // double offset of this lane's element 0 at chain position 0
+    static_assert(!PAIRED || SSTEP % 2 == 0, "a lane's segments must be whole orders apart");
+    long long base;     // double offset, at chain position 0, of the column of this lane's segment 0
     long long lda2;     // doubles between columns
-    int nseg;           // valid segments of the task, less this lane's own
-    int seg0;           // first valid one, less this lane's own (spin: order 0 has one column)
+    int nseg, seg0;     // the task's valid segments, less this lane's own (spin: order 0 has one column)
     int N, lane;
     __host__ __device__ __forceinline__ static int lane_seg(int lane) { return RPC < 32 ? lane / RPC : 0; }
-    __host__ __device__ __forceinline__ static int rr(int v, int lane) { return RPC >= 32 ? (v % RB) * 32 + lane : lane % RPC; }
-    // columns from segment s's column to the task's first column
+    __host__ __device__ __forceinline__ static int rr(int ph, int lane) { return RB > 1 ? ph * 32 + lane : lane % RPC; }
+    __host__ __device__ __forceinline__ static constexpr int seg(int ph) { return RB > 1 ? 0 : ph * SP; }
+    // columns from the task's first one to segment s's
     __host__ __device__ __forceinline__ static constexpr int col_of(int s) {
         return KIND == TRI ? s : KIND == RECT ? 2 * s : KIND == SPIN ? 4 * s : 4 * (s >> 1) + (s & 1);
     }
@@ -256,23 +263,27 @@ struct Mover {
             const long long most = (F.M - 1 - col0) / 4 + 1;
             if (nseg + ls > most) nseg = (int) most - ls;
         } else col0 = 2LL * t.mbase - 1;
-        // SP > 1 with paired columns: a lane's segments differ from its first by whole orders
         base = (col0 + col_of(ls)) * lda2;
     }
-    __host__ __device__ __forceinline__ bool seg_ok(int v) const { const int s = (v / RB) * SP; return s < nseg && s >= seg0; }
-    __host__ __device__ __forceinline__ bool row_ok(int v, int pmin, int emax) const {
-        const int r = rr(v, lane), p = pmin + r / (T::ES * T::CH);
+    // element v of phase ph belongs to a column of the task
+    __host__ __device__ __forceinline__ bool seg_ok(int ph, int v) const {
+        const int s = seg(ph) + v * SSTEP;
+        return s < nseg && s >= seg0;
+    }
+    __host__ __device__ __forceinline__ bool row_ok(int ph, int pmin, int emax) const {
+        const int r = rr(ph, lane), p = pmin + r / (T::ES * T::CH);
         return p >= 0 && p <= emax && T::CH * p + (r / T::ES) % T::CH < N;
     }
-    // double offset of element v of the chunk that starts at position pmin
-    __host__ __device__ __forceinline__ long long at(int v, int pmin) const {
-        return base + (long long) col_of((v / RB) * SP) * lda2 + (long long) T::ES * T::CH * pmin + rr(v, lane);
+    // double offset of element 0 of a phase in the chunk that starts at position pmin, and between elements
+    __host__ __device__ __forceinline__ long long at(int ph, int pmin) const {
+        return base + (long long) col_of(seg(ph)) * lda2 + (long long) T::ES * T::CH * pmin + rr(ph, lane);
     }
-    // its place in a ring slot
-    __host__ __device__ __forceinline__ int slot_at(int v) const {
-        const int r = rr(v, lane), pos = r / (T::ES * T::CH), c = (r / T::ES) % T::CH, part = r % T::ES;
+    __host__ __device__ __forceinline__ long long step() const { return (long long) col_of(SSTEP) * lda2; }
+    // place of element 0 of a phase in a ring slot
+    __host__ __device__ __forceinline__ int slot_at(int ph) const {
+        const int r = rr(ph, lane), pos = r / (T::ES * T::CH), c = (r / T::ES) % T::CH, part = r % T::ES;
         const int u = HI2LO ? E - 1 - pos : pos;
-        return (u * T::CH + c) * T::CPAD + ((v / RB) * SP + lane_seg(lane)) * T::ES + part;
+        return (u * T::CH + c) * T::CPAD + (seg(ph) + lane_seg(lane)) * T::ES + part;
     }
 };
 
@@ -609,11 +620,17 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const unsigned n = n0 + i;
                     const int pmin = P.pmin(i);
                     wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1);
-                    double * const slot = rings + (size_t) (n % SL) * SLOT;
+                    const uint32_t slot = tc::smem_addr(rings + (size_t) (n % SL) * SLOT);
+#pragma unroll 1
+                    for (int ph = 0; ph < MV::PH; ++ph) {
+                        const bool ok = mv.row_ok(ph, pmin, P.emax);
+                        const double * g = src + mv.at(ph, pmin);
+                        uint32_t sa = slot + 8u * mv.slot_at(ph);
 #pragma unroll 4
-                    for (int v = 0; v < MV::PER; ++v) {
-                        const bool valid = mv.seg_ok(v) && mv.row_ok(v, pmin, P.emax);
-                        copy_async8(slot + mv.slot_at(v), valid ? src + mv.at(v, pmin) : src, valid);
+                        for (int v = 0; v < MV::NV; ++v, g += mv.step(), sa += 8u * MV::SLOT_STEP) {
+                            const bool valid = ok && mv.seg_ok(ph, v);
+                            copy_async8(sa, valid ? g : src, valid);
+                        }
                     }
                     copy_async_arrive(&full[n % SL]);
                 };
@@ -650,12 +667,18 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const int pmin = P.pmin(i);
                     wait_bar(&bfull[n % SL], (n / SL) & 1);
                     const double * const slot = ring + (n % SL) * SLOT;
+#pragma unroll 1
+                    for (int ph = 0; ph < MV::PH; ++ph) {
+                        if (!mv.row_ok(ph, pmin, P.emax)) continue;
+                        double * g = F.out + mv.at(ph, pmin);
+                        const double * x = slot + mv.slot_at(ph);
 #pragma unroll 4
-                    for (int v = 0; v < MV::PER; ++v)
-                        if (mv.seg_ok(v) && mv.row_ok(v, pmin, P.emax)) __stcg(F.out + mv.at(v, pmin), slot[mv.slot_at(v)]);
+                        for (int v = 0; v < MV::NV; ++v, g += mv.step(), x += MV::SLOT_STEP)
+                            if (mv.seg_ok(ph, v)) __stcg(g, *x);
+                    }
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&bempt[n % SL]);
-                    if (++since < every && i + 1 < P.nchunk) continue;
+                    if (r + 1 == G.npass || (++since < every && i + 1 < P.nchunk)) continue;   // no pass follows the last
                     since = 0;
                     __syncwarp();
                     if (lane == 0) {
@@ -1114,6 +1137,7 @@ cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int
 // fast (the launch is then bound by the longest task's passes in turn); from about two passes of
 // 64 sweeps per SM on, throughput counts.
 int default_config(int kind, const RotLaunch & L, RotSchedule * sched, cudaStream_t st) {
+    if (L.nfields > 0 && L.fields[0].blk > 0) return 4;   // at most 31 sweeps a column: one pass of 4 x 8
     const bool pair = kind != TRI && kind != RECT;
     int len = 0;
     for (int f = 0; f < L.nfields; ++f) len = std::max(len, Geo::chain_len(kind, L.fields[f].N, 0));
