@@ -173,18 +173,20 @@ struct CallScratch {
     int prog_cap = 0;
 };
 
+// before: columns in front of in and out that an out-of-place call copies too
 bool rotations(ft_rotation_plan * RP, bool hi2lo, const double * in, double * out, int M, long long lda, cudaStream_t st,
-               const CallScratch * cs = nullptr) {
+               const CallScratch * cs = nullptr, int before = 0) {
     RotTask * d_tasks = nullptr;
     int ntasks = 0;
     if (!get_tasks(RP, M, &d_tasks, &ntasks)) return false;
-    if (in != out) {
-        const int nc = untouched_cols(RP->kind, M);
-        if (!cuda_ok(cudaMemcpy2DAsync(out, lda * sizeof(double), in, lda * sizeof(double), RP->n * sizeof(double), nc,
-                                       cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync")) return false;
-    }
-    if (ntasks == 0) return true;
+    const int nc = untouched_cols(RP->kind, M);
+    if (ntasks == 0)   // no launch to copy them
+        return in == out || cuda_ok(cudaMemcpy2DAsync(out - before * lda, lda * sizeof(double), in - before * lda, lda * sizeof(double),
+                                                      RP->n * sizeof(double), nc + before, cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync");
     static thread_local RotLaunch L;   // large parameter block; kept off the stack
+    L.lead0 = -before;
+    L.lead = nc;
+    L.counter0 = 0;
     L.nfields = 1;
     L.fields[0] = RotField{in, out, RP->d_skew, RP->n, M, RP->kind, lda, 0};
     L.tasks = d_tasks;
@@ -210,11 +212,10 @@ bool rotations(ft_rotation_plan * RP, bool hi2lo, const double * in, double * ou
 // later and has M - 2 columns; columns 0 and 1 are left alone.
 bool rotations_sphv(ft_rotation_plan * RP, bool hi2lo, const double * in, double * out, int M, long long lda,
                     cudaStream_t st, const CallScratch * cs = nullptr) {
-    const int lead = std::min(M, 2);
-    if (in != out && !cuda_ok(cudaMemcpy2DAsync(out, lda * sizeof(double), in, lda * sizeof(double), RP->n * sizeof(double),
-                                                lead, cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync")) return false;
-    if (M <= 2) return true;
-    return rotations(RP, hi2lo, in + 2 * lda, out + 2 * lda, M - 2, lda, st, cs);
+    if (M <= 2)
+        return in == out || cuda_ok(cudaMemcpy2DAsync(out, lda * sizeof(double), in, lda * sizeof(double), RP->n * sizeof(double), M,
+                                                      cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync");
+    return rotations(RP, hi2lo, in + 2 * lda, out + 2 * lda, M - 2, lda, st, cs, 2);
 }
 
 // sph and disk: order m occupies the column pair (2m - 1, 2m) for m = 2 .. M/2
@@ -285,7 +286,8 @@ bool trmm_right(const double * U, const double * in, double * out, int N, long l
 
 bool normalize(double * A, int N, int M, long long lda, bool transposed, cudaStream_t st) {
     prof_begin(FAM_OTHER, st);
-    const cudaError_t e = launch_cheb_normalize(A, N, M, lda, transposed, st);
+    (void) lda;   // the matrices are contiguous
+    const cudaError_t e = launch_cheb_normalize(&A, &N, &M, 1, transposed, st);
     prof_end(st);
     return cuda_ok(e, "normalize");
 }
@@ -743,12 +745,13 @@ int execute_batch_chunk(HarmonicPlan * const * H, bool forward, char TRANS, doub
             const double * in = from_A ? A[f] : S[f];
             double * out = to_A ? A[f] : S[f];
             L.fields[f] = RotField{in, out, H[f]->rp_arr[0]->d_skew, N[f], M[f], H[f]->kind, (long long) N[f], blk};
-            if (in != out) {
-                const int nc = untouched_cols(H[f]->kind, M[f]);
-                if (!cuda_ok(cudaMemcpy2DAsync(out, N[f] * sizeof(double), in, N[f] * sizeof(double), N[f] * sizeof(double), nc,
-                                               cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync")) return false;
-            }
+            if (in != out && B->ntasks == 0 &&    // no launch to copy them
+                !cuda_ok(cudaMemcpy2DAsync(out, N[f] * sizeof(double), in, N[f] * sizeof(double), N[f] * sizeof(double),
+                                           untouched_cols(kind, M[f]), cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync")) return false;
         }
+        L.lead0 = 0;
+        L.lead = untouched_cols(kind, 1 << 30);
+        L.counter0 = 0;
         L.tasks = B->d_tasks;
         L.ntasks = B->ntasks;
         L.counter = B->d_counter;
@@ -805,13 +808,10 @@ int execute_batch_chunk(HarmonicPlan * const * H, bool forward, char TRANS, doub
         return cuda_ok(e, "trmm kernel");
     };
     auto norm = [&](bool on_A, bool transposed) -> bool {
-        for (int f = 0; f < nf; f++) {
-            prof_begin(FAM_OTHER, st);
-            const cudaError_t e = launch_cheb_normalize(on_A ? A[f] : S[f], N[f], M[f], N[f], transposed, st);
-            prof_end(st);
-            if (!cuda_ok(e, "normalize")) return false;
-        }
-        return true;
+        prof_begin(FAM_OTHER, st);
+        const cudaError_t e = launch_cheb_normalize(on_A ? A : S.data(), N, M, nf, transposed, st);
+        prof_end(st);
+        return cuda_ok(e, "normalize");
     };
     // blocked products of the whole blocks, in place on the scratch matrices (on_A: on A)
     auto blocks = [&](bool hi2lo, bool on_A = false) -> bool {

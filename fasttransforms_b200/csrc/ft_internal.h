@@ -170,6 +170,10 @@ struct RotLaunch {
     const RotTask * tasks;     // device, longest first
     int ntasks;
     int * counter;             // device work counter (reset by the launcher)
+    int counter0;              // its value after the reset
+    // columns lead0 .. lead - 1 of every field have no sweeps (orders 0 and 1, and what lies before
+    // them): an out-of-place launch copies them from in to out
+    int lead0, lead;
     // Pass pipeline (null chains: each CTA runs every pass of a task itself).  Queue entry c
     // runs passes first, first + stride, ... of task chains[c].task (the launcher queues one
     // pass per entry); pass r streams down the columns behind pass r - 1 of the same task,
@@ -185,12 +189,15 @@ struct RotChain { int task, prog0, first, stride; };
 struct RotSchedule;
 RotSchedule * rot_schedule_new(const std::vector<RotTask> & tasks);
 void rot_schedule_free(RotSchedule * s);
+// The progress words of a launch follow its work counter at this distance (in words), so that one
+// fill resets both.
+constexpr int kProgLead = 64;
 int rotation_device_error();   // reads and clears the rotation kernel's status word (-1: read failed)
 // dead: per field, memory the caller has no live data in (N x M at the field's leading
 // dimension), or null.  With it, the first launch of a shape times every configuration
 // there and keeps the fastest for the shape (the autotuner; FT_B200_AUTOTUNE=0 turns it off).
 // sched: the task list's schedule (null: no pass pipeline).  prog_call: progress words of the
-// calling execute (prog_cap of them) for the pass pipeline instead of the schedule's own, so
+// calling execute (prog_cap of them, its work counter kProgLead words before them) for the pass pipeline instead of the schedule's own, so
 // that concurrent calls on one plan do not share them; a queue needing more runs without the
 // pipeline.
 cudaError_t launch_rotations(int kind, bool hi2lo, const RotLaunch & L, int max_ctas, cudaStream_t st,
@@ -244,8 +251,8 @@ void trmm_tile(int shape, int * rows, int * cols);
 // Right multiply for tri: Out = In * op(U) (rows of In are independent).
 cudaError_t launch_trmm_right(const double * U, const double * in, double * out, int n, int nrows,
                               long long ld, bool trans, cudaStream_t st);
-// tri normalisation (src/drivers.c:6-24), in place
-cudaError_t launch_cheb_normalize(double * A, int N, int M, long long lda, bool transposed, cudaStream_t st);
+// tri normalisation (src/drivers.c:6-24) of nf <= kMaxFields matrices, in place
+cudaError_t launch_cheb_normalize(double * const * A, const int * N, const int * M, int nf, bool transposed, cudaStream_t st);
 
 // Host plan generation (plan.cpp).
 void rotation_tables(int kind, int n, double alpha, double beta, double gamma, double * s, double * c);

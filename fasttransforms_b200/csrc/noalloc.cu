@@ -67,13 +67,14 @@ bool rot(HarmonicPlan * H, bool hi2lo, const double * in, double * out, int M, i
         return false;
     }
     const long long lda = H->n;
-    if (in != out) {
-        const int nc = std::min(M, H->kind == TRI ? 1 : 3);   // orders 0 and 1 have no sweeps
-        if (!ok(cudaMemcpy2DAsync(out, lda * sizeof(double), in, lda * sizeof(double), H->n * sizeof(double), nc,
-                                  cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync")) return false;
-    }
-    if (ntasks == 0) return true;
+    const int nc = std::min(M, H->kind == TRI ? 1 : 3);   // orders 0 and 1 have no sweeps
+    if (ntasks == 0)
+        return in == out || ok(cudaMemcpy2DAsync(out, lda * sizeof(double), in, lda * sizeof(double), H->n * sizeof(double), nc,
+                                                 cudaMemcpyDeviceToDevice, st), "cudaMemcpy2DAsync");
     static thread_local RotLaunch L;
+    L.lead0 = 0;
+    L.lead = nc;
+    L.counter0 = 0;
     L.nfields = 1;
     L.fields[0] = RotField{in, out, RP->d_skew, H->n, M, H->kind, lda, 0};
     L.tasks = tasks;
@@ -159,9 +160,9 @@ int run(HarmonicPlan * H, bool forward, char TRANS, double * A, int N, int M, cu
             if (!ok(launch_trmm_right(U1, cur, oth, N, N, lda, forward, st), "trmm kernel")) return ft_b200_last_status();
             flip();
         }
-        if (!ok(launch_cheb_normalize(cur, N, M, lda, !forward, st), "normalize")) return ft_b200_last_status();
+        if (!ok(launch_cheb_normalize(&cur, &N, &M, 1, !forward, st), "normalize")) return ft_b200_last_status();
     } else {
-        if (!ok(launch_cheb_normalize(A, N, M, lda, !forward, st), "normalize")) return ft_b200_last_status();
+        if (!ok(launch_cheb_normalize(&A, &N, &M, 1, !forward, st), "normalize")) return ft_b200_last_status();
         if (right) {
             if (!ok(launch_trmm_right(U1, cur, oth, N, N, lda, !forward, st), "trmm kernel")) return ft_b200_last_status();
             flip();

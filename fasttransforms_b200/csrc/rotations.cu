@@ -114,18 +114,24 @@ __device__ int g_rot_status;
 __device__ __forceinline__ void publish_progress(int * p, int v) {
     asm volatile("red.release.gpu.global.max.s32 [%0], %1;\n" :: "l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ bool gave_up(long long t0) {
+    if (*(volatile int *) &g_rot_status != 0) return true;
+    if (clock64() - t0 <= (1LL << 32)) return false;
+    atomicExch(&g_rot_status, 3);
+    return true;
+}
 // Waits until *p >= need and returns the value read; gives up after about 2^32 SM cycles,
 // setting the status word, and at once when the word is already set (so one failed wait costs
 // a launch about that long, not that long per unit).
-__device__ __forceinline__ int wait_progress(const int * p, int need) {
+// (The status word is a read of global memory, as slow as the progress word's own: only every 64th
+// poll looks at it.)
+__device__ __noinline__ int wait_progress(const int * p, int need) {
     const long long t0 = clock64();
-    for (;;) {
+    for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
         if (v >= need) return v;
-        if (*(volatile int *) &g_rot_status != 0) return v;
-        if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
-        __nanosleep(32);
+        if (i % 64 == 0 && gave_up(t0)) return v;
     }
 }
 // Whole-task launches run a task's passes one after another in one CTA, whose loading warps wait
@@ -137,14 +143,13 @@ __device__ __forceinline__ unsigned long long local_word(unsigned seq, int v) {
 __device__ __forceinline__ void publish_local(unsigned long long * p, unsigned long long w) {
     asm volatile("st.release.cta.shared::cta.u64 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "l"(w) : "memory");
 }
-__device__ __forceinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need) {
+__device__ __noinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need) {
     const long long t0 = clock64();
-    for (;;) {
+    for (unsigned i = 1;; ++i) {
         unsigned long long v;
         asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];\n" : "=l"(v) : "r"(tc::smem_addr(p)) : "memory");
         if (v >= need) return v;
-        if (*(volatile int *) &g_rot_status != 0) return v;
-        if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
+        if (i % 64 == 0 && gave_up(t0)) return v;
         __nanosleep(32);
     }
 }
@@ -290,48 +295,57 @@ struct Mover {
 // E steps of a stage.  The window is circular: at step u, window position x lives in register
 // slot (u - x) mod 2B.  The element leaving (position 2B - 1 of the previous step) sits in slot
 // u mod 2B, which the entering element (position 0) takes over.  OFF: step number of the chunk's
-// first step mod 2B.
-template <int KIND, bool HI2LO, int B, int E, int OFF>
-__device__ __forceinline__ void stage_steps(double (&win)[KT<KIND>::NCOL][2 * B], const double * bin, double * bout,
-                                            bool has_out, const double2 * const (&sc)[B]) {
-    using T = KT<KIND>;
+// first step mod 2B.  Without rotations (ROTATE false) every element leaves as it entered.
+// has_in / has_out are the same for the warp; elements are read and written in groups of SUB steps,
+// a branch a group (2 - 4 % faster than a condition on each access).
+template <bool HI2LO, int NCOL, int B, int E, int OFF, int STRIDE, int PAIR, int ROWLEN, int SUB, bool ROTATE>
+__device__ __forceinline__ void stage_steps(double (&win)[NCOL][2 * B], const double * bin, double * bout, bool has_in, bool has_out,
+                                            const double2 * const (&sc)[B]) {
     constexpr int W2 = 2 * B;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int u = OFF + e, pn = u % W2;
+    for (int e0 = 0; e0 < E; e0 += SUB) {
+        double in[SUB][NCOL], out[SUB][NCOL];
 #pragma unroll
-        for (int h = 0; h < T::NCOL; ++h) {
-            const double in = bin[e * T::CH * T::CPAD + h];
-            if (has_out) bout[e * T::CH * T::CPAD + h] = win[h][pn];
-            win[h][pn] = in;
+        for (int e = 0; e < SUB; ++e)
+#pragma unroll
+            for (int h = 0; h < NCOL; ++h) in[e][h] = 0.0;
+        if (has_in) {
+#pragma unroll
+            for (int e = 0; e < SUB; ++e)
+#pragma unroll
+                for (int h = 0; h < NCOL; ++h) in[e][h] = bin[(e0 + e) * STRIDE + h];
         }
 #pragma unroll
-        for (int b = 0; b < B; ++b) {
-            constexpr int RL = Geo::kSkewLen * T::CH;
-            const int pos = HI2LO ? E - 1 - e : e;
-            const double2 p = sc[b][(pos / Geo::kSkewLen) * Geo::kSkewRows * RL + (pos % Geo::kSkewLen) * T::CH];
-            const int xl = (u - 2 * b + 2 * W2) % W2;       // window position 2b
-            const int xu = (u - 2 * b - 1 + 2 * W2) % W2;   // window position 2b+1
+        for (int e = 0; e < SUB; ++e) {
+            const int u = OFF + e0 + e, pn = u % W2;
 #pragma unroll
-            for (int h = 0; h < T::NCOL; ++h) {
-                if (HI2LO) rot_hi2lo(win[h][xl], win[h][xu], p.x, p.y);
-                else       rot_lo2hi(win[h][xu], win[h][xl], p.x, p.y);
+            for (int h = 0; h < NCOL; ++h) {
+                out[e][h] = win[h][pn];
+                win[h][pn] = in[e][h];
+            }
+            if (ROTATE) {
+                // PAIR: pairs between positions of a row; rows of a chunk of kSkewLen positions are
+                // ROWLEN pairs long and a chunk of them kSkewRows rows
+                constexpr int SL = Geo::kSkewLen;
+                const int pos = HI2LO ? E - 1 - e0 - e : e0 + e;
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    const double2 p = sc[b][pos / SL * Geo::kSkewRows * ROWLEN + pos % SL * PAIR];
+                    const int xl = (u - 2 * b + 2 * W2) % W2;       // window position 2b
+                    const int xu = (u - 2 * b - 1 + 2 * W2) % W2;   // window position 2b+1
+#pragma unroll
+                    for (int h = 0; h < NCOL; ++h) {
+                        if (HI2LO) rot_hi2lo(win[h][xl], win[h][xu], p.x, p.y);
+                        else       rot_lo2hi(win[h][xu], win[h][xl], p.x, p.y);
+                    }
+                }
             }
         }
-    }
-}
-// The same without rotations: every element leaves the stage as it entered.
-template <int KIND, int B, int E, int OFF>
-__device__ __forceinline__ void shift_steps(double (&win)[KT<KIND>::NCOL][2 * B], const double * bin, double * bout, bool has_out) {
-    using T = KT<KIND>;
+        if (has_out) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int pn = (OFF + e) % (2 * B);
+            for (int e = 0; e < SUB; ++e)
 #pragma unroll
-        for (int h = 0; h < T::NCOL; ++h) {
-            const double in = bin[e * T::CH * T::CPAD + h];
-            if (has_out) bout[e * T::CH * T::CPAD + h] = win[h][pn];
-            win[h][pn] = in;
+                for (int h = 0; h < NCOL; ++h) bout[(e0 + e) * STRIDE + h] = out[e][h];
         }
     }
 }
@@ -342,11 +356,11 @@ __device__ __forceinline__ void publish_word(int * p, int v) {
 }
 __device__ __noinline__ int wait_word_slow(const int * p, int need) {
     const long long t0 = clock64();
-    for (;;) {
+    for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
-        if (v >= need || *(volatile int *) &g_rot_status != 0) return v;
-        if (clock64() - t0 > (1LL << 32)) { atomicExch(&g_rot_status, 3); return v; }
+        if (v >= need) return v;
+        if (i % 256 == 0 && gave_up(t0)) return v;
     }
 }
 __device__ __forceinline__ int wait_word(const int * p, int need) {
@@ -355,8 +369,8 @@ __device__ __forceinline__ int wait_word(const int * p, int need) {
     return v >= need ? v : wait_word_slow(p, need);
 }
 
-// E steps of one sequence of the resident kernel (stage_steps with the columns in place); ROTATE
-// false: the window only shifts.
+// E steps of one sequence of the resident kernel (stage_steps with the columns in place; a branch an
+// access here: groups measured 7 % slower).  ROTATE false: the window only shifts.
 template <bool HI2LO, int CH, int B, int E, int OFF, int ROW, bool ROTATE>
 __device__ __forceinline__ void resident_steps(double (&win)[2 * B], const double * bin, double * bout, bool has_in, bool has_out,
                                                const double2 * const (&sc)[B]) {
@@ -392,7 +406,7 @@ struct Shape {
     static constexpr int SCLEN = B * E * T::CH;          // pairs of a stage's chunk
     static constexpr int IDLEN = (E / Geo::kSkewLen - 1) * Geo::kSkewRows * Geo::kSkewLen * T::CH + Geo::kSkewLen * T::CH;   // a row's span in one
     static constexpr int UR = 4;                         // queue entries in flight in a CTA
-    static constexpr size_t doubles = (size_t) (W + 1) * SL * SLOT + SLOT;
+    static constexpr size_t doubles = (size_t) (W + 1) * SL * SLOT;
     static constexpr size_t pairs = (size_t) W * SCS * SCLEN + IDLEN;
     static constexpr size_t bytes = (doubles * sizeof(double) + 15) / 16 * 16 + pairs * sizeof(double2);
     static_assert(D >= 1 && D * E == 2 * B, "a window must hold whole chunks");
@@ -401,17 +415,27 @@ struct Shape {
                   "a stage's rows must lie one after the other in the skewed table");
 };
 
+// Columns without sweeps, in to out (one CTA a field; nothing when in place).
+__device__ __forceinline__ void copy_lead(const RotLaunch & L) {
+    for (int f = blockIdx.x; f < L.nfields; f += gridDim.x) {
+        const RotField & F = L.fields[f];
+        if (F.in == F.out) continue;
+        for (int c = L.lead0; c < min(L.lead, F.M); ++c)
+            for (int i = threadIdx.x; i < F.N; i += blockDim.x) F.out[c * F.lda + i] = __ldcg(F.in + c * F.lda + i);
+    }
+}
+
 template <int KIND, bool HI2LO, int W, int B, int E, int MINB>
 __global__ void __launch_bounds__(Shape<KIND, W, B, E>::WARPS * 32, MINB)
 rot_kernel(const __grid_constant__ RotLaunch L) {
     using T = KT<KIND>;
     using SH = Shape<KIND, W, B, E>;
     using MV = Mover<KIND, HI2LO, E>;
+    constexpr int SUBS = 2;   // 4 measured the same, 8 (more registers) 10 % slower
     constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, D = SH::D, SL = SH::SL, SCS = SH::SCS, NL = SH::NL, SLOT = SH::SLOT,
                   SCLEN = SH::SCLEN, UR = SH::UR;
     extern __shared__ __align__(16) double smem[];
     double * const rings = smem;                                  // ring q: input of stage q; ring W: output of the last stage
-    double * const zeros = smem + (size_t) (W + 1) * SL * SLOT;   // what a stage reads past the stream's end
     double2 * const pairs = reinterpret_cast<double2 *>(reinterpret_cast<unsigned char *>(smem) + (SH::doubles * sizeof(double) + 15) / 16 * 16);
     double2 * const ident = pairs + (size_t) W * SCS * SCLEN; // identity pairs, for sweeps a lane's order does not have
     __shared__ __align__(8) uint64_t full[(W + 1) * SL], empt[(W + 1) * SL], scbar[W * SCS], ufull[UR], uempt[UR];
@@ -419,7 +443,6 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     __shared__ int s_unit[UR];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < SLOT; i += blockDim.x) zeros[i] = 0.0;
     for (int i = threadIdx.x; i < SH::IDLEN; i += blockDim.x) ident[i] = make_double2(0.0, 1.0);
     if (threadIdx.x == 0) {
         for (int i = 0; i < (W + 1) * SL; ++i) { tc::mbar_init(&full[i], i < SL ? 32 : 1); tc::mbar_init(&empt[i], 1); }
@@ -429,6 +452,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+
+    if (L.lead > L.lead0) copy_lead(L);
 
     const bool pipe = L.chains != nullptr;
     const int nwork = pipe ? L.nchains : L.ntasks;
@@ -444,7 +469,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         if (warp == W) {
             wait_bar(&uempt[slot], ph ^ 1);
             if (lane == 0) {
-                id = atomicAdd(L.counter, 1);
+                id = atomicAdd(L.counter, 1) - L.counter0;
                 if (id >= nwork) id = -1;
                 s_unit[slot] = id;
                 tc::mbar_arrive(&ufull[slot]);
@@ -548,8 +573,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const int is = nin % SL, os = nout % SL;
                     if (has_in) wait_bar(&in_full[is], (nin / SL) & 1);
                     if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1);
-                    const double * const bin = (has_in ? in_ring + is * SLOT : zeros) + lane_off;
-                    double * const bout = out_ring + os * SLOT + lane_off;   // written once elements leave (has_out)
+                    const double * const bin = in_ring + is * SLOT + lane_off;    // read while elements enter (has_in)
+                    double * const bout = out_ring + os * SLOT + lane_off;        // written once elements leave (has_out)
                     const bool odd = D > 1 && (k & 1);   // the chunk starts halfway round the window
                     if (live & 1u) {
                         const int slot = sc_used % SCS;
@@ -559,11 +584,12 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
 #pragma unroll
                         for (int b = 0; b < B; ++b)
                             sc[b] = ((lane_mask >> b) & 1u ? sc_ring + slot * SCLEN + (HI2LO ? B - 1 - b : b) * Geo::kSkewLen * CH : ident) + c_lane;
-                        if (odd) stage_steps<KIND, HI2LO, B, E, E % (2 * B)>(win, bin, bout, has_out, sc);
-                        else     stage_steps<KIND, HI2LO, B, E, 0>(win, bin, bout, has_out, sc);
+                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
+                        else     stage_steps<HI2LO, NCOL, B, E, 0, CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
                     } else {
-                        if (odd) shift_steps<KIND, B, E, E % (2 * B)>(win, bin, bout, has_out);
-                        else     shift_steps<KIND, B, E, 0>(win, bin, bout, has_out);
+                        const double2 * const none[B] = {};
+                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
+                        else     stage_steps<HI2LO, NCOL, B, E, 0, CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
                     }
                     live >>= 1;
                     __syncwarp();
@@ -716,7 +742,7 @@ cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaS
     const int work = L.chains ? L.nchains : L.ntasks;   // queue entries: pipeline entries or tasks
     if (ctas > work) ctas = work;
     if (ctas <= 0) return cudaSuccess;
-    e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);
+    if (!L.chains) e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);   // with chains: launch_shape
     if (e != cudaSuccess) return e;
     kern<<<ctas, SH::WARPS * 32, SH::bytes, st>>>(L);
     count_launch();
@@ -767,6 +793,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
     __shared__ int prog[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+    if (L.lead > L.lead0) copy_lead(L);
     const RotTask task = L.tasks[blockIdx.x / R::SPLIT];
     const RotField & F = L.fields[task.field];
     const int N = F.N, mlast = Geo::last_order(KIND, F.M);
@@ -968,7 +995,7 @@ void set_rotation_config(int cfg) { g_rot_cfg = valid_config(cfg) ? cfg : -1; }
 
 struct RotSchedule {
     std::vector<RotTask> tasks;                          // host copy of the device list (same order)
-    struct Units { RotChain * d_chains = nullptr; int * d_prog = nullptr; int n = 0, nprog = 0; };
+    struct Units { RotChain * d_chains = nullptr; int * d_words = nullptr; int n = 0, nprog = 0; };   // words: counter, progress
     std::map<std::tuple<int, int, int>, Units> lists;    // (sweeps per pass, heads only, mode) -> queue
     std::mutex mu;
 };
@@ -981,7 +1008,7 @@ RotSchedule * rot_schedule_new(const std::vector<RotTask> & tasks) {
 
 void rot_schedule_free(RotSchedule * s) {
     if (!s) return;
-    for (auto & kv : s->lists) { cudaFree(kv.second.d_chains); cudaFree(kv.second.d_prog); }
+    for (auto & kv : s->lists) { cudaFree(kv.second.d_chains); cudaFree(kv.second.d_words); }
     delete s;
 }
 
@@ -1081,9 +1108,9 @@ const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotL
     U.nprog = nprog;
     if (U.n > 0) {
         if (cudaMalloc(&U.d_chains, sizeof(RotChain) * q.size()) != cudaSuccess ||
-            cudaMalloc(&U.d_prog, sizeof(int) * std::max(nprog, 1)) != cudaSuccess ||
+            cudaMalloc(&U.d_words, sizeof(int) * (size_t) (kProgLead + nprog)) != cudaSuccess ||
             cudaMemcpy(U.d_chains, q.data(), sizeof(RotChain) * q.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaFree(U.d_chains); cudaFree(U.d_prog);
+            cudaFree(U.d_chains); cudaFree(U.d_words);
             U = RotSchedule::Units{};
         }
     }
@@ -1102,6 +1129,17 @@ cudaError_t launch_with(int kind, bool hi2lo, int cfg, const RotLaunch & L, int 
     return cudaErrorInvalidValue;
 }
 
+bool resident_fits(int kind, const RotLaunch & L) {
+    switch (kind) {
+        case SPH:  return resident_fits<SPH>(L);
+        case TRI:  return resident_fits<TRI>(L);
+        case DISK: return resident_fits<DISK>(L);
+        case SPIN: return resident_fits<SPIN>(L);
+        case RECT: return resident_fits<RECT>(L);
+    }
+    return false;
+}
+
 // One launch in configuration cfg: shape cfg & 7, through the pass pipeline in mode cfg >> 3
 // (schedule_passes) when the task list has a schedule (else, and in mode 0, each CTA runs
 // every pass of its tasks).  The progress words are the call's own (prog_call) when it has
@@ -1109,16 +1147,19 @@ cudaError_t launch_with(int kind, bool hi2lo, int cfg, const RotLaunch & L, int 
 cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int max_ctas, cudaStream_t st,
                          RotSchedule * sched, int * prog_call = nullptr, int prog_cap = 0) {
     const int shape = cfg & 7, mode = cfg >> 3;
+    if (shape == 5 && resident_fits(kind, L)) return launch_with(kind, hi2lo, shape, L, max_ctas, st);   // no queue
     const RotSchedule::Units * U = (mode > 0 && sched) ? schedule_passes(sched, kind, L, shape_pass(shape), mode, st) : nullptr;
     // a call with words of its own too few for this queue runs whole tasks per CTA instead
     if (!U || (prog_call && U->nprog > prog_cap)) return launch_with(kind, hi2lo, shape, L, max_ctas, st);
-    int * const prog = prog_call ? prog_call : U->d_prog;
+    int * const words = prog_call ? prog_call - kProgLead : U->d_words;
     static thread_local RotLaunch P;
     P = L;
     P.chains = U->d_chains;
     P.nchains = U->n;
-    P.prog = prog;
-    const cudaError_t e = cudaMemsetAsync(prog, 0x80, sizeof(int) * U->nprog, st);   // below any position
+    P.counter = words;
+    P.prog = words + kProgLead;
+    P.counter0 = (int) 0x80808080;   // the fill also puts the progress words below any position
+    const cudaError_t e = cudaMemsetAsync(words, 0x80, sizeof(int) * (size_t) (kProgLead + U->nprog), st);
     if (e != cudaSuccess) return e;
     return launch_with(kind, hi2lo, shape, P, max_ctas, st);
 }

@@ -180,6 +180,7 @@ bool tri_sweeps(const ft_rotation_plan * RP1, const TriStage & T, bool hi2lo, do
         Lr.tasks = g.d_tasks;
         Lr.ntasks = g.ntasks;
         Lr.counter = RP1->d_counter;
+        Lr.lead0 = Lr.lead = Lr.counter0 = 0;
         Lr.chains = nullptr;
         Lr.nchains = 0;
         Lr.prog = nullptr;

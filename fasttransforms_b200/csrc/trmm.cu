@@ -365,15 +365,20 @@ cudaError_t run_gemm(const GemmParams & P, int rows, int cols, bool vec16, cudaS
 
 inline bool aligned16(const void * p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-__global__ void cheb_norm_kernel(double * A, int N, int M, long long lda, double r, double g) {
+struct NormLaunch {
+    double * A[kMaxFields];
+    int N[kMaxFields], M[kMaxFields];
+};
+__global__ void cheb_norm_kernel(const __grid_constant__ NormLaunch L, double r, double g) {
     // src/drivers.c:6-24: first column and first row scaled by r (entry (0,0) twice), all by g
-    const long long total = (long long) N * M;
+    double * const A = L.A[blockIdx.y];
+    const int N = L.N[blockIdx.y];
+    const long long total = (long long) N * L.M[blockIdx.y];
     for (long long e = blockIdx.x * (long long) blockDim.x + threadIdx.x; e < total; e += (long long) gridDim.x * blockDim.x) {
-        const int i = (int) (e % N), j = (int) (e / N);
-        double v = A[(long long) j * lda + i];
-        if (j == 0) v *= r;
-        if (i == 0) v *= r;
-        A[(long long) j * lda + i] = v * g;
+        double v = A[e];
+        if (e < N) v *= r;
+        if (e % N == 0) v *= r;
+        A[e] = v * g;
     }
 }
 
@@ -425,13 +430,20 @@ cudaError_t launch_trmm_right(const double * U, const double * in, double * out,
     return trans ? run_gemm<true, false>(P, nrows, n, vec, st) : run_gemm<true, true>(P, nrows, n, vec, st);
 }
 
-cudaError_t launch_cheb_normalize(double * A, int N, int M, long long lda, bool transposed, cudaStream_t st) {
+cudaError_t launch_cheb_normalize(double * const * A, const int * N, const int * M, int nf, bool transposed, cudaStream_t st) {
     const double r = transposed ? 1.41421356237309504880 : 0.70710678118654752440;   // M_SQRT2, M_SQRT1_2
     const double g = transposed ? 1.57079632679489661923 : 0.63661977236758134308;   // M_PI_2, M_2_PI
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cheb_norm_kernel<<<sms * 4, 256, 0, st>>>(A, N, M, lda, r, g);
+    static thread_local NormLaunch L;
+    long long most = 0;
+    for (int f = 0; f < nf; ++f) {
+        L.A[f] = A[f];
+        L.N[f] = N[f];
+        L.M[f] = M[f];
+        most = std::max(most, (long long) N[f] * M[f]);
+    }
+    // four elements a thread, up to four CTAs per SM over all fields
+    const int blocks = (int) std::max(1LL, std::min((most + 1023) / 1024, (long long) (592 / nf + 1)));
+    cheb_norm_kernel<<<dim3(blocks, nf), 256, 0, st>>>(L, r, g);
     count_launch();
     return cudaGetLastError();
 }
