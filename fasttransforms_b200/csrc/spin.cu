@@ -13,13 +13,14 @@
 //            down to (|m| + |s|) mod 2) with the sph table (the reference's s1, c1 hold
 //            the sph table's values).
 // lo2hi runs stage 2 then stage 1, each transposed.  Stage 2 is the rotation kernel's
-// SPIN kind (rotations.cu: one lane carries the real and imaginary parts of both
-// columns of an order through the sph wavefront); stage 1, at most |s| sweeps per
-// column, is spin_stage1_kernel below, one thread per column.  The connection multiply
+// SPIN kind (rotations.cu: one lane carries the real and imaginary parts of one column
+// through the sph wavefront); stage 1, at most |s| sweeps per column, is
+// spin_stage1_kernel below.  The connection multiply
 // (cblas_ztrmm with the real sph connection matrices stored as complex) is the real
 // class-structured multiply on the real and the imaginary parts, with the matrices of
 // the classes swapped for odd s.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -74,76 +75,127 @@ bool ok(cudaError_t e, const char * what) {
     return false;
 }
 
-// The reference's rotation on both parts (fused form): x' = fma(c, x, s y), y' = fma(c, y, -(s x));
+// The reference's rotation on both parts (fused form) is x' = fma(c, x, s y), y' = fma(c, y, -(s x));
 // the transposed rotation is the rotation by -s.
-__device__ __forceinline__ void rot(double2 & x, double2 & y, double s, double c, bool transposed) {
-    const double sg = transposed ? -s : s;
-    const double syr = __dmul_rn(sg, y.x), sxr = __dmul_rn(sg, x.x);
-    const double syi = __dmul_rn(sg, y.y), sxi = __dmul_rn(sg, x.y);
-    const double2 xn = make_double2(__fma_rn(c, x.x, syr), __fma_rn(c, x.y, syi));
-    const double2 yn = make_double2(__fma_rn(c, y.x, -sxr), __fma_rn(c, y.y, -sxi));
-    x = xn;
-    y = yn;
+//
+// Stage 1: the sweeps j = j0 .. j0 + SB - 1 of every column in one pass down (hi2lo) or up (lo2hi) the
+// rows.  One warp per kS1Cols columns, one lane per column and part; the lane keeps 2 SB consecutive
+// rows in registers, in which the SB sweeps rotate two rows apart, as in rot_kernel.  Rows and table
+// pairs come through shared memory in chunks of kS1Rows rows, read and written in whole segments of
+// the columns, the next chunk's on their way while one is worked on.  Bound: the rotations' own
+// chain and one warp's issue rate, about 80 ns a row: 82 us at n = 1024, s = 2.  One thread per column walking
+// global memory sweep by sweep (eight rows loaded ahead) took 268 - 308 us there.
+constexpr int kS1Cols = 8, kS1Rows = 32, kS1Ld = kS1Rows + 1;
+template <int SB>
+constexpr size_t stage1_bytes() { return sizeof(double2) * (size_t) kS1Cols * kS1Ld * (2 * (1 + SB) + 1); }
+
+__device__ __forceinline__ void s1_copy16(double2 * dst, const double2 * src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                 :: "r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-// Stage 1, one thread per complex column.  A sweep carries one element down (hi2lo) or up
-// (lo2hi) the column; the elements and table pairs of the next LA positions are loaded
-// together before any of them is rotated (none of them is written before it is loaded), so
-// LA loads are in flight per thread instead of one.
-constexpr int LA = 8;
-__global__ void __launch_bounds__(64) spin_stage1_kernel(double2 * A, const double2 * __restrict__ tab, int N, int M,
-                                                         int s, bool hi2lo) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= M) return;
-    const int m = col == 0 ? 0 : ((col & 1) ? -((col + 1) / 2) : col / 2);
-    const int as = abs(s), am = abs(m), d = abs(am - as), nsw = min(am, as);
-    if (nsw == 0) return;
+template <int SB, bool HI2LO>
+__global__ void __launch_bounds__(32) spin_stage1_kernel(double2 * A, const double2 * __restrict__ tab, int N, int M, int s, int j0) {
+    constexpr int W2 = 2 * SB, R = kS1Rows, LD = kS1Ld, TILE = kS1Cols * LD;
+    static_assert(R % W2 == 0, "the window must go round a whole number of times in a chunk");
+    extern __shared__ __align__(16) double2 tiles[];
+    double2 * const out_tile = tiles + 2 * (1 + SB) * TILE;
+    const int lane = threadIdx.x, as = abs(s), col0 = blockIdx.x * kS1Cols;
+    auto order = [](int col) { return col == 0 ? 0 : ((col & 1) ? -((col + 1) / 2) : col / 2); };
+    // the lane's column and part
+    const int lc = lane / 2 % kS1Cols, part = lane & 1, col = col0 + lc, m = order(col);   // lanes past 2 kS1Cols repeat others
+    const int d = abs(abs(m) - as), nsw = min(abs(m), as);
     // hi2lo: forward for m s >= 0; lo2hi: the transposes of those
-    const bool transposed = (m * s >= 0) != hi2lo;
-    double2 * a = A + (long long) col * N;
-    const double2 * t = tab + (long long) d * as * N;
-    double2 xs[LA], sc[LA];
-    if (hi2lo) {
-        for (int j = nsw - 1; j >= 0; --j) {
-            const int top = N - 2 - d - j;   // rotations (k, k + 1), k = top .. 0
-            if (top < 0) continue;
-            const double2 * tj = t + (long long) j * N;
-            double2 y = a[top + 1];
-            for (int k0 = top; k0 >= 0; k0 -= LA) {
+    const bool transposed = (m * s >= 0) != HI2LO;
+    // sweep b of the pass and its last rotation (k, k + 1); none where the column has no such sweep
+    int top[SB];
 #pragma unroll
-                for (int i = 0; i < LA; ++i)
-                    if (k0 - i >= 0) { xs[i] = a[k0 - i]; sc[i] = tj[k0 - i]; }
-#pragma unroll
-                for (int i = 0; i < LA; ++i)
-                    if (k0 - i >= 0) {
-                        rot(xs[i], y, sc[i].x, sc[i].y, transposed);
-                        a[k0 - i + 1] = y;
-                        y = xs[i];
-                    }
-            }
-            a[0] = y;
-        }
-    } else {
-        for (int j = 0; j < nsw; ++j) {
-            const int top = N - 2 - d - j;   // rotations (k, k + 1), k = 0 .. top
-            if (top < 0) continue;
-            const double2 * tj = t + (long long) j * N;
-            double2 x = a[0];
-            for (int k0 = 0; k0 <= top; k0 += LA) {
-#pragma unroll
-                for (int i = 0; i < LA; ++i)
-                    if (k0 + i <= top) { xs[i] = a[k0 + i + 1]; sc[i] = tj[k0 + i]; }
-#pragma unroll
-                for (int i = 0; i < LA; ++i)
-                    if (k0 + i <= top) {
-                        rot(x, xs[i], sc[i].x, sc[i].y, transposed);
-                        a[k0 + i] = x;
-                        x = xs[i];
-                    }
-            }
-            a[top + 1] = x;
-        }
+    for (int b = 0; b < SB; ++b) {
+        const int j = HI2LO ? j0 + SB - 1 - b : j0 + b;
+        top[b] = (col < M && j < nsw) ? N - 2 - d - j : -1;
     }
+    const int nchunk = (N + W2 + R - 1) / R;
+    // chunk k: the row entering at its first step, and the rows of sweep b's rotations
+    auto row_of = [&](int tau) { return HI2LO ? N - 1 - tau : tau; };
+    auto rot_of = [&](int tau, int b) { return HI2LO ? N - 1 - tau + 2 * b : tau - 2 * b - 1; };
+    auto fetch = [&](int k) {
+        double2 * const t = tiles + (k & 1) * (1 + SB) * TILE;
+        const int tau = k * R + lane;
+        const int row = row_of(tau);
+        for (int c = 0; c < kS1Cols; ++c) {
+            const bool there = col0 + c < M;
+            const bool in = there && row >= 0 && row < N;
+            s1_copy16(t + c * LD + lane, A + (in ? (long long) (col0 + c) * N + row : 0), in);
+            const int am = abs(order(col0 + c)), dc = abs(am - as);
+#pragma unroll
+            for (int b = 0; b < SB; ++b) {
+                const int j = HI2LO ? j0 + SB - 1 - b : j0 + b, r = rot_of(tau, b);
+                const bool has = there && j < min(am, as) && r >= 0 && r <= N - 2 - dc - j;
+                s1_copy16(t + (1 + b) * TILE + c * LD + lane, tab + (has ? ((long long) dc * as + j) * N + r : 0), has);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double win[W2];
+#pragma unroll
+    for (int x = 0; x < W2; ++x) win[x] = 0.0;
+    fetch(0);
+    for (int k = 0; k < nchunk; ++k) {
+        if (k + 1 < nchunk) {
+            fetch(k + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncwarp();
+        const double2 * const t = tiles + (k & 1) * (1 + SB) * TILE + lc * LD;
+        double * const o = reinterpret_cast<double *>(out_tile + lc * LD) + part;
+        for (int e0 = 0; e0 < R; e0 += 8) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int e = e0 + i, u = i;      // window slots repeat every W2 <= 8 steps
+                o[2 * e] = win[u % W2];
+                win[u % W2] = reinterpret_cast<const double *>(t + e)[part];
+#pragma unroll
+                for (int b = 0; b < SB; ++b) {
+                    const double2 p = t[(1 + b) * TILE + e];
+                    const int r = rot_of(k * R + e, b);
+                    const bool on = r >= 0 && r <= top[b];
+                    double & lo = win[(u - 2 * b + (HI2LO ? 0 : -1) + 2 * W2) % W2];   // row r
+                    double & hi = win[(u - 2 * b + (HI2LO ? -1 : 0) + 2 * W2) % W2];   // row r + 1
+                    const double sg = transposed ? -p.x : p.x;
+                    const double x = __fma_rn(p.y, lo, __dmul_rn(sg, hi)), y = __fma_rn(p.y, hi, -__dmul_rn(sg, lo));
+                    lo = on ? x : lo;
+                    hi = on ? y : hi;
+                }
+            }
+        }
+        __syncwarp();
+        // rows that left the window: those that entered W2 steps before
+        const int row = row_of(k * R + lane - W2);
+        if (k * R + lane >= W2 && row >= 0 && row < N)
+            for (int c = 0; c < kS1Cols; ++c)
+                if (col0 + c < M) __stcg(A + (long long) (col0 + c) * N + row, out_tile[c * LD + lane]);
+        __syncwarp();
+    }
+}
+
+template <int SB, bool HI2LO>
+cudaError_t launch_stage1(double2 * A, const double2 * tab, int N, int M, int s, int j0, cudaStream_t st) {
+    static std::atomic<unsigned> ready{0};
+    auto kern = spin_stage1_kernel<SB, HI2LO>;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned bit = dev < 32 ? 1u << dev : 0u;
+    if (!(ready.load(std::memory_order_acquire) & bit)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) stage1_bytes<SB>());
+        if (e != cudaSuccess) return e;
+        ready.fetch_or(bit, std::memory_order_release);
+    }
+    kern<<<(M + kS1Cols - 1) / kS1Cols, 32, stage1_bytes<SB>(), st>>>(A, tab, N, M, s, j0);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // complex N x M (interleaved) <-> real parts and imaginary parts, two N x M matrices
@@ -246,9 +298,18 @@ bool spin_tasks(SpinRotPlan * P, int M, RotTask ** d, int * nt, RotSchedule ** s
 
 bool stage1(SpinRotPlan * P, bool hi2lo, double * A, int M, cudaStream_t st) {
     if (P->s == 0 || M < 1) return true;
-    spin_stage1_kernel<<<(M + 63) / 64, 64, 0, st>>>(reinterpret_cast<double2 *>(A), P->d_sc2, P->n, M, P->s, hi2lo);
-    count_launch();
-    return ok(cudaGetLastError(), "spin stage 1");
+    // four sweeps a pass, hi2lo from the highest down, lo2hi from the lowest up
+    double2 * const X = reinterpret_cast<double2 *>(A);
+    const int as = std::abs(P->s), passes = (as + 3) / 4;
+    for (int q = 0; q < passes; q++) {
+        const int j0 = 4 * (hi2lo ? passes - 1 - q : q), n = std::min(4, as - j0);
+        cudaError_t e;
+        if (n == 1)      e = hi2lo ? launch_stage1<1, true>(X, P->d_sc2, P->n, M, P->s, j0, st) : launch_stage1<1, false>(X, P->d_sc2, P->n, M, P->s, j0, st);
+        else if (n == 2) e = hi2lo ? launch_stage1<2, true>(X, P->d_sc2, P->n, M, P->s, j0, st) : launch_stage1<2, false>(X, P->d_sc2, P->n, M, P->s, j0, st);
+        else             e = hi2lo ? launch_stage1<4, true>(X, P->d_sc2, P->n, M, P->s, j0, st) : launch_stage1<4, false>(X, P->d_sc2, P->n, M, P->s, j0, st);
+        if (!ok(e, "spin stage 1")) return false;
+    }
+    return true;
 }
 
 bool stage2(SpinRotPlan * P, bool hi2lo, double * A, int M, cudaStream_t st) {
@@ -263,6 +324,7 @@ bool stage2(SpinRotPlan * P, bool hi2lo, double * A, int M, cudaStream_t st) {
     L.tasks = dt;
     L.ntasks = nt;
     L.counter = P->d_counter;
+    L.lead0 = L.lead = L.counter0 = 0;
     L.chains = nullptr;
     L.nchains = 0;
     L.prog = nullptr;
