@@ -14,7 +14,8 @@
 //
 // Summation: the accumulators sum one chunk of 256 consecutive k (k / 256 equal) at a time; at the
 // end of each chunk a thread adds them into its outputs in C (which it alone writes) and starts the
-// next chunk from zero.  A single accumulation over all n terms lets the rounding error grow with
+// next chunk from zero.  The additions are reductions at L2: reading the sums back held the warps for
+// a round trip every 16 slabs (sph degree 4095 4752 -> 4511 us, 2047 630 -> 594).  A single accumulation over all n terms lets the rounding error grow with
 // n; chunked sums, like a BLAS's K panels, keep it near that of 256 terms plus n / 256 additions (the
 // reference's round trips, which amplify this error in the ill-conditioned triangle transforms,
 // then match its BLAS build).  The chunks do not depend on the tile, so every shape gives the same
@@ -36,13 +37,13 @@ void trmm_tile(int shape, int * rows, int * cols) {
 
 // A launch takes about its slabs' time over the SMs plus the tail in which the longest tiles run
 // alone, which is where the smaller tiles win: they are more and shorter, but load more per flop.
-// Per slab of 16 k, in us: with the chip full, 1.30, 0.67 and 0.18 (128 x 64, 64 x 64, 32 x 32: 29.0,
-// 28.3 and 26.0 TFLOP/s at sph degree 4095); of the longest tile, 0.75, 0.55 and 0.4.  Measured per
-// launch (us; 128 x 64 / 64 x 64 / 32 x 32): sph 64 13 / 11 / 8, 301 50 / 39 / 18, 512 56 / 39 / 24,
-// 1024 135 / 114 / 95, 1501 347 / 317 / 348, 2048 633 / 630 / 673, 4096 4752 / 4837 / 5250; tri 1001
-// 132 / 106 / 69, 2048 349 / 332 / 339.
+// Per slab of 16 k, in us: with the chip full, 1.18, 0.62 and 0.18 (128 x 64, 64 x 64, 32 x 32: 30.5,
+// 30.0 and 25.7 TFLOP/s at sph degree 4095; 0.20 with odd n, whose copies are single doubles); of the
+// longest tile, 0.75, 0.5 and 0.25.  Measured per launch (us; 128 x 64 / 64 x 64 / 32 x 32): sph 64
+// 13 / 11 / 8, 301 40 / 29 / 16, 512 54 / 37 / 25, 1024 127 / 106 / 97, 1501 291 / 282 / 345, 2048
+// 604 / 595 / 688, 4096 4515 / 4598 / 5371; tri 1001 115 / 89 / 66, 2048 321 / 313 / 340.
 int trmm_shape(const std::vector<TrmmExtent> & x) {
-    static const double full[3] = {1.30, 0.67, 0.184}, tail[3] = {0.75, 0.55, 0.4};
+    static const double full[3] = {1.18, 0.623, 0.184}, tail[3] = {0.75, 0.5, 0.25};
     int best = 0;
     double least = 0.0;
     for (int s = 0; s < 3; ++s) {
@@ -52,7 +53,7 @@ int trmm_shape(const std::vector<TrmmExtent> & x) {
         for (const TrmmExtent & e : x) {
             const int tm = (e.mrows + bm - 1) / bm, tn = (e.ncols + bn - 1) / bn;
             // a tile's K runs from its place on the diagonal to the matrix's end: half of it on average
-            slabs += 0.5 * tm * tn * (e.n + (e.mode < 2 ? bm : bn)) / 16.0;
+            slabs += 0.5 * tm * tn * (e.n + (e.mode < 2 ? bm : bn)) / 16.0 * (s == 2 && e.n % 2 ? 1.1 : 1.0);
             longest = std::max(longest, e.n / 16.0);
         }
         const double t = slabs * full[s] / 148.0 + longest * tail[s];
@@ -118,33 +119,29 @@ struct GemmParams {
     int mode;           // 0: left N (k >= i), 1: left T (k <= i), 2: right N (k <= j), 3: right T (k >= j)
 };
 
-// A thread's accumulators (rows m0 + 8a, columns n0 + 8b + {0, 1}) into C:
-// C = acc (first chunk) or C + acc, then acc = 0 when more chunks follow.  All
-// loads are issued before any store, so they are in flight together.
+// A thread's accumulators (rows m0 + 8a, columns n0 + 8b + {0, 1}) into C: C = acc (first chunk) or
+// C + acc (a reduction, which the thread does not wait for; only this thread adds to its outputs, so
+// the order of the additions is its own), then acc = 0 when more chunks follow.
+__device__ __forceinline__ void add_to(double * p, double v) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;\n" :: "l"(p), "d"(v) : "memory");
+}
 template <int FA, int FB>
 __device__ __forceinline__ void flush_partial(const GemmClass & C, const int m0, const int n0, double (&acc)[FA][FB][2],
                                               const bool add, const bool restart) {
-    if (add) {
-#pragma unroll
-        for (int a = 0; a < FA; ++a) {
-            const int m = m0 + a * 8;
-#pragma unroll
-            for (int b = 0; b < FB; ++b) {
-                const int nn = n0 + b * 8;
-                if (m < C.mrows && nn < C.ncols) acc[a][b][0] += C.c[(long long) nn * C.c_ld + m];
-                if (m < C.mrows && nn + 1 < C.ncols) acc[a][b][1] += C.c[(long long) (nn + 1) * C.c_ld + m];
-            }
-        }
-    }
 #pragma unroll
     for (int a = 0; a < FA; ++a) {
         const int m = m0 + a * 8;
 #pragma unroll
         for (int b = 0; b < FB; ++b) {
             const int nn = n0 + b * 8;
-            if (m < C.mrows && nn < C.ncols) C.c[(long long) nn * C.c_ld + m] = acc[a][b][0];
-            if (m < C.mrows && nn + 1 < C.ncols) C.c[(long long) (nn + 1) * C.c_ld + m] = acc[a][b][1];
-            if (restart) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (m < C.mrows && nn + h < C.ncols) {
+                    double * const p = C.c + (long long) (nn + h) * C.c_ld + m;
+                    if (add) add_to(p, acc[a][b][h]); else *p = acc[a][b][h];
+                }
+                if (restart) acc[a][b][h] = 0.0;
+            }
         }
     }
 }
