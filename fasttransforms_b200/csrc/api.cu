@@ -612,10 +612,10 @@ bool upload(BatchCtx * B, const std::vector<T> & v, T ** d) {
     return v.empty() || cuda_ok(cudaMemcpy(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch table)");
 }
 
-// tiles of every class, ordered longest K first for each multiply mode
-bool build_trmm_set(BatchCtx * B, const std::vector<TrmmBatchClass> & cls, TrmmSet * T) {
+// tiles of every class, ordered longest K first for each multiply mode of a side (left: 0, 1; right: 2, 3)
+bool build_trmm_set(BatchCtx * B, const std::vector<TrmmBatchClass> & cls, TrmmSet * T, bool right) {
     if (!upload(B, cls, &T->d_classes)) return false;
-    for (int m = 0; m < 4; m++) {
+    for (int m = right ? 2 : 0; m < (right ? 4 : 2); m++) {
         std::vector<TrmmExtent> x;
         for (const TrmmBatchClass & k : cls) x.push_back({k.mrows, k.ncols, k.n, m});
         T->shape[m] = trmm_shape(x);
@@ -690,8 +690,8 @@ BatchCtx * get_batch(HarmonicPlan * const * H, const int * N, const int * M, int
     }
     size_t work = 0;
     for (int f = 0; f < nf; f++) { B->work_off.push_back(work); work += (size_t) N[f] * M[f]; work = (work + 1) & ~(size_t) 1; }
-    bool ok = upload(B, tasks, &B->d_tasks) && build_trmm_set(B, left, &B->left) &&
-              (kind != TRI || build_trmm_set(B, right, &B->right)) &&
+    bool ok = upload(B, tasks, &B->d_tasks) && build_trmm_set(B, left, &B->left, false) &&
+              (kind != TRI || build_trmm_set(B, right, &B->right, true)) &&
               cuda_ok(cudaMalloc(&B->d_work, sizeof(double) * std::max<size_t>(1, work)), "cudaMalloc(batch workspace)") &&
               cuda_ok(cudaMalloc(&B->d_counter, sizeof(int)), "cudaMalloc(batch counter)");
     if (B->d_work) B->allocs.push_back(B->d_work);

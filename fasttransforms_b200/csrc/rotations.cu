@@ -58,17 +58,26 @@
 namespace ftb {
 namespace {
 
-template <int KIND>
+// NC: sequences a lane carries, all those of an order (1 or 2) or one.
+constexpr int order_sequences(int kind) { return kind == TRI || kind == RECT ? 1 : 2; }
+template <int KIND, int NC = order_sequences(KIND)>
 struct KT {
     static constexpr int CH = (KIND == SPH || KIND == SPIN || KIND == RECT) ? 2 : 1;   // chains per column
     static constexpr int STEP = KIND == TRI ? 1 : 2;      // order step between sweeps
     // sequences per order sharing the rotations: cos, sin columns (sph, disk), the column
     // (tri, rect), or the real and imaginary parts of the column of -m or of m (spin)
-    static constexpr int NCOL = (KIND == TRI || KIND == RECT) ? 1 : 2;
+    static constexpr int SEQ = order_sequences(KIND);
+    static constexpr int NCOL = NC;
     static constexpr int ES = KIND == SPIN ? 2 : 1;       // doubles per element (interleaved complex)
-    static constexpr int ORD = 32 / CH;                   // orders per task (one lane per order and chain)
-    static constexpr int COLS = ORD * NCOL;               // sequences per task
-    static constexpr int CPAD = COLS + 1;                 // padded column dimension of the stage buffers
+    static constexpr int ORD = 32 * NC / (CH * SEQ);      // orders per group of 32 lanes
+    static constexpr int COLS = ORD * SEQ;                // sequences of those, both chains as one
+    // a step's elements in a ring: lanes with all sequences read theirs next to each other, chain by
+    // chain; lanes with one sequence read element [lane]
+    static constexpr int CPAD = COLS + 1;
+    static constexpr int ROWD = NC == SEQ ? CH * CPAD : 33;
+    __host__ __device__ static constexpr int place(int c, int cl) { return NC == SEQ ? c * CPAD + cl : cl * CH + c; }
+    __host__ __device__ static constexpr int lane_order(int lane) { return NC == SEQ ? lane / CH : lane / (CH * SEQ); }
+    __host__ __device__ static constexpr int lane_place(int lane) { return NC == SEQ ? lane % CH * CPAD + lane / CH * NC : lane; }
 };
 
 // Builds the skewed table (Geo::skew_at): CTA (beta, p) fills block beta of parity p.
@@ -154,20 +163,22 @@ __device__ __noinline__ unsigned long long wait_local(const unsigned long long *
     }
 }
 // Bounded mbarrier wait: a wait that runs out sets the status word, after which every wait of
-// the launch returns at once and the kernel runs to its end on whatever the buffers hold.
+// the launch returns false at once, the loops over queue entries end, and the kernel with them.
 // (The slow path is a call: the kernel's warps run different code at the same time, and what they
 // run between them has to stay small to be served from the instruction cache.)
-__device__ __noinline__ void wait_bar_slow(uint64_t * bar, uint32_t parity) {
-    if (!tc::mbar_wait(bar, parity, (volatile int *) &g_rot_status)) atomicCAS(&g_rot_status, 0, 5);
+__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, uint32_t parity) {
+    if (tc::mbar_wait(bar, parity, (volatile int *) &g_rot_status)) return true;
+    atomicCAS(&g_rot_status, 0, 5);
+    return false;
 }
-__device__ __forceinline__ void wait_bar(uint64_t * bar, uint32_t parity) {
+__device__ __forceinline__ bool wait_bar(uint64_t * bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok) : "r"(tc::smem_addr(bar)), "r"(parity) : "memory");
-    if (!ok) wait_bar_slow(bar, parity);
+    return ok || wait_bar_slow(bar, parity);
 }
 
 // Asynchronous 8-byte copy global -> shared (0 bytes read, zeros written when !valid), and the
@@ -210,15 +221,15 @@ struct Pass {
 };
 
 // A task's sweeps and passes.
-template <int KIND, int W, int B>
+template <int KIND, int NC, int W, int B>
 struct TaskGeo {
     int N, M, mbase, mlast, jpar, nsw, jlo, jhi, npass;
-    __host__ __device__ __forceinline__ TaskGeo(const RotField & F, const RotTask & t) {
+    __host__ __device__ __forceinline__ TaskGeo(const RotField & F, const RotTask & t) {   // t: a group of KT<KIND, NC>::ORD orders
         N = F.N; M = F.M; mbase = t.mbase;
         mlast = Geo::last_order(KIND, M);
         // lowest sweep of every column (spin: the parity of the effective orders |m - s|)
         jpar = KIND == TRI ? 0 : (KIND == SPIN ? ((mbase + F.spin) & 1) : (mbase & 1));
-        nsw = Geo::task_sweeps(KIND, M, mbase, F.blk, &jlo, &jhi, F.spin);
+        nsw = mbase > mlast ? 0 : Geo::task_sweeps(KIND, M, mbase, F.blk, &jlo, &jhi, F.spin, KT<KIND, NC>::ORD);
         npass = (nsw + W * B - 1) / (W * B);
     }
 };
@@ -226,9 +237,9 @@ struct TaskGeo {
 // The elements of one chunk as a warp moves them between global memory and a ring slot.  A column's
 // part of a chunk is a segment of E * CH * ES consecutive doubles; a lane takes, in each of PH
 // phases, the same double of every SSTEP-th segment, so that its addresses advance by constants.
-template <int KIND, bool HI2LO, int E>
+template <int KIND, int NC, bool HI2LO, int E>
 struct Mover {
-    using T = KT<KIND>;
+    using T = KT<KIND, NC>;
     static constexpr int RPC = E * T::CH * T::ES;                  // doubles of a segment
     static constexpr int SEGS = T::COLS / T::ES;                   // segments (columns) of a task
     static constexpr int PER = T::COLS * E * T::CH / 32;           // elements of a lane
@@ -238,7 +249,7 @@ struct Mover {
     static constexpr int PH = RB > 1 ? RB : (PAIRED && SP == 1) ? 2 : 1;
     static constexpr int NV = PER / PH;                            // elements of a lane in a phase
     static constexpr int SSTEP = RB > 1 ? 1 : SP * PH;
-    static constexpr int SLOT_STEP = SSTEP * T::ES;                // ring slot doubles between them
+    static constexpr int SLOT_STEP = T::place(0, SSTEP * T::ES);   // ring slot doubles between them
     static_assert(RPC % 32 == 0 || 32 % RPC == 0, "a segment must split evenly over the lanes");
     static_assert(!PAIRED || SSTEP % 2 == 0, "a lane's segments must be whole orders apart");
     long long base;     // double offset, at chain position 0, of the column of this lane's segment 0
@@ -288,7 +299,7 @@ struct Mover {
     __host__ __device__ __forceinline__ int slot_at(int ph) const {
         const int r = rr(ph, lane), pos = r / (T::ES * T::CH), c = (r / T::ES) % T::CH, part = r % T::ES;
         const int u = HI2LO ? E - 1 - pos : pos;
-        return (u * T::CH + c) * T::CPAD + (seg(ph) + lane_seg(lane)) * T::ES + part;
+        return u * T::ROWD + T::place(c, (seg(ph) + lane_seg(lane)) * T::ES + part);
     }
 };
 
@@ -394,15 +405,16 @@ __device__ __forceinline__ void resident_steps(double (&win)[2 * B], const doubl
 }
 
 // Compile-time layout of a launch shape.
-template <int KIND, int W, int B, int E>
+template <int KIND, int NC, int W, int B, int E>
 struct Shape {
-    using T = KT<KIND>;
+    using T = KT<KIND, NC>;
+    static constexpr int SPLIT = KT<KIND>::ORD / T::ORD;  // groups of a task of the list
     static constexpr int D = 2 * B / E;                  // chunks an element spends in a stage's window
     static constexpr int SL = 2;                         // slots of a ring
     static constexpr int SCS = E >= 16 ? 2 : 3;          // staged (sin, cos) chunks of a stage
     static constexpr int NL = 1;                         // loading warps
     static constexpr int WARPS = W + NL + 1;
-    static constexpr int SLOT = E * T::CH * T::CPAD;     // doubles of a ring slot
+    static constexpr int SLOT = E * T::ROWD;     // doubles of a ring slot
     static constexpr int SCLEN = B * E * T::CH;          // pairs of a stage's chunk
     static constexpr int IDLEN = (E / Geo::kSkewLen - 1) * Geo::kSkewRows * Geo::kSkewLen * T::CH + Geo::kSkewLen * T::CH;   // a row's span in one
     static constexpr int UR = 4;                         // queue entries in flight in a CTA
@@ -425,12 +437,12 @@ __device__ __forceinline__ void copy_lead(const RotLaunch & L) {
     }
 }
 
-template <int KIND, bool HI2LO, int W, int B, int E, int MINB>
-__global__ void __launch_bounds__(Shape<KIND, W, B, E>::WARPS * 32, MINB)
+template <int KIND, int NC, bool HI2LO, int W, int B, int E, int MINB>
+__global__ void __launch_bounds__(Shape<KIND, NC, W, B, E>::WARPS * 32, MINB)
 rot_kernel(const __grid_constant__ RotLaunch L) {
-    using T = KT<KIND>;
-    using SH = Shape<KIND, W, B, E>;
-    using MV = Mover<KIND, HI2LO, E>;
+    using T = KT<KIND, NC>;
+    using SH = Shape<KIND, NC, W, B, E>;
+    using MV = Mover<KIND, NC, HI2LO, E>;
     constexpr int SUBS = 2;   // 4 measured the same, 8 (more registers) 10 % slower
     constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, D = SH::D, SL = SH::SL, SCS = SH::SCS, NL = SH::NL, SLOT = SH::SLOT,
                   SCLEN = SH::SCLEN, UR = SH::UR;
@@ -456,7 +468,13 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     if (L.lead > L.lead0) copy_lead(L);
 
     const bool pipe = L.chains != nullptr;
-    const int nwork = pipe ? L.nchains : L.ntasks;
+    const int nwork = pipe ? L.nchains : L.ntasks * SH::SPLIT;
+    // group g of the list: orders g % SPLIT of its task
+    auto group = [&](int g) {
+        RotTask t = L.tasks[g / SH::SPLIT];
+        t.mbase += T::STEP * T::ORD * (g % SH::SPLIT);
+        return t;
+    };
     unsigned nunit = 0;        // queue entries taken so far
     unsigned seq = 0;          // passes begun so far
     // The first loading warp takes an entry from the queue and hands it to the other warps, which
@@ -467,7 +485,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         ++nunit;
         int id = 0;
         if (warp == W) {
-            wait_bar(&uempt[slot], ph ^ 1);
+            if (!__all_sync(0xffffffffu, wait_bar(&uempt[slot], ph ^ 1))) return -1;
             if (lane == 0) {
                 id = atomicAdd(L.counter, 1) - L.counter0;
                 if (id >= nwork) id = -1;
@@ -476,7 +494,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             }
             id = __shfl_sync(0xffffffffu, id, 0);
         } else {
-            wait_bar(&ufull[slot], ph);
+            if (!__all_sync(0xffffffffu, wait_bar(&ufull[slot], ph))) return -1;
             id = *(volatile int *) &s_unit[slot];
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&uempt[slot]);
@@ -487,8 +505,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     if (warp < W) {
         // ---------------- a stage: B consecutive sweeps of each pass ----------------
         const int q = warp;
-        const int o_lane = lane / CH, c_lane = lane % CH;
-        const int lane_off = c_lane * T::CPAD + o_lane * NCOL;
+        const int o_lane = T::lane_order(lane), c_lane = lane % CH, lane_off = T::lane_place(lane);
         uint64_t * const in_full = full + q * SL, * const in_empty = empt + q * SL;
         uint64_t * const out_full = full + (q + 1) * SL, * const out_empty = empt + (q + 1) * SL;
         double * const in_ring = rings + (size_t) q * SL * SLOT, * const out_ring = in_ring + (size_t) SL * SLOT;
@@ -500,9 +517,9 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const int id = next_unit();
             if (id < 0) break;
             const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
-            const RotTask task = L.tasks[chain.task];
+            const RotTask task = group(chain.task);
             const RotField & F = L.fields[task.field];
-            const TaskGeo<KIND, W, B> G(F, task);
+            const TaskGeo<KIND, NC, W, B> G(F, task);
             const int N = G.N;
             const int jpar = G.jpar;
             // the order whose sweeps this lane runs (spin: |m - s|), and its lowest sweep: with
@@ -523,7 +540,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
 #pragma unroll
                         for (int e = 0; e < E; ++e)
 #pragma unroll
-                            for (int h = 0; h < NCOL; ++h) bout[e * CH * T::CPAD + h] = bin[e * CH * T::CPAD + h];
+                            for (int h = 0; h < NCOL; ++h) bout[e * T::ROWD + h] = bin[e * T::ROWD + h];
                         __syncwarp();
                         if (lane == 0) { tc::mbar_arrive(&in_empty[nin % SL]); tc::mbar_arrive(&out_full[nout % SL]); }
                         ++nin; ++nout;
@@ -584,12 +601,12 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
 #pragma unroll
                         for (int b = 0; b < B; ++b)
                             sc[b] = ((lane_mask >> b) & 1u ? sc_ring + slot * SCLEN + (HI2LO ? B - 1 - b : b) * Geo::kSkewLen * CH : ident) + c_lane;
-                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
-                        else     stage_steps<HI2LO, NCOL, B, E, 0, CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
+                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), T::ROWD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
+                        else     stage_steps<HI2LO, NCOL, B, E, 0, T::ROWD, CH, Geo::kSkewLen * CH, SUBS, true>(win, bin, bout, has_in, has_out, sc);
                     } else {
                         const double2 * const none[B] = {};
-                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
-                        else     stage_steps<HI2LO, NCOL, B, E, 0, CH * T::CPAD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
+                        if (odd) stage_steps<HI2LO, NCOL, B, E, E % (2 * B), T::ROWD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
+                        else     stage_steps<HI2LO, NCOL, B, E, 0, T::ROWD, CH, Geo::kSkewLen * CH, SUBS, false>(win, bin, bout, has_in, has_out, none);
                     }
                     live >>= 1;
                     __syncwarp();
@@ -614,9 +631,9 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const int id = next_unit();
             if (id < 0) break;
             const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
-            const RotTask task = L.tasks[chain.task];
+            const RotTask task = group(chain.task);
             const RotField & F = L.fields[task.field];
-            const TaskGeo<KIND, W, B> G(F, task);
+            const TaskGeo<KIND, NC, W, B> G(F, task);
             if (w == 0 && lane == 0 && G.nsw > 0 && (chain.first >= G.npass || chain.stride < 1))
                 atomicExch(&g_rot_status, 4);   // a schedule that does not match this launch shape
             const MV mv(F, task, G.mlast, lane);
@@ -663,7 +680,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 wait_chunk(0);
                 // hi2lo: the positions above this pass's range are final once the predecessor has
                 // finished the first chunk's (they belong to earlier passes only)
-                if (pipe && w == 0 && lane == 0) publish_progress(L.prog + chain.prog0 + r, HI2LO ? -(P.emax + 1) : -1);
+                if (HI2LO && pipe && w == 0 && lane == 0 && r + 1 < G.npass) publish_progress(L.prog + chain.prog0 + r, -(P.emax + 1));
                 for (int i = w; i < P.nchunk; i += NL) { wait_chunk(i); fetch(i); }
                 n0 += P.nchunk;
             }
@@ -678,9 +695,9 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const int id = next_unit();
             if (id < 0) break;
             const RotChain chain = pipe ? L.chains[id] : RotChain{id, 0, 0, 1};
-            const RotTask task = L.tasks[chain.task];
+            const RotTask task = group(chain.task);
             const RotField & F = L.fields[task.field];
-            const TaskGeo<KIND, W, B> G(F, task);
+            const TaskGeo<KIND, NC, W, B> G(F, task);
             const MV mv(F, task, G.mlast, lane);
             // publish every 16 positions for short columns, every 64 for long ones (and at the end): a
             // successor trailing by a little more loses little of a long pass
@@ -718,10 +735,10 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     }
 }
 
-template <int KIND, bool HI2LO, int W, int B, int E, int MINB>
+template <int KIND, int NC, bool HI2LO, int W, int B, int E, int MINB>
 cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaStream_t st) {
-    using SH = Shape<KIND, W, B, E>;
-    auto kern = rot_kernel<KIND, HI2LO, W, B, E, MINB>;
+    using SH = Shape<KIND, NC, W, B, E>;
+    auto kern = rot_kernel<KIND, NC, HI2LO, W, B, E, MINB>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -739,7 +756,7 @@ cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaS
     }
     int ctas = (room >> 8) * (per_sm_most > 0 ? std::min(per_sm_most, room & 255) : room & 255);
     if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
-    const int work = L.chains ? L.nchains : L.ntasks;   // queue entries: pipeline entries or tasks
+    const int work = L.chains ? L.nchains : L.ntasks * SH::SPLIT;   // queue entries: pipeline entries or groups
     if (ctas > work) ctas = work;
     if (ctas <= 0) return cudaSuccess;
     if (!L.chains) e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);   // with chains: launch_shape
@@ -767,7 +784,7 @@ cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaS
 // ---------------------------------------------------------------------------
 template <int KIND>
 struct RT {
-    static constexpr int CH = KT<KIND>::CH, STEP = KT<KIND>::STEP, ES = KT<KIND>::ES, NC = KT<KIND>::NCOL;
+    static constexpr int CH = KT<KIND>::CH, STEP = KT<KIND>::STEP, ES = KT<KIND>::ES, NC = KT<KIND>::SEQ;
     static constexpr int ORD = 32 / (CH * NC);                  // orders of a CTA
     static constexpr int SPLIT = KT<KIND>::ORD / ORD;           // CTAs of a task of the list
     static constexpr int W = 8, B = 8, E = 8, D = 2 * B / E, SCS = 3;
@@ -961,17 +978,19 @@ cudaError_t launch_resident(const RotLaunch & L, cudaStream_t st) {
 
 }  // namespace
 
-// Launch shapes: 0 .. 4 rot_kernel with W stage warps x B sweeps per warp, chunk E, CTAs per SM
-// (0: as many as fit); 5 rot_resident_kernel.
-//   0: 8 x 8 x 16    1: 8 x 8 x 8    2: 4 x 8 x 8, one CTA per SM    3: 8 x 4 x 8    4: 4 x 8 x 8
+// Launch shapes: 0 .. 4 rot_kernel with W stage warps x B sweeps per warp, chunk E; 5
+// rot_resident_kernel.
+//   0: 8 x 8 x 16    1: 8 x 8 x 8    2: 4 x 8 x 8, one CTA per SM    4: 4 x 8 x 8, as many as fit
+//   3: 8 x 8 x 8 with one sequence a lane (half the orders a group, twice the groups)
 template <int KIND, bool HI2LO>
 cudaError_t launch_kind(int cfg, const RotLaunch & L, int max_ctas, cudaStream_t st) {
+    constexpr int NC = order_sequences(KIND);
     if (cfg == 5 && resident_fits<KIND>(L)) return launch_resident<KIND, HI2LO>(L, st);
-    if (cfg == 1) return launch_cfg<KIND, HI2LO, 8, 8, 8, 1>(L, max_ctas, 0, st);
-    if (cfg == 2) return launch_cfg<KIND, HI2LO, 4, 8, 8, 2>(L, max_ctas, 1, st);
-    if (cfg == 3) return launch_cfg<KIND, HI2LO, 8, 4, 8, 1>(L, max_ctas, 0, st);
-    if (cfg == 4) return launch_cfg<KIND, HI2LO, 4, 8, 8, 2>(L, max_ctas, 0, st);
-    return launch_cfg<KIND, HI2LO, 8, 8, 16, 1>(L, max_ctas, 0, st);
+    if (cfg == 1) return launch_cfg<KIND, NC, HI2LO, 8, 8, 8, 1>(L, max_ctas, 0, st);
+    if (cfg == 2) return launch_cfg<KIND, NC, HI2LO, 4, 8, 8, 2>(L, max_ctas, 1, st);
+    if (cfg == 3) return launch_cfg<KIND, 1, HI2LO, 8, 8, 8, 1>(L, max_ctas, 1, st);
+    if (cfg == 4) return launch_cfg<KIND, NC, HI2LO, 4, 8, 8, 2>(L, max_ctas, 0, st);
+    return launch_cfg<KIND, NC, HI2LO, 8, 8, 16, 1>(L, max_ctas, 0, st);
 }
 
 int g_rot_cfg = -2;
@@ -996,7 +1015,7 @@ void set_rotation_config(int cfg) { g_rot_cfg = valid_config(cfg) ? cfg : -1; }
 struct RotSchedule {
     std::vector<RotTask> tasks;                          // host copy of the device list (same order)
     struct Units { RotChain * d_chains = nullptr; int * d_words = nullptr; int n = 0, nprog = 0; };   // words: counter, progress
-    std::map<std::tuple<int, int, int>, Units> lists;    // (sweeps per pass, heads only, mode) -> queue
+    std::map<std::tuple<int, int, int>, Units> lists;    // (sweeps per pass and split, heads only, mode) -> queue
     std::mutex mu;
 };
 
@@ -1008,7 +1027,7 @@ RotSchedule * rot_schedule_new(const std::vector<RotTask> & tasks) {
 
 void rot_schedule_free(RotSchedule * s) {
     if (!s) return;
-    for (auto & kv : s->lists) { cudaFree(kv.second.d_chains); cudaFree(kv.second.d_words); }
+    for (auto & kv : s->lists) cudaFree(kv.second.d_chains);   // the words are in the same allocation
     delete s;
 }
 
@@ -1047,9 +1066,11 @@ namespace {
 
 // Sweeps per pass (W x B) of each launch shape.
 int shape_pass(int cfg) {
-    static const int wb[6] = {64, 64, 32, 32, 32, 64};
+    static const int wb[6] = {64, 64, 32, 64, 32, 64};
     return (cfg >= 0 && cfg < 6) ? wb[cfg] : 64;
 }
+// Groups that a shape makes of a task of the list (Shape::SPLIT).
+int shape_split(int cfg, int kind) { return cfg == 3 ? order_sequences(kind) : 1; }
 
 // The queue of the pass pipeline for L's tasks with passes of wb sweeps, built on first use;
 // null when the stream is capturing then (the upload synchronises) or on an allocation
@@ -1064,22 +1085,23 @@ int shape_pass(int cfg) {
 // (so consecutive passes of a task still find them there), then every other task as one
 // entry running all its passes, longest first: the long tasks no longer end the launch alone,
 // and the short ones fill in at the end.
-const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotLaunch & L, int wb, int mode, cudaStream_t st) {
+const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotLaunch & L, int wb, int split, int mode, cudaStream_t st) {
     const int blk = L.fields[0].blk;
     std::lock_guard<std::mutex> lk(S->mu);
-    const auto key = std::make_tuple(wb, blk > 0 ? 1 : 0, mode);
+    const auto key = std::make_tuple(wb * 8 + split, blk > 0 ? 1 : 0, mode);
     auto it = S->lists.find(key);
     if (it != S->lists.end()) return it->second.d_chains ? &it->second : nullptr;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
-    const int nt = (int) S->tasks.size();
+    const int nt = (int) S->tasks.size() * split, orders = Geo::task_orders(kind) / split;   // groups, and their orders
     std::vector<int> npass(nt, 0), prog0(nt, 0);
     int nprog = 0, maxp = 0;
     for (int t = 0; t < nt; ++t) {
-        const RotTask & T = S->tasks[t];
+        const RotTask & T = S->tasks[t / split];
         const RotField & F = L.fields[T.field];
+        const int mbase = T.mbase + Geo::step(kind) * orders * (t % split);
         int jlo, jhi;
-        const int nsw = Geo::task_sweeps(kind, F.M, T.mbase, F.blk, &jlo, &jhi, F.spin);
+        const int nsw = mbase > Geo::last_order(kind, F.M) ? 0 : Geo::task_sweeps(kind, F.M, mbase, F.blk, &jlo, &jhi, F.spin, orders);
         npass[t] = (nsw + wb - 1) / wb;
         prog0[t] = nprog;
         nprog += npass[t];
@@ -1093,7 +1115,7 @@ const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotL
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
         const int seqs = (kind == TRI || kind == RECT) ? 1 : 2;   // doubles per order and row
-        const long long cols = (long long) Geo::task_orders(kind) * seqs;
+        const long long cols = (long long) orders * seqs;
         const long long foot = cols * (long long) L.fields[0].N * (long long) sizeof(double);
         npipe = (int) std::min<long long>(nt, std::max<long long>(1, (l2 / 2) / std::max<long long>(foot, 1)));
     }
@@ -1107,11 +1129,13 @@ const RotSchedule::Units * schedule_passes(RotSchedule * S, int kind, const RotL
     U.n = (int) q.size();
     U.nprog = nprog;
     if (U.n > 0) {
-        if (cudaMalloc(&U.d_chains, sizeof(RotChain) * q.size()) != cudaSuccess ||
-            cudaMalloc(&U.d_words, sizeof(int) * (size_t) (kProgLead + nprog)) != cudaSuccess ||
+        const size_t list = (sizeof(RotChain) * q.size() + 255) & ~(size_t) 255;
+        if (cudaMalloc(&U.d_chains, list + sizeof(int) * (size_t) (kProgLead + nprog)) != cudaSuccess ||
             cudaMemcpy(U.d_chains, q.data(), sizeof(RotChain) * q.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaFree(U.d_chains); cudaFree(U.d_words);
+            cudaFree(U.d_chains);
             U = RotSchedule::Units{};
+        } else {
+            U.d_words = reinterpret_cast<int *>(reinterpret_cast<char *>(U.d_chains) + list);
         }
     }
     S->lists[key] = U;
@@ -1148,7 +1172,7 @@ cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int
                          RotSchedule * sched, int * prog_call = nullptr, int prog_cap = 0) {
     const int shape = cfg & 7, mode = cfg >> 3;
     if (shape == 5 && resident_fits(kind, L)) return launch_with(kind, hi2lo, shape, L, max_ctas, st);   // no queue
-    const RotSchedule::Units * U = (mode > 0 && sched) ? schedule_passes(sched, kind, L, shape_pass(shape), mode, st) : nullptr;
+    const RotSchedule::Units * U = (mode > 0 && sched) ? schedule_passes(sched, kind, L, shape_pass(shape), shape_split(shape, kind), mode, st) : nullptr;
     // a call with words of its own too few for this queue runs whole tasks per CTA instead
     if (!U || (prog_call && U->nprog > prog_cap)) return launch_with(kind, hi2lo, shape, L, max_ctas, st);
     int * const words = prog_call ? prog_call - kProgLead : U->d_words;
@@ -1164,27 +1188,32 @@ cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int
     return launch_with(kind, hi2lo, shape, P, max_ctas, st);
 }
 
-// Configuration without measurements (in-place launches, capturing streams, the first launches of
-// the spin and tetrahedral sweeps).  Measured per launch in us, one field in place, resident /
-// 4 x 8 x 8 on one CTA per SM / 8 x 8 x 16, the last two through the pass pipeline:
-//   sph 301 60 / 100 / 107, 767 210 / 245 / 294, 1024 328 / 348 / 403, 1500 - / 798 / 668
-//   disk 301 138 / 185 / 219, 512 318 / 320 / 397, 1501 - / 2730 / 2000
-//   tri 301 133 / 134 / 138, 512 310 / 224 / 249, 1001 - / 470 / 509, 2048 - / 2510 / 1650
-//   rect 301 58 / 72 / 73, 1024 319 / 248 / 258
-// The resident kernel wins until its CTAs' own work, which grows with the cube of n on a number of
-// SMs that grows with n, passes what the pipeline spreads over the whole chip: chains of 512
-// positions for two columns an order, 300 for one (half the CTAs for the same work).  Past that,
-// few passes leave the SMs to single warps per sub-partition, which run a pass's steps twice as
-// fast (the launch is then bound by the longest task's passes in turn); from about two passes of
-// 64 sweeps per SM on, throughput counts.
+// Configuration without measurements (in-place launches, capturing streams, the spin and tetrahedral
+// sweeps).  Measured per launch in us, one field in place, resident / 8 x 8 x 8 with one sequence a
+// lane (tri, rect: 4 x 8 x 8) / 8 x 8 x 16, the last two through the pass pipeline:
+//   sph 301 60 / 70 / 98, 600 141 / 141 / 204, 767 203 / 182 / 266, 1024 320 / 288 / 365,
+//       1200 425 / 414 / 455, 1500 - / 710 / 603, 2048 - / 1670 / 1210
+//   disk 301 142 / 158 / 200, 400 210 / 182 / 275, 700 555 / 375 / 505, 1024 - / 890 / 803
+//   spin 512 147 / 155 / 202, 767 273 / 307 / 340, 1024 530 / 560 / 491
+//   tri 301 133 / 134 / 138, 400 208 / 164 / 180, 1001 - / 450 / 475, 2048 - / 2400 / 1500
+//   rect 301 58 / 72 / 73, 512 107 / 111 / 114, 767 199 / 162 / 173, 1024 316 / 235 / 240
+// A launch of few passes is bound by the longest task's passes following each other, and a stage
+// follows the one before at 2B + E steps, a step taking a warp four cycles per FP64 instruction.
+// Resident columns have no passes, and win until a CTA's own work, which grows with the cube of n,
+// takes over: chains of 300 positions, more where their CTAs fill the chip.  Then one sequence a
+// lane halves a step, at half the rotations per (sin, cos) load, until about 400 passes of 64
+// sweeps give every SM enough of them for throughput to count.
 int default_config(int kind, const RotLaunch & L, RotSchedule * sched, cudaStream_t st) {
     if (L.nfields > 0 && L.fields[0].blk > 0) return 4;   // at most 31 sweeps a column: one pass of 4 x 8
-    const bool pair = kind != TRI && kind != RECT;
+    const bool pair = order_sequences(kind) == 2;
     int len = 0;
     for (int f = 0; f < L.nfields; ++f) len = std::max(len, Geo::chain_len(kind, L.fields[f].N, 0));
-    const RotSchedule::Units * const U = sched && len > (pair ? 512 : 300) ? schedule_passes(sched, kind, L, shape_pass(0), 1, st) : nullptr;
+    const int ctas = L.ntasks * order_sequences(kind);    // of the resident kernel
+    const RotSchedule::Units * const U =
+        sched && len > (pair && ctas >= 148 ? 400 : 300) ? schedule_passes(sched, kind, L, shape_pass(0), 1, 1, st) : nullptr;
     if (!U) return 5;             // whole tasks: resident where they fit, else 8 x 8 x 16
-    return 8 + (U->n <= 300 ? 2 : 0);
+    if (pair) return U->n <= 400 ? 8 + 3 : 8;
+    return U->n <= 300 ? 8 + 2 : 8;
 }
 
 // The autotuner's choices, by launch shape: family, direction, heads only or all sweeps,
