@@ -847,46 +847,66 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
         const int row = x / ES, h = ES == 2 ? x % 2 : s % SEGC;
         return row / CH * ROW + (s / SEGC * NC + h) * CH + row % CH;
     };
-    for (int s = warp; s < ORD * SEGC; s += W) {
-        long long at;
-        const bool there = column_at(s, &at);
-#pragma unroll 4
-        for (int x = lane; x < len; x += 32) col[place(s, x)] = there ? __ldcg(F.in + at + x) : 0.0;
-    }
-    __syncthreads();
-
     const int nblk = (nsw + B - 1) / B;
-    const int c_lane = lane % CH, m_lane = mbase + STEP * (lane / (CH * NC));
-    const int me_lane = KIND == SPIN ? abs(m_lane - F.spin) : m_lane;
-    const int jcut = F.blk > 0 ? m_lane - STEP * (((m_lane - jpar) / STEP) % F.blk) : jpar;
     double2 * const sc_ring = pairs + warp * SCS * SCLEN;
     uint64_t * const bars = scbar + warp * SCS;
     unsigned sc_issued = 0, sc_used = 0;
-    for (int g = warp; g < nblk; g += W) {
-        const int i0 = (jlo - jpar) / STEP + (HI2LO ? nblk - 1 - g : g) * B;
+    // the warp's block: its lowest sweep, highest chunk, steps of a chunk, pairs
+    int i0 = 0, chi = 0, K = 0, nk = 0;
+    const double2 * rows = nullptr;
+    unsigned live = 0;          // bit i: the pairs of chunk k + i are staged
+    auto stage_sc = [&](int k) -> bool {
+        const int kappa = HI2LO ? chi + D - k : k;
+        if (k >= K || kappa >= nk) return false;
+        if (lane == 0) {
+            uint64_t * const bar = &bars[sc_issued % SCS];
+            tc::mbar_arrive_expect_tx(bar, (uint32_t) (SCLEN * sizeof(double2)));
+            tc::bulk_g2s(sc_ring + (sc_issued % SCS) * SCLEN, rows + kappa * Geo::skew_chunk(KIND), (uint32_t) (SCLEN * sizeof(double2)), bar);
+        }
+        ++sc_issued;
+        return true;
+    };
+    auto begin = [&](int g) {
+        i0 = (jlo - jpar) / STEP + (HI2LO ? nblk - 1 - g : g) * B;
         // chunk c covers positions cE .. cE + E - 1 (hi2lo, from the highest with a rotation down)
         // or cE - 1 .. cE + E - 2 (lo2hi, from 0 up), aligned as the skewed table is
         const int last = Geo::chain_len(KIND, N, 0) - 1;
         const int emax = max(0, min(last, Geo::top(KIND, N, jpar + STEP * i0, 0) + 1));
-        const int chi = HI2LO ? emax / E : (emax + 1) / E;
-        const int K = chi + 1 + D;
+        chi = HI2LO ? emax / E : (emax + 1) / E;
+        K = chi + 1 + D;
         const int beta = i0 / Geo::kSkewRows;
-        const int nk = beta < Geo::skew_blocks(KIND, N, jpar) ? Geo::skew_chunks(KIND, N, jpar, beta) : 0;
-        const double2 * const rows = F.sc + Geo::skew_at(KIND, N, jpar, beta);
-        auto stage_sc = [&](int k) -> bool {
-            const int kappa = HI2LO ? chi + D - k : k;
-            if (k >= K || kappa >= nk) return false;
-            if (lane == 0) {
-                uint64_t * const bar = &bars[sc_issued % SCS];
-                tc::mbar_arrive_expect_tx(bar, (uint32_t) (SCLEN * sizeof(double2)));
-                tc::bulk_g2s(sc_ring + (sc_issued % SCS) * SCLEN, rows + kappa * Geo::skew_chunk(KIND), (uint32_t) (SCLEN * sizeof(double2)), bar);
-            }
-            ++sc_issued;
-            return true;
-        };
-        unsigned live = 0;
+        nk = beta < Geo::skew_blocks(KIND, N, jpar) ? Geo::skew_chunks(KIND, N, jpar, beta) : 0;
+        rows = F.sc + Geo::skew_at(KIND, N, jpar, beta);
+        live = 0;
 #pragma unroll
         for (int i = 0; i + 1 < SCS; ++i) live |= stage_sc(i) ? 1u << i : 0u;
+    };
+    if (warp < nblk) begin(warp);                 // its first pairs land while the columns do
+    // a warp's columns together, so that their loads are in flight at the same time
+    constexpr int SW = ORD * SEGC / W;
+    static_assert(ORD * SEGC % W == 0, "the columns must split evenly over the warps");
+    {
+        const double * from[SW];
+#pragma unroll
+        for (int i = 0; i < SW; ++i) {
+            long long at;
+            from[i] = column_at(warp + i * W, &at) ? F.in + at : nullptr;
+        }
+#pragma unroll 2
+        for (int x = lane; x < len; x += 32) {
+            double v[SW];
+#pragma unroll
+            for (int i = 0; i < SW; ++i) v[i] = from[i] ? __ldcg(from[i] + x) : 0.0;
+#pragma unroll
+            for (int i = 0; i < SW; ++i) col[place(warp + i * W, x)] = v[i];
+        }
+    }
+    __syncthreads();
+
+    const int c_lane = lane % CH, m_lane = mbase + STEP * (lane / (CH * NC));
+    const int me_lane = KIND == SPIN ? abs(m_lane - F.spin) : m_lane;
+    const int jcut = F.blk > 0 ? m_lane - STEP * (((m_lane - jpar) / STEP) % F.blk) : jpar;
+    for (int g = warp; g < nblk; g += W) {
         unsigned lane_mask = 0;
 #pragma unroll
         for (int b = 0; b < B; ++b) {
@@ -934,6 +954,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
             __syncwarp();
             if (lane == 0 && has_out) publish_word(&prog[warp], g * 4096 + (k + 1 == K ? 4095 : HI2LO ? 2048 - cout : cout + 1));
         }
+        if (g + W < nblk) begin(g + W);
     }
     for (; sc_used != sc_issued; ++sc_used) {     // only after a wait that ran out: no copy may outlive the CTA
         const long long t0 = clock64();
