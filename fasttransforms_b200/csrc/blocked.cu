@@ -993,7 +993,8 @@ size_t blocked_mixed_T_elems(void * plan, int ntasks, int N) {
 }
 
 // S (the fields' FP64 matrices) <-> T (task-major FP32 copy of the columns the
-// blocks apply to); one CTA per (task, 32 positions of both slots).
+// blocks apply to); one CTA per (task, 32 positions of both slots).  Bound: DRAM.  The columns' places
+// are worked out once a CTA (per element they took as long as the copies).
 struct TransLaunch {
     double * A[kMaxFields];
     int nf, N, M, Lq;
@@ -1007,6 +1008,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __grid_constant__ 
     // [row of the chunk][column]; chunk row rr holds position pl = 0 .. 31 of the chunk in
     // slot c: rr = 2 pl + c (sph: the rows of the matrix in order) or 32 c + pl
     __shared__ float tile[64][MX_COLS + 1];
+    __shared__ double * s_col[2][MX_COLS];              // first row of the columns of slot c
     const BlkTask t = L.tasks[blockIdx.x];
     const int q = blockIdx.y;                           // positions 32q .. 32q + 31
     const int tid = threadIdx.x;
@@ -1019,14 +1021,28 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __grid_constant__ 
     const int rr = tid & 63;
     const int c_r = two ? (rr & 1) : (rr >> 5), pl_r = two ? (rr >> 1) : (rr & 31);
     const int row = L.sh.row(32 * q + pl_r, c_r);        // matrix row of chunk row rr
+    {
+        int f;
+        const int c = tid >> 7, i = tid & (MX_COLS - 1);
+        const long long col = L.sh.column(t, MX_COLS, c, i, mlast, f);
+        s_col[c][i] = (col >= 0 && f < L.nf) ? L.A[f] + col * N : nullptr;
+    }
+    __syncthreads();
+    // eight columns a thread at a time, so that as many loads are in flight
     if (TO_T) {
-        for (int i = tid >> 6; i < MX_COLS; i += 4) {
-            int f;
-            const long long col = L.sh.column(t, MX_COLS, c_r, i, mlast, f);
-            tile[rr][i] = (col >= 0 && f < L.nf && row < N) ? (float) __ldcg(L.A[f] + col * N + row) : 0.0f;
+        for (int i0 = tid >> 6; i0 < MX_COLS; i0 += 32) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const double * const col = s_col[c_r][i0 + 4 * u];
+                v[u] = (col && row < N) ? __ldcg(col + row) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) tile[rr][i0 + 4 * u] = (float) v[u];
         }
         __syncthreads();
         const int i = tid & (MX_COLS - 1);
+#pragma unroll
         for (int e = tid >> 7; e < 16; e += 2) {       // e = 2 * (quad - 8q) + c
             const int c = e & 1, qd = e >> 1, Q = 8 * q + qd;
             if (Q < L.Lq) {
@@ -1036,18 +1052,23 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __grid_constant__ 
             }
         }
     } else {
-        const int i = tid & (MX_COLS - 1);
-        for (int e = tid >> 7; e < 16; e += 2) {       // e = 2 * (quad - 8q) + c
-            const int c = e & 1, qd = e >> 1, Q = 8 * q + qd;
-            const float4 v = Q < L.Lq ? __ldcg(reinterpret_cast<const float4 *>(Tt + at(c, 4 * Q, i))) : make_float4(0.f, 0.f, 0.f, 0.f);
-            tile[chunk_row(c, 4 * qd)][i] = v.x; tile[chunk_row(c, 4 * qd + 1)][i] = v.y;
-            tile[chunk_row(c, 4 * qd + 2)][i] = v.z; tile[chunk_row(c, 4 * qd + 3)][i] = v.w;
+        const int i = tid & (MX_COLS - 1), c = tid >> 7;
+        float4 v[8];
+#pragma unroll
+        for (int qd = 0; qd < 8; ++qd) {
+            const int Q = 8 * q + qd;
+            v[qd] = Q < L.Lq ? __ldcg(reinterpret_cast<const float4 *>(Tt + at(c, 4 * Q, i))) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int qd = 0; qd < 8; ++qd) {
+            tile[chunk_row(c, 4 * qd)][i] = v[qd].x; tile[chunk_row(c, 4 * qd + 1)][i] = v[qd].y;
+            tile[chunk_row(c, 4 * qd + 2)][i] = v[qd].z; tile[chunk_row(c, 4 * qd + 3)][i] = v[qd].w;
         }
         __syncthreads();
+#pragma unroll 8
         for (int i2 = tid >> 6; i2 < MX_COLS; i2 += 4) {
-            int f;
-            const long long col = L.sh.column(t, MX_COLS, c_r, i2, mlast, f);
-            if (col >= 0 && f < L.nf && row < N) __stcg(L.A[f] + col * N + row, (double) tile[rr][i2]);
+            double * const col = s_col[c_r][i2];
+            if (col && row < N) __stcg(col + row, (double) tile[rr][i2]);
         }
     }
 }

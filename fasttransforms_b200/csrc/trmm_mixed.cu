@@ -511,67 +511,66 @@ struct SliceX8Launch {
     double * inv;                       // [field][cls][jt][TBN]: 1 / sX per column
 };
 
-// One warp per input column: its power-of-two scale over all n rows.
-__global__ void column_scale_kernel(const __grid_constant__ SliceX8Launch L, int TBN) {
-    const int lane = threadIdx.x & 31;
-    const long long w = (long long) blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const long long per_f = (long long) L.ncls * L.njt * TBN;
-    if (w >= per_f * L.nf) return;                     // the whole warp: w is uniform
-    const int f = (int) (w / per_f);
-    const long long rem = w % per_f;
-    const int r = (int) (rem / ((long long) L.njt * TBN)), j = (int) (rem % ((long long) L.njt * TBN));
-    double amax = 0.0;
-    if (j < class_cols(L.M, r, L.ncls)) {
-        const double * col = L.in[f] + (long long) (r + (long long) L.ncls * j) * L.n;
-        for (int k = lane; k < L.n; k += 32) amax = fmax(amax, fabs(__ldcg(col + k)));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    int ex = 0;
-    if (amax > 0) (void) frexp(amax, &ex);
-    if (lane == 0) L.inv[w] = amax > 0 ? ldexp(1.0, ex - 6) : 1.0;   // 1 / s, |s x| < 64
-}
-
-// One CTA per (field, class, column tile, 256 rows), one warp per column at a time, each lane
-// 8 consecutive rows: NX digits into the column's row of the K-tile pieces.
+// One CTA per (field, class, column tile) and kSliceCols columns of it, one warp per column at a time:
+// the column's power-of-two scale over all n rows, then its digits, each lane 8 consecutive rows of
+// every 256, into the column's row of the K-tile pieces.  The second reading of a column finds it in
+// L2.  Bound: DRAM, a column read and its digits written once (with the scales in a kernel of their
+// own the input was read twice: 2.0 ms for 16 sph fields of degree 4095).
+constexpr int kSliceCols = 32;
 template <int NX, int TBN>
 __global__ void __launch_bounds__(256) slice_input_s8_kernel(const __grid_constant__ SliceX8Launch L) {
     constexpr int XPIECE = TBN * KT8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nch = (L.nkt + 3) / 4;                    // 256-row chunks: four K-tiles of 64
     int b = blockIdx.x;
-    const int q = b % nch; b /= nch;
     const int jt = b % L.njt; b /= L.njt;
     const int r = b % L.ncls;
     const int f = b / L.ncls;
     const int ncols = class_cols(L.M, r, L.ncls);
     const long long tile_base = ((long long) (f * L.ncls + r) * L.njt + jt);
-    const int kt = q * 4 + lane / 8;                    // K-tile of this lane's 8 rows
-    const int kb = 8 * (lane % 8);                      // their first byte in the 64-byte row
-    if (kt >= L.nkt) return;
-    for (int ci = warp; ci < TBN; ci += 8) {
+    const int kb = 8 * (lane % 8);                      // first byte of the lane's rows in the 64-byte row
+    for (int ci = blockIdx.y * kSliceCols + warp; ci < min(TBN, ((int) blockIdx.y + 1) * kSliceCols); ci += 8) {
         const int j = jt * TBN + ci;
         const bool cok = j < ncols;
-        const double s = 1.0 / L.inv[tile_base * TBN + ci];
         const double * col = L.in[f] + (long long) (r + (long long) L.ncls * j) * L.n;
-        uint32_t w[NX][2];
-#pragma unroll
-        for (int a = 0; a < NX; ++a) { w[a][0] = 0u; w[a][1] = 0u; }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int row = kt * KT8 + kb + e;
-            double t = (cok && row < L.n) ? __ldcg(col + row) * s : 0.0;
-#pragma unroll
-            for (int a = 0; a < NX; ++a) {
-                const double i = rint(t);
-                w[a][e >> 2] |= ((uint32_t) (int) i & 0xFFu) << (8 * (e & 3));
-                t = (t - i) * 128.0;
-            }
+        double amax = 0.0;
+        if (cok) {
+#pragma unroll 8
+            for (int k = lane; k < L.n; k += 32) amax = fmax(amax, fabs(__ldcg(col + k)));
         }
-        unsigned char * base = L.img + (tile_base * L.nkt + kt) * NX * XPIECE;
-        const uint32_t off = tc::sw64_byte(ci, kb);
 #pragma unroll
-        for (int a = 0; a < NX; ++a) *reinterpret_cast<uint2 *>(base + a * XPIECE + off) = make_uint2(w[a][0], w[a][1]);
+        for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        int ex = 0;
+        if (amax > 0) (void) frexp(amax, &ex);
+        const double inv = amax > 0 ? ldexp(1.0, ex - 6) : 1.0;   // 1 / s, |s x| < 64
+        const double s = 1.0 / inv;
+        if (lane == 0) L.inv[tile_base * TBN + ci] = inv;
+        const uint32_t off = tc::sw64_byte(ci, kb);
+        for (int kt = lane / 8; kt < L.nkt; kt += 4) {  // K-tile of the lane's 8 rows
+            const int row0 = kt * KT8 + kb;
+            double x[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = (cok && row0 + e < L.n) ? __ldg(col + row0 + e) * s : 0.0;
+            uint32_t w[NX][2];
+#pragma unroll
+            for (int a = 0; a < NX; ++a) { w[a][0] = 0u; w[a][1] = 0u; }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                double t = x[e];
+                double unit = 1.5 * 4503599627370496.0;   // 1.5 * 2^52, then 2^-7 of it a digit
+#pragma unroll
+                for (int a = 0; a < NX; ++a, unit *= 0.0078125) {
+                    // adding it rounds t to the nearest multiple of 2^(-7 a), ties to even, and leaves
+                    // that multiple in the low bits; subtracting it back and from t is exact (rint and
+                    // the conversion run at a fraction of the addition's rate)
+                    const double u = __dadd_rn(t, unit);
+                    w[a][e >> 2] |= ((uint32_t) __double2loint(u) & 0xFFu) << (8 * (e & 3));
+                    t = __dsub_rn(t, __dsub_rn(u, unit));
+                }
+            }
+            unsigned char * base = L.img + (tile_base * L.nkt + kt) * NX * XPIECE;
+#pragma unroll
+            for (int a = 0; a < NX; ++a) *reinterpret_cast<uint2 *>(base + a * XPIECE + off) = make_uint2(w[a][0], w[a][1]);
+        }
     }
 }
 
@@ -911,21 +910,16 @@ cudaError_t launch_trmm_s8(HarmonicPlan * H, MixedTrmmPlan * T, MixedTrmmWork * 
             if (e != cudaSuccess) return e;
         }
     }
-    // the input's column scales, then its digits
+    // the input's column scales and digits
     static thread_local SliceX8Launch SX;
     for (int f = 0; f < nf; ++f) SX.in[f] = in[f];
     SX.nf = nf; SX.n = n; SX.M = M; SX.nkt = nkt; SX.njt = X.njt; SX.ncls = ncls;
     SX.img = X.ximg; SX.inv = X.xinv;
-    const long long ncolw = (long long) nf * ncls * X.njt * tbn;        // one warp per column
-    column_scale_kernel<<<(unsigned) ((ncolw + 7) / 8), 256, 0, st>>>(SX, tbn);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const int sgrid = nf * ncls * X.njt * ((nkt + 3) / 4);
+    const dim3 sgrid((unsigned) (nf * ncls * X.njt), (unsigned) ((tbn + kSliceCols - 1) / kSliceCols));
     if (cfg) slice_input_s8_kernel<5, TBN8_5><<<sgrid, 256, 0, st>>>(SX);
     else     slice_input_s8_kernel<4, TBN8_4><<<sgrid, 256, 0, st>>>(SX);
     count_launch();
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     static thread_local Mix8Launch L;
     for (int f = 0; f < nf; ++f) L.out[f] = out[f];
