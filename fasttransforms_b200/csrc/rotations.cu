@@ -810,6 +810,8 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
     __shared__ int prog[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+    allow_next();
+    wait_for_previous();
     if (L.lead > L.lead0) copy_lead(L);
     const RotTask task = L.tasks[blockIdx.x / R::SPLIT];
     const RotField & F = L.fields[task.field];
@@ -992,9 +994,8 @@ cudaError_t launch_resident(const RotLaunch & L, cudaStream_t st) {
         if (e != cudaSuccess) return e;
         if (dev < 16) ready[dev].store(true, std::memory_order_release);
     }
-    kern<<<L.ntasks * R::SPLIT, R::W * 32, R::bytes(nmax), st>>>(L);
     count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(kern, dim3(L.ntasks * R::SPLIT), R::W * 32, R::bytes(nmax), st, L);
 }
 
 }  // namespace

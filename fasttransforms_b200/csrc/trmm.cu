@@ -281,6 +281,8 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
 template <int S, bool A_MC, bool B_KC, bool VEC16>
 __global__ void __launch_bounds__(TileLayout<S, A_MC, B_KC>::THREADS, TileShape<S>::CTAS)
 gemm_tri_kernel(const __grid_constant__ GemmParams P) {
+    allow_next();
+    wait_for_previous();
     // block -> (tile along the triangle, class, other tile): tiles with the most K work first,
     // whatever their class
     const int along = P.mode < 2 ? P.tiles_m : P.tiles_n, across = P.mode < 2 ? P.tiles_n : P.tiles_m;
@@ -296,6 +298,8 @@ gemm_tri_kernel(const __grid_constant__ GemmParams P) {
 template <int S, int MODE, bool VEC16>
 __global__ void __launch_bounds__(TileLayout<S, MODE != 1, MODE != 3>::THREADS, TileShape<S>::CTAS)
 gemm_tri_batched_kernel(const __grid_constant__ TrmmBatch P) {
+    allow_next();
+    wait_for_previous();
     const TrmmTile t = P.tiles[blockIdx.x];
     const TrmmBatchClass c = P.classes[t.cls];
     GemmClass C;
@@ -311,8 +315,8 @@ gemm_tri_batched_kernel(const __grid_constant__ TrmmBatch P) {
 }
 
 // One launch; the kernel's shared-memory limit is raised once per device.
-template <class K, class P>
-cudaError_t launch_tiles(K kern, const P & p, int blocks, int threads, size_t shm, std::atomic<unsigned> & ready, cudaStream_t st) {
+template <class P>
+cudaError_t launch_tiles(void (*kern)(P), const P & p, int blocks, int threads, size_t shm, std::atomic<unsigned> & ready, cudaStream_t st) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -322,9 +326,8 @@ cudaError_t launch_tiles(K kern, const P & p, int blocks, int threads, size_t sh
         if (e != cudaSuccess) return e;
         ready.fetch_or(bit, std::memory_order_release);
     }
-    kern<<<blocks, threads, shm, st>>>(p);
     count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(kern, dim3(blocks), threads, shm, st, p);
 }
 
 template <int S, int MODE, bool VEC16>
@@ -367,6 +370,8 @@ struct NormLaunch {
     int N[kMaxFields], M[kMaxFields];
 };
 __global__ void cheb_norm_kernel(const __grid_constant__ NormLaunch L, double r, double g) {
+    allow_next();
+    wait_for_previous();
     // src/drivers.c:6-24: first column and first row scaled by r (entry (0,0) twice), all by g
     double * const A = L.A[blockIdx.y];
     const int N = L.N[blockIdx.y];
@@ -440,9 +445,8 @@ cudaError_t launch_cheb_normalize(double * const * A, const int * N, const int *
     }
     // four elements a thread, up to four CTAs per SM over all fields
     const int blocks = (int) std::max(1LL, std::min((most + 1023) / 1024, (long long) (592 / nf + 1)));
-    cheb_norm_kernel<<<dim3(blocks, nf), 256, 0, st>>>(L, r, g);
     count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(cheb_norm_kernel, dim3(blocks, nf), 256, 0, st, L, r, g);
 }
 
 }  // namespace ftb
