@@ -16,17 +16,30 @@
 //
 // The cosine transforms go through complex FFTs of length N (Makhoul's reordering):
 //   DCT-II:  v = (x_0, x_2, x_4, .., x_5, x_3, x_1), V = DFT(v),
-//            y_k = 2 Re(exp(-i pi k / 2N) V_k);
-//   DCT-III: V_k = (y_k - i y_{N-k}) exp(i pi k / 2N) (y_N = 0), a Hermitian
-//            spectrum, v = unnormalised inverse DFT(V), x = v un-permuted;
+//            y_k = exp(-i pi k / 2N) V_k + exp(i pi k / 2N) V_{N-k}
+//                  (2 Re(exp(-i pi k / 2N) V_k) for real x);
+//   DCT-III: V_k = (y_k - i y_{N-k}) exp(i pi k / 2N) (y_N = 0; Hermitian for real y),
+//            v = unnormalised inverse DFT(V), x = v un-permuted;
 // and the sine transforms through them: DST-II(x)_k = DCT-II((-1)^n x_n)_{N-1-k},
 // DST-III(x)_k = (-1)^k DCT-III(x reversed)_k.  The DFTs are cuFFT's (library
-// FFTs, batched over all M columns at once); the reorderings, twiddles, scalings and
+// FFTs, batched over all columns at once); the reorderings, twiddles, scalings and
 // the half-spectrum packing are this file's kernels.
+//
+// The sphere's stages run on complex data throughout.  Around a real DFT of odd length (M is odd, and N
+// often is) the library runs passes of its own, and the kernels here read and wrote the matrix once
+// more on each side.  Columns 2j - 1 and 2j have the same kind and are the two parts of frequency j, so
+// the theta stage transforms the (M + 1) / 2 complex columns X(2j) - i X(2j - 1) (the transforms are
+// linear); the phi stage transforms rows 2p and 2p + 1 as one complex row (of the disk and the annulus
+// too).  The kernel between the two DFTs goes from one form to the other and leaves X alone.  What is
+// left is the library's DFTs (of prime lengths by Bluestein's algorithm, 190 of 343 us below) and four
+// or five passes at 4 - 6 TB/s.  Synthesis and analysis together, us: n = 64 58 -> 50, 300 80 -> 50, 301
+// 107 -> 68, 1024 248 -> 167, 1501 837 -> 687, 2400 1726 -> 1292, 4096 3740 -> 2743.  Errors against
+// long double sums, relative 2-norm, n = 33 .. 2000: 2.4e-16 .. 7.9e-16, as before (2.6e-16 .. 7.8e-16).
 //
 // The spin-weighted sphere's grid (a complex N x M matrix, src/fftw.c:755-960) runs the same
 // theta stage on the 2M real columns of its split parts, and a complex DFT along the rows around
 // the reference's column permutation (columns 2j and 2j - 1 to j and M - j).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -79,14 +92,14 @@ struct SphereGridPlan {
     int device = 0;
     cufftHandle t_r2c = 0;       // length N, batch M (cosine type II)
     cufftHandle t_c2r = 0;       // length N, batch M (cosine type III)
-    cufftHandle p_r2c = 0;       // length M along rows, batch N
-    cufftHandle p_c2r = 0;
-    cufftHandle p_z2z = 0;       // spin: complex DFT of length M along rows, batch N
-    bool have_t_r2c = false, have_t_c2r = false, have_p_r2c = false, have_p_c2r = false, have_p_z2z = false;
+    cufftHandle t_z2z = 0;       // sphere: length N, batch M / 2 + 1 complex columns
+    cufftHandle p_z2z = 0;       // complex DFT of length M along rows: (N + 1) / 2 pairs of rows (spin: N rows)
+    bool have_t_r2c = false, have_t_c2r = false, have_t_z2z = false, have_p_z2z = false;
     // (spin: the theta stage runs on 2M real columns, so the work buffers below hold 2M columns)
-    double * d_work = nullptr;   // N x M real
-    double2 * d_cwork = nullptr; // (N/2 + 1) x M complex
-    double2 * d_Y = nullptr;     // N x (M/2 + 1) complex, element (i, j) at i + j N (spin: N x M)
+    double * d_work = nullptr;   // N x M real (not the sphere)
+    double2 * d_cwork = nullptr; // (N/2 + 1) x M complex: the theta stage's spectra; the phi stage's row pairs
+    double2 * d_Y = nullptr;     // sphere: N x (M/2 + 1) complex columns; spin: N x M
+    double2 * d_tw = nullptr;    // sphere: (cos, sin)(pi k / 2N), k < N
     double * d_stage = nullptr;  // N x M, host-pointer calls
     // disk: the DCT-IV of the columns of classes 1 and 2 (nq of them) as a zero-padded complex
     // DFT of length 2N
@@ -102,7 +115,7 @@ struct SphereGridPlan {
 namespace {
 
 // ---------------------------------------------------------------------------
-// theta stage kernels: one thread per (entry, column); column j uses the kind of
+// theta stage kernels of the other families: one thread per (entry, column); column j uses the kind of
 // its class, cls(j) = j mod 4 in {0, 3} -> kind[0], {1, 2} -> kind[1]
 // ---------------------------------------------------------------------------
 // k1dst bit 1 set: the classes are the even and odd columns instead (the rectangularised disk's);
@@ -277,28 +290,199 @@ __global__ void tri_scale(double * X, int N, int M, double ef, double s, double 
 // ---------------------------------------------------------------------------
 // phi stage packing and the scalings
 // ---------------------------------------------------------------------------
-// Y(i, 0) = (s X(i, 0)) f0; Y(i, j) = s (X(i, 2j) - i X(i, 2j - 1)), j = 1 .. M/2
-__global__ void pack_r2c(const double * __restrict__ X, double2 * __restrict__ Y, int N, int M, double s, double f0) {
-    const int H = M / 2 + 1;
-    const long long idx = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long) N * H) return;
-    const int j = (int) (idx / N), i = (int) (idx % N);
-    double2 v;
-    if (j == 0) v = make_double2((s * X[i]) * f0, 0.0);
-    else        v = make_double2(s * X[i + (long long) (2 * j) * N], -s * X[i + (long long) (2 * j - 1) * N]);
-    Y[idx] = v;
+// The phi spectrum of X: F(i, 0) = (s X(i, 0)) f0, F(i, j) = s (X(i, 2j) - i X(i, 2j - 1)), j = 1 ..
+// M/2, and X from F by the same formula read backwards (Re F(i, 0) for column 0).  Its rows are held
+// in pairs: Z(p, j) = F(2p, j) + i F(2p + 1, j) for all M frequencies j, F(i, M - j) = conj(F(i, j)), so
+// Z's DFT along the rows is x(2p, .) + i x(2p + 1, .).  Z is NP x M, NP = (N + 1) / 2; row N of an odd N is 0.
+//
+// A thread of the kernels below has a pair (k, k') of rows (or of spectrum entries) of column j, so
+// that each of its complex numbers is read once; blockIdx.x runs over the columns (up to 2^31 of them),
+// blockIdx.y and a loop over the rows, 64 threads each, two columns a block.
+struct Ends { int row, odd; double f; };   // X's entries of that row in the columns of odd / even j times f
+struct Phi { double s, f0; };
+
+constexpr int kGridRows = 64, kGridCols = 2;
+
+__device__ __forceinline__ double2 take_x(const double * __restrict__ X, int N, int j, int i, Ends e) {
+    double2 v = j == 0 ? make_double2(X[i], 0.0)
+                       : make_double2(X[(long long) (2 * j) * N + i], -X[(long long) (2 * j - 1) * N + i]);
+    if (i == e.row && (j & 1) == e.odd) { v.x *= e.f; v.y *= e.f; }
+    return v;
+}
+__device__ __forceinline__ void put_x(double * __restrict__ X, int N, int j, int i, double2 v, Ends e) {
+    if (i == e.row && (j & 1) == e.odd) { v.x *= e.f; v.y *= e.f; }
+    if (j == 0) { X[i] = v.x; return; }
+    X[(long long) (2 * j) * N + i] = v.x;
+    X[(long long) (2 * j - 1) * N + i] = -v.y;
+}
+// F(2p, j) and F(2p + 1, j), scaled, from the pair's spectrum
+__device__ __forceinline__ void take_pair(const double2 * __restrict__ Z, int NP, int M, int j, int p, Phi h, double2 & u, double2 & v) {
+    const double2 a = Z[(long long) j * NP + p];
+    if (j == 0) {
+        u = make_double2((h.s * a.x) * h.f0, 0.0);
+        v = make_double2((h.s * a.y) * h.f0, 0.0);
+        return;
+    }
+    const double2 b = Z[(long long) (M - j) * NP + p];
+    const double t = 0.5 * h.s;
+    u = make_double2(t * (a.x + b.x), t * (a.y - b.y));
+    v = make_double2(t * (a.y + b.y), t * (b.x - a.x));
+}
+__device__ __forceinline__ void put_pair(double2 * __restrict__ Z, int NP, int M, int j, int p, Phi h, double2 u, double2 v) {
+    if (j == 0) {
+        Z[p] = make_double2((h.s * u.x) * h.f0, (h.s * v.x) * h.f0);
+        return;
+    }
+    u.x *= h.s; u.y *= h.s; v.x *= h.s; v.y *= h.s;
+    Z[(long long) j * NP + p] = make_double2(u.x - v.y, u.y + v.x);
+    Z[(long long) (M - j) * NP + p] = make_double2(u.x + v.y, v.x - u.y);
 }
 
-// X(i, 0) = (s Re Y(i, 0)) f0; X(i, 2j) = s Re Y(i, j); X(i, 2j - 1) = s (-Im Y(i, j))
-__global__ void unpack_c2r(const double2 * __restrict__ Y, double * __restrict__ X, int N, int M, double s, double f0) {
-    const int H = M / 2 + 1;
-    const long long idx = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long) N * H) return;
-    const int j = (int) (idx / N), i = (int) (idx % N);
-    const double2 v = Y[idx];
-    if (j == 0) { X[i] = (s * v.x) * f0; return; }
-    X[i + (long long) (2 * j) * N] = s * v.x;
-    X[i + (long long) (2 * j - 1) * N] = -s * v.y;
+// X -> Z
+__global__ void pack_pairs(const double * __restrict__ X, double2 * __restrict__ Z, int N, int M, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows)
+        put_pair(Z, NP, M, j, p, h, take_x(X, N, j, 2 * p, Ends{-1, 0, 1.0}),
+                 2 * p + 1 < N ? take_x(X, N, j, 2 * p + 1, Ends{-1, 0, 1.0}) : make_double2(0.0, 0.0));
+}
+// Z -> X
+__global__ void unpack_pairs(const double2 * __restrict__ Z, double * __restrict__ X, int N, int M, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows) {
+        double2 u, v;
+        take_pair(Z, NP, M, j, p, h, u, v);
+        put_x(X, N, j, 2 * p, u, Ends{-1, 0, 1.0});
+        if (2 * p + 1 < N) put_x(X, N, j, 2 * p + 1, v, Ends{-1, 0, 1.0});
+    }
+}
+// The rows themselves: Z(p, k) = X(2p, k) + i X(2p + 1, k) (odd N, or X not 16-byte aligned; else the
+// matrix is already laid out like this), and back
+__global__ void join_rows(const double * __restrict__ X, double2 * __restrict__ Z, int N, int M) {
+    const int k = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (k >= M) return;
+    const double * const x = X + (long long) k * N;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows)
+        Z[(long long) k * NP + p] = make_double2(x[2 * p], 2 * p + 1 < N ? x[2 * p + 1] : 0.0);
+}
+__global__ void split_rows(const double2 * __restrict__ Z, double * __restrict__ X, int N, int M) {
+    const int k = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (k >= M) return;
+    double * const x = X + (long long) k * N;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows) {
+        const double2 z = Z[(long long) k * NP + p];
+        x[2 * p] = z.x;
+        if (2 * p + 1 < N) x[2 * p + 1] = z.y;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The sphere's theta stage on the complex columns C (N x (M/2 + 1)).  Column j takes kind j & 1, a
+// sine transform where that bit of `dst` is set.
+// ---------------------------------------------------------------------------
+__global__ void twiddles(double2 * tw, int N) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= N) return;
+    double s, c;
+    sincospi((double) k / (2.0 * N), &s, &c);
+    tw[k] = make_double2(c, s);
+}
+
+// Before the DFT, from X (rows scaled by e) or from the phi spectrum (FROM_Z).
+// Type II: entry n of C is row 2n or 2 (N - 1 - n) + 1, so a thread takes rows 2p and 2p + 1.
+template <bool FROM_Z>
+__global__ void t2_pre_c(const double * __restrict__ X, const double2 * __restrict__ Z, double2 * __restrict__ C, int N, int M,
+                         int dst, Ends e, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    const bool sine = (dst >> (j & 1)) & 1;
+    double2 * const c = C + (long long) j * N;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows) {
+        double2 u, v = make_double2(0.0, 0.0);
+        if (FROM_Z) take_pair(Z, NP, M, j, p, h, u, v);
+        else {
+            u = take_x(X, N, j, 2 * p, e);
+            if (2 * p + 1 < N) v = take_x(X, N, j, 2 * p + 1, e);
+        }
+        c[p] = u;
+        if (2 * p + 1 < N) c[N - 1 - p] = sine ? make_double2(-v.x, -v.y) : v;   // (-1)^n x_n
+    }
+}
+// Type III: V_k = (y_k - i y_{N-k}) exp(i pi k / 2N), with y reversed for sine columns; a thread takes k
+// and N - k.
+template <bool FROM_Z>
+__global__ void t3_pre_c(const double * __restrict__ X, const double2 * __restrict__ Z, double2 * __restrict__ C,
+                         const double2 * __restrict__ tw, int N, int M, int dst, Ends e, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    const bool sine = (dst >> (j & 1)) & 1;
+    double2 * const c = C + (long long) j * N;
+    auto y = [&](int t) {
+        const int i = sine ? N - 1 - t : t;
+        if (!FROM_Z) return take_x(X, N, j, i, e);
+        double2 u, v;
+        take_pair(Z, NP, M, j, i >> 1, h, u, v);
+        return (i & 1) ? v : u;
+    };
+    for (int k = blockIdx.y * kGridRows + threadIdx.x; k <= N / 2; k += gridDim.y * kGridRows) {
+        const double2 a = y(k), b = k == 0 ? make_double2(0.0, 0.0) : y(N - k);
+        auto turned = [&](double2 p, double2 q, double2 w) {   // (p - i q) w
+            const double re = p.x + q.y, im = p.y - q.x;
+            return make_double2(re * w.x - im * w.y, re * w.y + im * w.x);
+        };
+        c[k] = turned(a, b, tw[k]);
+        if (k > 0 && k < N - k) c[N - k] = turned(b, a, tw[N - k]);
+    }
+}
+// After the DFT, to X (rows scaled by e) or to the phi spectrum (TO_Z).
+// Type II: y_k = exp(-i pi k / 2N) V_k + exp(i pi k / 2N) V_{N-k}, reversed for sine columns.  To X a
+// thread takes k and N - k, to the spectrum the rows 2p and 2p + 1.
+__device__ __forceinline__ double2 t2_value(double2 v, double2 w, double2 t) {
+    return make_double2(t.x * (v.x + w.x) + t.y * (v.y - w.y), t.x * (v.y + w.y) - t.y * (v.x - w.x));
+}
+template <bool TO_Z>
+__global__ void t2_post_c(const double2 * __restrict__ C, double * __restrict__ X, double2 * __restrict__ Z,
+                          const double2 * __restrict__ tw, int N, int M, int dst, Ends e, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    const bool sine = (dst >> (j & 1)) & 1;
+    const double2 * const c = C + (long long) j * N;
+    if (TO_Z) {
+        auto row = [&](int i) {
+            const int k = sine ? N - 1 - i : i;
+            return t2_value(c[k], c[k == 0 ? 0 : N - k], tw[k]);
+        };
+        for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows)
+            put_pair(Z, NP, M, j, p, h, row(2 * p), 2 * p + 1 < N ? row(2 * p + 1) : make_double2(0.0, 0.0));
+    } else {
+        for (int k = blockIdx.y * kGridRows + threadIdx.x; k <= N / 2; k += gridDim.y * kGridRows) {
+            const int m = k == 0 ? 0 : N - k;
+            const double2 v = c[k], w = c[m];
+            put_x(X, N, j, sine ? N - 1 - k : k, t2_value(v, w, tw[k]), e);
+            if (k > 0 && k < m) put_x(X, N, j, sine ? N - 1 - m : m, t2_value(w, v, tw[m]), e);
+        }
+    }
+}
+// Type III: rows 2p and 2p + 1 are entries p and N - 1 - p; (-1)^row for sine columns.
+template <bool TO_Z>
+__global__ void t3_post_c(const double2 * __restrict__ C, double * __restrict__ X, double2 * __restrict__ Z, int N, int M,
+                          int dst, Ends e, Phi h) {
+    const int j = blockIdx.x * kGridCols + threadIdx.y, NP = (N + 1) / 2;
+    if (j > M / 2) return;
+    const bool sine = (dst >> (j & 1)) & 1;
+    const double2 * const c = C + (long long) j * N;
+    for (int p = blockIdx.y * kGridRows + threadIdx.x; p < NP; p += gridDim.y * kGridRows) {
+        const double2 u = c[p];
+        double2 v = make_double2(0.0, 0.0);
+        if (2 * p + 1 < N) v = c[N - 1 - p];
+        if (sine) { v.x = -v.x; v.y = -v.y; }
+        if (TO_Z) put_pair(Z, NP, M, j, p, h, u, v);
+        else {
+            put_x(X, N, j, 2 * p, u, e);
+            if (2 * p + 1 < N) put_x(X, N, j, 2 * p + 1, v, e);
+        }
+    }
 }
 
 // Multiplies the first (last = 0) or last (last = 1) entry of the columns
@@ -370,6 +554,12 @@ bool fok(cufftResult r, const char * what) {
 }
 
 unsigned blocks(long long n) { return (unsigned) ((n + 255) / 256); }
+// columns and rows (in pairs) of the complex kernels; a thread runs up to four of its rows' places
+dim3 col_blocks(int cols, int places) {
+    return dim3((unsigned) ((cols + kGridCols - 1) / kGridCols),
+                (unsigned) std::min(65535, (places + 4 * kGridRows - 1) / (4 * kGridRows)));
+}
+const dim3 kGridBlock(kGridRows, kGridCols);
 
 SphereGridPlan * make_plan(int N, int M, int k0, int k1, int family = F_SPHERE, int krows = 0, double rho = 0.0) {
     clear_error();
@@ -395,9 +585,11 @@ SphereGridPlan * make_plan(int N, int M, int k0, int k1, int family = F_SPHERE, 
     const bool spin = family == F_SPIN;
     const int TM = spin ? 2 * M : M;   // real columns of the theta stage
     const size_t nm = (size_t) N * TM;
-    bool good = ok(cudaMalloc(&P->d_work, sizeof(double) * nm), "cudaMalloc(grid work)") &&
+    const bool sphere = family == F_SPHERE;
+    bool good = (sphere || ok(cudaMalloc(&P->d_work, sizeof(double) * nm), "cudaMalloc(grid work)")) &&
                 ok(cudaMalloc(&P->d_cwork, sizeof(double2) * (size_t) (N / 2 + 1) * TM), "cudaMalloc(grid work)") &&
-                (nophi || ok(cudaMalloc(&P->d_Y, sizeof(double2) * (size_t) N * (spin ? M : M / 2 + 1)), "cudaMalloc(grid spectrum)")) &&
+                (!(sphere || spin) || ok(cudaMalloc(&P->d_Y, sizeof(double2) * (size_t) N * (spin ? M : M / 2 + 1)), "cudaMalloc(grid spectrum)")) &&
+                (!sphere || ok(cudaMalloc(&P->d_tw, sizeof(double2) * (size_t) N), "cudaMalloc(grid twiddles)")) &&
                 (!(nophi || spin) || ok(cudaMalloc(&P->d_work2, sizeof(double) * nm), "cudaMalloc(grid work)")) &&
                 ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     if (good && family == F_DISK) {
@@ -409,7 +601,14 @@ SphereGridPlan * make_plan(int N, int M, int k0, int k1, int family = F_SPHERE, 
             P->have_t4 = good;
         }
     }
-    if (good) {
+    if (good && sphere) {
+        int n[1] = {N};
+        twiddles<<<blocks(N), 256, 0, P->stream>>>(P->d_tw, N);
+        count_launch();
+        good = ok(cudaGetLastError(), "twiddles") && ok(cudaStreamSynchronize(P->stream), "twiddles") &&
+               fok(cufftPlanMany(&P->t_z2z, 1, n, nullptr, 1, N, nullptr, 1, N, CUFFT_Z2Z, M / 2 + 1), "cufftPlanMany");
+        P->have_t_z2z = good;
+    } else if (good) {
         int n[1] = {N};
         if (is_type3(k0)) {
             good = fok(cufftPlanMany(&P->t_c2r, 1, n, nullptr, 1, N / 2 + 1, nullptr, 1, N, CUFFT_Z2D, TM), "cufftPlanMany");
@@ -435,14 +634,11 @@ SphereGridPlan * make_plan(int N, int M, int k0, int k1, int family = F_SPHERE, 
         good = fok(cufftPlanMany(&P->p_z2z, 1, m, m, N, 1, m, N, 1, CUFFT_Z2Z, N), "cufftPlanMany");
         P->have_p_z2z = good;
     } else if (good && !nophi) {
-        // phi: along rows, element stride N, rows one apart
-        int m[1] = {M}, hm[1] = {M / 2 + 1};
-        good = fok(cufftPlanMany(&P->p_c2r, 1, m, hm, N, 1, m, N, 1, CUFFT_Z2D, N), "cufftPlanMany");
-        P->have_p_c2r = good;
-        if (good) {
-            good = fok(cufftPlanMany(&P->p_r2c, 1, m, m, N, 1, hm, N, 1, CUFFT_D2Z, N), "cufftPlanMany");
-            P->have_p_r2c = good;
-        }
+        // phi: pairs of rows, element stride NP, pairs one apart
+        int m[1] = {M};
+        const int NP = (N + 1) / 2;
+        good = fok(cufftPlanMany(&P->p_z2z, 1, m, m, NP, 1, m, NP, 1, CUFFT_Z2Z, NP), "cufftPlanMany");
+        P->have_p_z2z = good;
     }
     if (!good) {
         ft_destroy_sphere_fftw_plan(reinterpret_cast<ft_sphere_fftw_plan *>(P));
@@ -451,11 +647,11 @@ SphereGridPlan * make_plan(int N, int M, int k0, int k1, int family = F_SPHERE, 
     return P;
 }
 
-// theta transforms of all M columns in place (the plan's kinds by column class; disk: kind[0]
-// on every column here, the DCT-IV of classes 1 and 2 in theta_disk)
+// theta transforms of all M columns in place, for the other families (the plan's kinds by column class;
+// disk: kind[0] on every column here, the DCT-IV of classes 1 and 2 in theta_disk)
 bool theta(SphereGridPlan * P, double * X, cudaStream_t st, bool rows = false) {
     const int N = P->N, M = P->family == F_SPIN ? 2 * P->M : P->M;
-    int d0 = is_dst(P->kind[0]), d1 = P->family == F_SPHERE ? is_dst(P->kind[1]) : d0;
+    int d0 = is_dst(P->kind[0]), d1 = d0;
     if (P->family == F_SPIN) d1 = is_dst(P->kind[1]) | 4;   // W's columns by their complex column's class
     if (P->family == F_RECT) {
         if (rows) { d0 = is_dst(P->kind_rows); d1 = d0; }   // every column of the transposed matrix
@@ -572,22 +768,64 @@ bool tri_scaling(SphereGridPlan * P, double * X, double ef, double s, double d, 
     return ok(cudaGetLastError(), "tri_scale");
 }
 
-bool phi_c2r(SphereGridPlan * P, const double * X, double s, double f0, cudaStream_t st) {
-    const int N = P->N, M = P->M;
-    pack_r2c<<<blocks((long long) N * (M / 2 + 1)), 256, 0, st>>>(X, P->d_Y, N, M, s, f0);
+// The DFT of the row pairs, between their spectrum Z (d_cwork) and the matrix X
+bool rows_are_pairs(const SphereGridPlan * P, const double * X) {
+    return P->N % 2 == 0 && reinterpret_cast<uintptr_t>(X) % sizeof(double2) == 0;
+}
+bool pairs_to_rows(SphereGridPlan * P, double * X, cudaStream_t st) {
+    cufftDoubleComplex * const Z = reinterpret_cast<cufftDoubleComplex *>(P->d_cwork);
+    const bool direct = rows_are_pairs(P, X);
+    if (!fok(cufftSetStream(P->p_z2z, st), "cufftSetStream") ||
+        !fok(cufftExecZ2Z(P->p_z2z, Z, direct ? reinterpret_cast<cufftDoubleComplex *>(X) : Z, CUFFT_INVERSE), "cufftExecZ2Z")) return false;
+    if (direct) return true;
+    split_rows<<<col_blocks(P->M, (P->N + 1) / 2), kGridBlock, 0, st>>>(P->d_cwork, X, P->N, P->M);
     count_launch();
-    if (!ok(cudaGetLastError(), "pack_r2c")) return false;
-    return fok(cufftSetStream(P->p_c2r, st), "cufftSetStream") &&
-           fok(cufftExecZ2D(P->p_c2r, reinterpret_cast<cufftDoubleComplex *>(P->d_Y), const_cast<double *>(X)), "cufftExecZ2D");
+    return ok(cudaGetLastError(), "split_rows");
+}
+bool rows_to_pairs(SphereGridPlan * P, double * X, cudaStream_t st) {
+    cufftDoubleComplex * const Z = reinterpret_cast<cufftDoubleComplex *>(P->d_cwork);
+    const bool direct = rows_are_pairs(P, X);
+    if (!direct) {
+        join_rows<<<col_blocks(P->M, (P->N + 1) / 2), kGridBlock, 0, st>>>(X, P->d_cwork, P->N, P->M);
+        count_launch();
+        if (!ok(cudaGetLastError(), "join_rows")) return false;
+    }
+    return fok(cufftSetStream(P->p_z2z, st), "cufftSetStream") &&
+           fok(cufftExecZ2Z(P->p_z2z, direct ? reinterpret_cast<cufftDoubleComplex *>(X) : Z, Z, CUFFT_FORWARD), "cufftExecZ2Z");
+}
+
+bool phi_c2r(SphereGridPlan * P, double * X, double s, double f0, cudaStream_t st) {
+    pack_pairs<<<col_blocks(P->M / 2 + 1, (P->N + 1) / 2), kGridBlock, 0, st>>>(X, P->d_cwork, P->N, P->M, Phi{s, f0});
+    count_launch();
+    return ok(cudaGetLastError(), "pack_pairs") && pairs_to_rows(P, X, st);
 }
 
 bool phi_r2c(SphereGridPlan * P, double * X, double s, double f0, cudaStream_t st) {
-    const int N = P->N, M = P->M;
-    if (!fok(cufftSetStream(P->p_r2c, st), "cufftSetStream") ||
-        !fok(cufftExecD2Z(P->p_r2c, X, reinterpret_cast<cufftDoubleComplex *>(P->d_Y)), "cufftExecD2Z")) return false;
-    unpack_c2r<<<blocks((long long) N * (M / 2 + 1)), 256, 0, st>>>(P->d_Y, X, N, M, s, f0);
+    if (!rows_to_pairs(P, X, st)) return false;
+    unpack_pairs<<<col_blocks(P->M / 2 + 1, (P->N + 1) / 2), kGridBlock, 0, st>>>(P->d_cwork, X, P->N, P->M, Phi{s, f0});
     count_launch();
-    return ok(cudaGetLastError(), "unpack_c2r");
+    return ok(cudaGetLastError(), "unpack_pairs");
+}
+
+// The sphere's whole grid stage: theta then phi (phi_last), from X's coefficients scaled by e, or phi
+// then theta, to X's coefficients scaled by e.
+bool sphere(SphereGridPlan * P, double * X, bool phi_last, Ends e, Phi h, cudaStream_t st) {
+    const int N = P->N, M = P->M, dst = (is_dst(P->kind[0]) ? 1 : 0) | (is_dst(P->kind[1]) ? 2 : 0);
+    const bool type3 = is_type3(P->kind[0]);
+    double2 * const C = P->d_Y, * const Z = P->d_cwork;
+    if (!phi_last && !rows_to_pairs(P, X, st)) return false;
+    const dim3 rows = col_blocks(M / 2 + 1, (N + 1) / 2), freqs = col_blocks(M / 2 + 1, N / 2 + 1);
+    if (type3) (phi_last ? t3_pre_c<false> : t3_pre_c<true>)<<<freqs, kGridBlock, 0, st>>>(X, Z, C, P->d_tw, N, M, dst, e, h);
+    else       (phi_last ? t2_pre_c<false> : t2_pre_c<true>)<<<rows, kGridBlock, 0, st>>>(X, Z, C, N, M, dst, e, h);
+    count_launch();
+    if (!ok(cudaGetLastError(), "theta") || !fok(cufftSetStream(P->t_z2z, st), "cufftSetStream") ||
+        !fok(cufftExecZ2Z(P->t_z2z, reinterpret_cast<cufftDoubleComplex *>(C), reinterpret_cast<cufftDoubleComplex *>(C),
+                          type3 ? CUFFT_INVERSE : CUFFT_FORWARD), "cufftExecZ2Z")) return false;
+    if (type3)         (phi_last ? t3_post_c<true> : t3_post_c<false>)<<<rows, kGridBlock, 0, st>>>(C, X, Z, N, M, dst, e, h);
+    else if (phi_last) t2_post_c<true><<<rows, kGridBlock, 0, st>>>(C, X, Z, P->d_tw, N, M, dst, e, h);
+    else               t2_post_c<false><<<freqs, kGridBlock, 0, st>>>(C, X, Z, P->d_tw, N, M, dst, e, h);
+    count_launch();
+    return ok(cudaGetLastError(), "theta") && (!phi_last || pairs_to_rows(P, X, st));
 }
 
 bool ends(SphereGridPlan * P, double * X, bool last, int c0, int start, double f, cudaStream_t st) {
@@ -694,15 +932,16 @@ bool run(SphereGridPlan * P, int op, char T, double * X, cudaStream_t st) {
         if (T == 'N') return theta_tri(P, X, st) && tri_scaling(P, X, 0.5, 1.0, nm, st);
         return tri_scaling(P, X, 1.0, 1.0, nm, st) && theta_tri(P, X, st);
     }
+    // j of column 2j - 1 or 2j is even in the columns {0, 3, 4, 7, 8, ..} and odd in {1, 2, 5, 6, ..}
     const bool sph = op == SPH_SYN || op == SPH_ANA;
-    auto first = [&](double f) { return sph ? ends(P, X, false, 0, 3, f, st) : ends(P, X, false, -1, 1, f, st); };
-    auto last = [&](double f) { return sph ? ends(P, X, true, -1, 1, f, st) : ends(P, X, true, 0, 3, f, st); };
+    const Ends first{0, sph ? 0 : 1, 1.0}, last{N - 1, sph ? 1 : 0, 1.0};
+    auto times = [](Ends e, double f) { e.f = f; return e; };
     if (op == SPH_SYN || op == SPHV_SYN) {
-        if (T == 'N') return first(2.0) && theta(P, X, st) && phi_c2r(P, X, C_1_4_SQRT_PI, C_SQRT2, st);
-        return phi_r2c(P, X, C_1_2_SQRT_PI, C_SQRT1_2, st) && theta(P, X, st) && last(0.5);
+        if (T == 'N') return sphere(P, X, true, times(first, 2.0), Phi{C_1_4_SQRT_PI, C_SQRT2}, st);
+        return sphere(P, X, false, times(last, 0.5), Phi{C_1_2_SQRT_PI, C_SQRT1_2}, st);
     }
-    if (T == 'N') return phi_r2c(P, X, C_4_SQRT_PI / nm2, C_SQRT1_2, st) && theta(P, X, st) && first(0.5);
-    return last(2.0) && theta(P, X, st) && phi_c2r(P, X, C_2_SQRT_PI / nm2, C_SQRT2, st);
+    if (T == 'N') return sphere(P, X, false, times(first, 0.5), Phi{C_4_SQRT_PI / nm2, C_SQRT1_2}, st);
+    return sphere(P, X, true, times(last, 2.0), Phi{C_2_SQRT_PI / nm2, C_SQRT2}, st);
 }
 
 SphereGridPlan * as_grid(const ft_sphere_fftw_plan * P) {
@@ -769,11 +1008,10 @@ void ft_destroy_sphere_fftw_plan(ft_sphere_fftw_plan * Pp) {
     if (!P) return;
     if (P->have_t_r2c) cufftDestroy(P->t_r2c);
     if (P->have_t_c2r) cufftDestroy(P->t_c2r);
-    if (P->have_p_r2c) cufftDestroy(P->p_r2c);
-    if (P->have_p_c2r) cufftDestroy(P->p_c2r);
+    if (P->have_t_z2z) cufftDestroy(P->t_z2z);
     if (P->have_t4) cufftDestroy(P->t4);
     if (P->have_p_z2z) cufftDestroy(P->p_z2z);
-    cudaFree(P->d_work); cudaFree(P->d_cwork); cudaFree(P->d_Y); cudaFree(P->d_stage); cudaFree(P->d_u); cudaFree(P->d_work2);
+    cudaFree(P->d_work); cudaFree(P->d_cwork); cudaFree(P->d_Y); cudaFree(P->d_tw); cudaFree(P->d_stage); cudaFree(P->d_u); cudaFree(P->d_work2);
     cudaFree(P->d_w);
     if (P->stream) cudaStreamDestroy(P->stream);
     P->magic = 0;
