@@ -33,7 +33,7 @@
 // of code (16 steps of 8 sweeps on 2 columns), which the stages run at different places at the
 // same time: with unrolled loading and storing loops beside them (register staging, about 50 KB in
 // all) the instruction cache missed and the launch took 10.8 ms at sph degree 4095; with the
-// compact loops 8.5 ms (9.8 ms for the former kernel, whose stages met at a barrier per chunk).
+// compact loops 7.97 ms (9.8 ms for the former kernel, whose stages met at a barrier per chunk).
 //
 // rot_resident_kernel: columns resident in shared memory
 // ------------------------------------------------------
@@ -1281,7 +1281,8 @@ int tune(int kind, bool hi2lo, const RotLaunch & L, double * const * dead, int m
     // columns would leave L2 between passes)
     for (int cfg = 0; cfg < 8 * kPipeModes; ++cfg) {
         if ((cfg & 7) > 5) continue;
-        if ((cfg >> 3) && !sched) continue;
+        // head sweeps are one pass in every shape: the pipeline's queue is the task list again
+        if ((cfg >> 3) && (!sched || L.fields[0].blk > 0)) continue;
         if (launch_shape(kind, hi2lo, cfg, S, max_ctas, st, sched, prog_call, prog_cap) != cudaSuccess) { best = -1; break; }
         if (cudaEventRecord(e0, st) != cudaSuccess) { best = -1; break; }
         if (launch_shape(kind, hi2lo, cfg, S, max_ctas, st, sched, prog_call, prog_cap) != cudaSuccess) { best = -1; break; }

@@ -15,11 +15,12 @@
 // Summation: the accumulators sum one chunk of 256 consecutive k (k / 256 equal) at a time; at the
 // end of each chunk a thread adds them into its outputs in C (which it alone writes) and starts the
 // next chunk from zero.  The additions are reductions at L2: reading the sums back held the warps for
-// a round trip every 16 slabs (sph degree 4095 4752 -> 4511 us, 2047 630 -> 594).  A single accumulation over all n terms lets the rounding error grow with
-// n; chunked sums, like a BLAS's K panels, keep it near that of 256 terms plus n / 256 additions (the
-// reference's round trips, which amplify this error in the ill-conditioned triangle transforms,
-// then match its BLAS build).  The chunks do not depend on the tile, so every shape gives the same
-// bits.  C must not alias the inputs (every caller multiplies out of place).
+// a round trip every 16 slabs (sph degree 4095 4752 -> 4511 us, 2047 630 -> 594).  A single
+// accumulation over all n terms lets the rounding error grow with n; chunked sums, like a BLAS's K
+// panels, keep it near that of 256 terms plus n / 256 additions (the reference's round trips, which
+// amplify this error in the ill-conditioned triangle transforms, then match its BLAS build).  The
+// chunks do not depend on the tile, so every shape gives the same bits.  C must not alias the inputs
+// (every caller multiplies out of place).
 
 #include <algorithm>
 #include <atomic>
