@@ -31,7 +31,7 @@ __all__ = [
     "plan_rotsphere", "plan_rottriangle", "plan_rotdisk",
     "execute_sph_hi2lo", "execute_sph_lo2hi", "execute_tri_hi2lo", "execute_tri_lo2hi",
     "execute_disk_hi2lo", "execute_disk_lo2hi",
-    "execute_dev", "execute_shared_dev", "execute_shared_host", "FP64", "FP64_BLOCKED", "MIXED_BF16", "MIXED_BF16X4", "device_status", "execute_noalloc_dev", "NOALLOC_MAX_ELEMS", "execute_batched_dev", "rotations_dev", "kernel_launches", "profile", "profile_read", "set_rotation_config",
+    "execute_dev", "execute_shared_dev", "execute_shared_host", "FP64", "FP64_BLOCKED", "MIXED_BF16", "MIXED_BF16X4", "device_status", "rotation_status", "execute_noalloc_dev", "NOALLOC_MAX_ELEMS", "execute_batched_dev", "rotations_dev", "kernel_launches", "profile", "profile_read", "set_rotation_config",
     "layout_cols", "rand_layout", "sphrand", "trirand", "diskrand",
     "SphereGridPlan", "plan_sph_synthesis", "plan_sph_analysis", "plan_sphv_synthesis", "plan_sphv_analysis",
     "execute_sph_synthesis", "execute_sph_analysis", "execute_sphv_synthesis", "execute_sphv_analysis",
@@ -92,6 +92,7 @@ def _load() -> C.CDLL:
         "ft_b200_execute_shared_dev": (i, [vp, i, ch, C.POINTER(vp), i, i, vp]),
         "ft_b200_execute_shared_host": (i, [vp, i, C.POINTER(i), C.c_char_p, C.POINTER(vp), i, i]),
         "ft_b200_device_status": (i, [vp]),
+        "ft_b200_rotation_status": (i, [i]),
         "ft_b200_profile": (i, [i]), "ft_b200_profile_read": (i, [i, C.POINTER(C.c_double), C.POINTER(i)]),
         "ft_b200_set_rotation_config": (None, [i]),
         "ft_plan_sph_synthesis": (vp, [i, i, C.c_uint]), "ft_plan_sph_analysis": (vp, [i, i, C.c_uint]),
@@ -842,6 +843,15 @@ def execute_shared_host(P: HarmonicPlan, ops: Sequence[tuple], arrays: Sequence,
 def device_status(P: HarmonicPlan) -> int:
     """Read and clear the plan's device status word (nonzero: a tensor-core wait gave up)."""
     v = lib.ft_b200_device_status(P.ptr)
+    if v < 0:
+        _check()
+    return v
+
+
+def rotation_status(value: int = 0) -> int:
+    """The rotation kernels' status word on the current device, replaced by ``value`` (nonzero: a
+    bounded wait of a rotation launch ran out and that launch's output is not valid)."""
+    v = lib.ft_b200_rotation_status(value)
     if v < 0:
         _check()
     return v

@@ -131,7 +131,7 @@ ft_rotation_plan * make_rotation_plan(int kind, int n, double alpha, double beta
     for (long long i = 0; i < len; i++) sc[i] = make_double2(RP->s[i], RP->c[i]);
     if (!cuda_ok(cudaMalloc(&RP->d_sc, sizeof(double2) * len), "cudaMalloc(table)") ||
         !cuda_ok(cudaMemcpy(RP->d_sc, sc.data(), sizeof(double2) * len, cudaMemcpyHostToDevice), "cudaMemcpy(table)") ||
-        !cuda_ok(cudaMalloc(&RP->d_counter, sizeof(int)), "cudaMalloc(counter)") || !rotation_plan_skew(RP)) {
+        !cuda_ok(cudaMalloc(&RP->d_counter, sizeof(int) * kCounterWords), "cudaMalloc(counter)") || !rotation_plan_skew(RP)) {
         ft_destroy_rotation_plan(RP);
         return nullptr;
     }
@@ -693,7 +693,7 @@ BatchCtx * get_batch(HarmonicPlan * const * H, const int * N, const int * M, int
     bool ok = upload(B, tasks, &B->d_tasks) && build_trmm_set(B, left, &B->left, false) &&
               (kind != TRI || build_trmm_set(B, right, &B->right, true)) &&
               cuda_ok(cudaMalloc(&B->d_work, sizeof(double) * std::max<size_t>(1, work)), "cudaMalloc(batch workspace)") &&
-              cuda_ok(cudaMalloc(&B->d_counter, sizeof(int)), "cudaMalloc(batch counter)");
+              cuda_ok(cudaMalloc(&B->d_counter, sizeof(int) * kCounterWords), "cudaMalloc(batch counter)");
     if (B->d_work) B->allocs.push_back(B->d_work);
     if (B->d_counter) B->allocs.push_back(B->d_counter);
     if (!ok) {
@@ -1249,8 +1249,16 @@ int ft_b200_device_status(const ft_harmonic_plan * P) {
     if (!H) { set_error(FT_B200_EINVAL, "not a plan created by this library"); return -1; }
     const int a = H->blocked ? blocked_device_error(H->blocked) : 0;
     const int b = H->mixed_trmm ? mixed_trmm_device_error(H->mixed_trmm) : 0;
-    const int c = rotation_device_error();   // the rotation kernel's pass-pipeline waits (library-wide)
+    const int c = rotation_status(0);   // the waits of the rotation kernels (every plan of the device)
     return a ? a : (b ? b : c);
+}
+
+int ft_b200_rotation_status(int value) {
+    clear_error();
+    if (value < 0) { set_error(FT_B200_EINVAL, "value must not be negative"); return -1; }
+    const int v = rotation_status(value);
+    if (v < 0) set_error(FT_B200_ECUDA, "reading or writing the rotation status word failed");
+    return v;
 }
 
 int ft_b200_plan_kind(const ft_harmonic_plan * P) {

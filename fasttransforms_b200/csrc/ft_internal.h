@@ -164,13 +164,14 @@ struct RotField {
 // Kernel launchers (rotations.cu).  The field table travels by value in the
 // kernel parameters (kept under the classic 4 KB parameter limit).
 constexpr int kMaxFields = 64;
+constexpr int kCounterWords = 2;
 struct RotLaunch {
     RotField fields[kMaxFields];
     int nfields;
     const RotTask * tasks;     // device, longest first
     int ntasks;
-    int * counter;             // device work counter (reset by the launcher)
-    int counter0;              // its value after the reset
+    int * counter;             // device work counter and the launch's give-up word (kCounterWords, reset by the launcher)
+    int counter0;              // their value after the reset
     // columns lead0 .. lead - 1 of every field have no sweeps (orders 0 and 1, and what lies before
     // them): an out-of-place launch copies them from in to out
     int lead0, lead;
@@ -192,7 +193,7 @@ void rot_schedule_free(RotSchedule * s);
 // The progress words of a launch follow its work counter at this distance (in words), so that one
 // fill resets both.
 constexpr int kProgLead = 64;
-int rotation_device_error();   // reads and clears the rotation kernel's status word (-1: read failed)
+int rotation_status(int value);   // returns the rotation kernels' report word (current device) and stores value in it; -1: failed
 // dead: per field, memory the caller has no live data in (N x M at the field's leading
 // dimension), or null.  With it, the first launch of a shape times every configuration
 // there and keeps the fastest for the shape (the autotuner; FT_B200_AUTOTUNE=0 turns it off).

@@ -39,8 +39,8 @@
 // ------------------------------------------------------
 // For chains that fit; see there.
 //
-// Every wait is bounded, after which the launch records a device status and every later wait gives
-// up at once.  Every global access is bounds-checked against the field's N, M.
+// Every wait is bounded, after which the launch leaves a status to report and its other waits end at
+// once; later launches start afresh.  Every global access is bounds-checked against the field's N, M.
 
 #include <atomic>
 #include <cstdio>
@@ -109,8 +109,9 @@ __device__ __forceinline__ void rot_lo2hi(double & x, double & y, double s, doub
     x = xn; y = yn;
 }
 
-// Status word of the rotation kernel: nonzero once a bounded wait ran out (the output is then not
-// valid).  Read and cleared by rotation_device_error().
+// Report word of the rotation kernels: nonzero once a bounded wait ran out (that launch's output is
+// not valid).  Read and replaced by rotation_status(); no wait looks at it, so a launch that gave up
+// leaves no trace in the launches after it.
 __device__ int g_rot_status;
 
 // Progress of a pass over its columns: hi2lo, -X where every position >= X is final for the pass;
@@ -123,24 +124,29 @@ __device__ int g_rot_status;
 __device__ __forceinline__ void publish_progress(int * p, int v) {
     asm volatile("red.release.gpu.global.max.s32 [%0], %1;\n" :: "l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ bool gave_up(long long t0) {
-    if (*(volatile int *) &g_rot_status != 0) return true;
+// The word in which a launch (resident kernel: a CTA) keeps that one of its waits ran out: its other
+// waits then return at once, so one failed wait costs the launch about that long, not that long per
+// unit.  Streaming launches hold it behind their work counter, reset by the same fill.
+struct GiveUp { int * word; int clean; };
+__device__ __forceinline__ bool given_up(GiveUp g) { return *(volatile int *) g.word != g.clean; }
+// true once the wait that began at t0 is to end: about 2^32 SM cycles later, or when another one ran out
+__device__ __forceinline__ bool gave_up(long long t0, GiveUp g, int code) {
+    if (given_up(g)) return true;
     if (clock64() - t0 <= (1LL << 32)) return false;
-    atomicExch(&g_rot_status, 3);
+    atomicExch(g.word, g.clean + 1);
+    atomicCAS(&g_rot_status, 0, code);
     return true;
 }
-// Waits until *p >= need and returns the value read; gives up after about 2^32 SM cycles,
-// setting the status word, and at once when the word is already set (so one failed wait costs
-// a launch about that long, not that long per unit).
-// (The status word is a read of global memory, as slow as the progress word's own: only every 64th
+// Waits until *p >= need and returns the value read (a smaller one if the wait ended before).
+// (The launch's word is a read of global memory, as slow as the progress word's own: only every 64th
 // poll looks at it.)
-__device__ __noinline__ int wait_progress(const int * p, int need) {
+__device__ __noinline__ int wait_progress(const int * p, int need, GiveUp g) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
         if (v >= need) return v;
-        if (i % 64 == 0 && gave_up(t0)) return v;
+        if (i % 64 == 0 && gave_up(t0, g, 3)) return v;
     }
 }
 // Whole-task launches run a task's passes one after another in one CTA, whose loading warps wait
@@ -152,33 +158,35 @@ __device__ __forceinline__ unsigned long long local_word(unsigned seq, int v) {
 __device__ __forceinline__ void publish_local(unsigned long long * p, unsigned long long w) {
     asm volatile("st.release.cta.shared::cta.u64 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "l"(w) : "memory");
 }
-__device__ __noinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need) {
+__device__ __noinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need, GiveUp g) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         unsigned long long v;
         asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];\n" : "=l"(v) : "r"(tc::smem_addr(p)) : "memory");
         if (v >= need) return v;
-        if (i % 64 == 0 && gave_up(t0)) return v;
+        if (i % 64 == 0 && gave_up(t0, g, 3)) return v;
         __nanosleep(32);
     }
 }
-// Bounded mbarrier wait: a wait that runs out sets the status word, after which every wait of
-// the launch returns false at once, the loops over queue entries end, and the kernel with them.
+// Bounded mbarrier wait: false once a wait of the launch ran out; the loops over queue entries then
+// end, and the kernel with them.
 // (The slow path is a call: the kernel's warps run different code at the same time, and what they
 // run between them has to stay small to be served from the instruction cache.)
-__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, uint32_t parity) {
-    if (tc::mbar_wait(bar, parity, (volatile int *) &g_rot_status)) return true;
-    atomicCAS(&g_rot_status, 0, 5);
-    return false;
+__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, uint32_t parity, GiveUp g) {
+    if (given_up(g)) return false;
+    const long long t0 = clock64();
+    while (!tc::mbar_try_wait(bar, parity))
+        if (gave_up(t0, g, 5)) return false;
+    return true;
 }
-__device__ __forceinline__ bool wait_bar(uint64_t * bar, uint32_t parity) {
+__device__ __forceinline__ bool wait_bar(uint64_t * bar, uint32_t parity, GiveUp g) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok) : "r"(tc::smem_addr(bar)), "r"(parity) : "memory");
-    return ok || wait_bar_slow(bar, parity);
+    return ok || wait_bar_slow(bar, parity, g);
 }
 
 // Asynchronous 8-byte copy global -> shared (0 bytes read, zeros written when !valid), and the
@@ -365,19 +373,19 @@ __device__ __forceinline__ void stage_steps(double (&win)[NCOL][2 * B], const do
 __device__ __forceinline__ void publish_word(int * p, int v) {
     asm volatile("st.release.cta.shared::cta.s32 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "r"(v) : "memory");
 }
-__device__ __noinline__ int wait_word_slow(const int * p, int need) {
+__device__ __noinline__ int wait_word_slow(const int * p, int need, GiveUp g) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
         if (v >= need) return v;
-        if (i % 256 == 0 && gave_up(t0)) return v;
+        if (i % 256 == 0 && gave_up(t0, g, 3)) return v;
     }
 }
-__device__ __forceinline__ int wait_word(const int * p, int need) {
+__device__ __forceinline__ int wait_word(const int * p, int need, GiveUp g) {
     int v;
     asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
-    return v >= need ? v : wait_word_slow(p, need);
+    return v >= need ? v : wait_word_slow(p, need, g);
 }
 
 // E steps of one sequence of the resident kernel (stage_steps with the columns in place; a branch an
@@ -454,6 +462,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     __shared__ unsigned long long s_local;
     __shared__ int s_unit[UR];
 
+    const GiveUp giveup{L.counter + 1, L.counter0};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < SH::IDLEN; i += blockDim.x) ident[i] = make_double2(0.0, 1.0);
     if (threadIdx.x == 0) {
@@ -485,7 +494,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         ++nunit;
         int id = 0;
         if (warp == W) {
-            if (!__all_sync(0xffffffffu, wait_bar(&uempt[slot], ph ^ 1))) return -1;
+            if (!__all_sync(0xffffffffu, wait_bar(&uempt[slot], ph ^ 1, giveup))) return -1;
             if (lane == 0) {
                 id = atomicAdd(L.counter, 1) - L.counter0;
                 if (id >= nwork) id = -1;
@@ -494,7 +503,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             }
             id = __shfl_sync(0xffffffffu, id, 0);
         } else {
-            if (!__all_sync(0xffffffffu, wait_bar(&ufull[slot], ph))) return -1;
+            if (!__all_sync(0xffffffffu, wait_bar(&ufull[slot], ph, giveup))) return -1;
             id = *(volatile int *) &s_unit[slot];
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&uempt[slot]);
@@ -533,8 +542,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 if (q >= P.stages) {
                     // no sweep of the pass: hand the chunks on
                     for (int k = 0; k < P.nchunk; ++k) {
-                        wait_bar(&in_full[nin % SL], (nin / SL) & 1);
-                        wait_bar(&out_empty[nout % SL], ((nout / SL) & 1) ^ 1);
+                        wait_bar(&in_full[nin % SL], (nin / SL) & 1, giveup);
+                        wait_bar(&out_empty[nout % SL], ((nout / SL) & 1) ^ 1, giveup);
                         const double * const bin = in_ring + (nin % SL) * SLOT + lane_off;
                         double * const bout = out_ring + (nout % SL) * SLOT + lane_off;
 #pragma unroll
@@ -588,14 +597,14 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     live |= stage_sc(k + SCS - 1) ? 1u << (SCS - 1) : 0u;
                     const bool has_in = k < P.nchunk, has_out = k >= D;
                     const int is = nin % SL, os = nout % SL;
-                    if (has_in) wait_bar(&in_full[is], (nin / SL) & 1);
-                    if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1);
+                    if (has_in) wait_bar(&in_full[is], (nin / SL) & 1, giveup);
+                    if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1, giveup);
                     const double * const bin = in_ring + is * SLOT + lane_off;    // read while elements enter (has_in)
                     double * const bout = out_ring + os * SLOT + lane_off;        // written once elements leave (has_out)
                     const bool odd = D > 1 && (k & 1);   // the chunk starts halfway round the window
                     if (live & 1u) {
                         const int slot = sc_used % SCS;
-                        wait_bar(&scbar[q * SCS + slot], (sc_used / SCS) & 1);
+                        wait_bar(&scbar[q * SCS + slot], (sc_used / SCS) & 1, giveup);
                         ++sc_used;
                         const double2 * sc[B];
 #pragma unroll
@@ -635,7 +644,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const RotField & F = L.fields[task.field];
             const TaskGeo<KIND, NC, W, B> G(F, task);
             if (w == 0 && lane == 0 && G.nsw > 0 && (chain.first >= G.npass || chain.stride < 1))
-                atomicExch(&g_rot_status, 4);   // a schedule that does not match this launch shape
+                atomicCAS(&g_rot_status, 0, 4);   // a schedule that does not match this launch shape
             const MV mv(F, task, G.mlast, lane);
             for (int r = chain.first; r < G.npass; r += chain.stride) {
                 const Pass<KIND, HI2LO, W, B, E> P(G.N, G.nsw, G.npass, G.jpar, G.jlo, r, r == 0 && F.in != F.out);
@@ -651,10 +660,10 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const int pmin = P.pmin(i), pmax = pmin + E - 1;
                     const int need = HI2LO ? -max(pmin, 0) : min(pmax, P.emax);
                     if (prev) {
-                        if (seen < need) { if (lane == 0) seen = wait_progress(prev, need); seen = __shfl_sync(0xffffffffu, seen, 0); }
+                        if (seen < need) { if (lane == 0) seen = wait_progress(prev, need, giveup); seen = __shfl_sync(0xffffffffu, seen, 0); }
                     } else {
                         const unsigned long long want = local_word(seq - 1, need);
-                        if (seen_local < want) { if (lane == 0) seen_local = wait_local(&s_local, want); seen_local = __shfl_sync(0xffffffffu, seen_local, 0); }
+                        if (seen_local < want) { if (lane == 0) seen_local = wait_local(&s_local, want, giveup); seen_local = __shfl_sync(0xffffffffu, seen_local, 0); }
                     }
                     __syncwarp();
                 };
@@ -662,7 +671,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 auto fetch = [&](int i) {
                     const unsigned n = n0 + i;
                     const int pmin = P.pmin(i);
-                    wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1);
+                    wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1, giveup);
                     const uint32_t slot = tc::smem_addr(rings + (size_t) (n % SL) * SLOT);
 #pragma unroll 1
                     for (int ph = 0; ph < MV::PH; ++ph) {
@@ -708,7 +717,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 int since = 0;
                 for (int i = 0; i < P.nchunk; ++i, ++n) {
                     const int pmin = P.pmin(i);
-                    wait_bar(&bfull[n % SL], (n / SL) & 1);
+                    wait_bar(&bfull[n % SL], (n / SL) & 1, giveup);
                     const double * const slot = ring + (n % SL) * SLOT;
 #pragma unroll 1
                     for (int ph = 0; ph < MV::PH; ++ph) {
@@ -759,7 +768,7 @@ cudaError_t launch_cfg(const RotLaunch & L, int max_ctas, int per_sm_most, cudaS
     const int work = L.chains ? L.nchains : L.ntasks * SH::SPLIT;   // queue entries: pipeline entries or groups
     if (ctas > work) ctas = work;
     if (ctas <= 0) return cudaSuccess;
-    if (!L.chains) e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);   // with chains: launch_shape
+    if (!L.chains) e = cudaMemsetAsync(L.counter, 0, sizeof(int) * kCounterWords, st);   // with chains: launch_shape
     if (e != cudaSuccess) return e;
     kern<<<ctas, SH::WARPS * 32, SH::bytes, st>>>(L);
     count_launch();
@@ -807,7 +816,8 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
     double2 * const ident = pairs + W * SCS * SCLEN;
     double * const col = reinterpret_cast<double *>(ident + R::IDLEN) + ROW;   // position p of lane l at col[p * ROW + l]
     __shared__ __align__(8) uint64_t scbar[W * SCS];
-    __shared__ int prog[W];
+    __shared__ int prog[W], s_giveup;
+    const GiveUp giveup{&s_giveup, 0};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     allow_next();
@@ -825,6 +835,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
 
     if (threadIdx.x < W) prog[threadIdx.x] = -1;
     if (threadIdx.x == 0) {
+        s_giveup = 0;
         for (int i = 0; i < W * SCS; ++i) tc::mbar_init(&scbar[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -931,7 +942,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
             const int cin = HI2LO ? chi - k : k, cout = HI2LO ? cin + D : cin - D;
             if (has_in && g > 0) {
                 const int need = (g - 1) * 4096 + (HI2LO ? 2048 - cin : cin + 1);
-                if (seen < need) seen = wait_word(before, need);
+                if (seen < need) seen = wait_word(before, need, giveup);
             }
             // position of the chunk's first step, and the way the steps go
             const double * const bin = col + (HI2LO ? cin * E + E - 1 : cin * E - 1) * ROW + lane;
@@ -939,7 +950,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
             const bool odd = D > 1 && (k & 1);
             if (live & 1u) {
                 const int slot = sc_used % SCS;
-                wait_bar(&bars[slot], (sc_used / SCS) & 1);
+                wait_bar(&bars[slot], (sc_used / SCS) & 1, giveup);
                 ++sc_used;
                 const double2 * sc[B];
 #pragma unroll
@@ -1074,13 +1085,10 @@ bool rotation_plan_skew(ft_rotation_plan * RP) {
     return true;
 }
 
-int rotation_device_error() {
+int rotation_status(int value) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_rot_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v) {
-        const int z = 0;
-        if (cudaMemcpyToSymbol(g_rot_status, &z, sizeof(int)) != cudaSuccess) return -1;
-    }
+    if (v != value && cudaMemcpyToSymbol(g_rot_status, &value, sizeof(int)) != cudaSuccess) return -1;
     return v;
 }
 

@@ -258,7 +258,7 @@ SpinRotPlan * make_srp(int n, int s) {
             }
     if (!ok(cudaMalloc(&P->d_sc2, sizeof(double2) * sc.size()), "cudaMalloc(spin table)") ||
         !ok(cudaMemcpy(P->d_sc2, sc.data(), sizeof(double2) * sc.size(), cudaMemcpyHostToDevice), "cudaMemcpy(spin table)") ||
-        !ok(cudaMalloc(&P->d_counter, sizeof(int)), "cudaMalloc(counter)") ||
+        !ok(cudaMalloc(&P->d_counter, sizeof(int) * kCounterWords), "cudaMalloc(counter)") ||
         !ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "cudaStreamCreate")) {
         destroy_srp(P);
         return nullptr;

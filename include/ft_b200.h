@@ -505,9 +505,18 @@ int ft_b200_execute_shared_host(const ft_harmonic_plan * P, int nops, const int 
 
 /* Reads and clears the plan's device status word: 0 normally; nonzero when a
  * wait inside one of its tensor-core kernels gave up (the kernel then stops
- * early and its output is not valid).  Synchronises with the device.  No
+ * early and its output is not valid), or one of the rotation kernels' (as
+ * ft_b200_rotation_status(0)).  Synchronises with the device.  No
  * counterpart in the reference, whose kernels have no device waits. */
 int ft_b200_device_status(const ft_harmonic_plan * P);
+
+/* Status word of the rotation kernels on the current device, whatever the plan
+ * (rotation and spin plans have no other way to it): returns it, and stores value
+ * (>= 0; 0 clears it) in its place; -1 on failure.  Nonzero: a bounded wait of a
+ * rotation launch ran out since the word was last cleared, and that launch's output
+ * is not valid.  It is a report only: later launches run as usual whatever it holds.
+ * Synchronises with the device. */
+int ft_b200_rotation_status(int value);
 
 /* Kind of a plan (FT_B200_SPH / TRI / DISK), or -1. */
 int ft_b200_plan_kind(const ft_harmonic_plan * P);
