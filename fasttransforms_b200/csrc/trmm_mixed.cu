@@ -541,6 +541,7 @@ __global__ void __launch_bounds__(256) slice_input_s8_kernel(const __grid_consta
         for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         int ex = 0;
         if (amax > 0) (void) frexp(amax, &ex);
+        ex = max(ex, -1016);                                      // s stays finite: a smaller column has fewer digits
         const double inv = amax > 0 ? ldexp(1.0, ex - 6) : 1.0;   // 1 / s, |s x| < 64
         const double s = 1.0 / inv;
         if (lane == 0) L.inv[tile_base * TBN + ci] = inv;
