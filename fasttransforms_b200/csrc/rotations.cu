@@ -1013,8 +1013,14 @@ cudaError_t launch_resident(const RotLaunch & L, cudaStream_t st) {
 
 // Launch shapes: 0 .. 4 rot_kernel with W stage warps x B sweeps per warp, chunk E; 5
 // rot_resident_kernel.
-//   0: 8 x 8 x 16    1: 8 x 8 x 8    2: 4 x 8 x 8, one CTA per SM    4: 4 x 8 x 8, as many as fit
-//   3: 8 x 8 x 8 with one sequence a lane (half the orders a group, twice the groups)
+//   0: 8 x 8 x 16    1: 8 x 8 x 8    2: 4 x 8 x 8, one CTA per SM
+// with one sequence a lane (half the orders a group, twice the groups):
+//   3: 8 x 8 x 8, one CTA per SM    4: 4 x 8 x 16, two CTAs per SM
+// Shape 4 is the heads' (one pass of at most 31 sweeps): two CTAs with chunks of 16 fit because a ring
+// holds half the columns, and a stage's 16 steps have no second copy for the other half of its window.
+// us a launch, against 4 x 8 x 8 with both sequences a lane, two CTAs per SM: sph 4095 x 16 fields 4667 /
+// 4804, 2047 x 8 657 / 729, 1023 x 8 201 / 231, disk 1500 x 6 589 / 735, tri 767 x 12 180 / 200; whole
+// sweeps through the pipeline sph 1024 269 / 395, disk 700 355 / 543.
 template <int KIND, bool HI2LO>
 cudaError_t launch_kind(int cfg, const RotLaunch & L, int max_ctas, cudaStream_t st) {
     constexpr int NC = order_sequences(KIND);
@@ -1022,7 +1028,7 @@ cudaError_t launch_kind(int cfg, const RotLaunch & L, int max_ctas, cudaStream_t
     if (cfg == 1) return launch_cfg<KIND, NC, HI2LO, 8, 8, 8, 1>(L, max_ctas, 0, st);
     if (cfg == 2) return launch_cfg<KIND, NC, HI2LO, 4, 8, 8, 2>(L, max_ctas, 1, st);
     if (cfg == 3) return launch_cfg<KIND, 1, HI2LO, 8, 8, 8, 1>(L, max_ctas, 1, st);
-    if (cfg == 4) return launch_cfg<KIND, NC, HI2LO, 4, 8, 8, 2>(L, max_ctas, 0, st);
+    if (cfg == 4) return launch_cfg<KIND, 1, HI2LO, 4, 8, 16, 2>(L, max_ctas, 0, st);
     return launch_cfg<KIND, NC, HI2LO, 8, 8, 16, 1>(L, max_ctas, 0, st);
 }
 
@@ -1100,7 +1106,7 @@ int shape_pass(int cfg) {
     return (cfg >= 0 && cfg < 6) ? wb[cfg] : 64;
 }
 // Groups that a shape makes of a task of the list (Shape::SPLIT).
-int shape_split(int cfg, int kind) { return cfg == 3 ? order_sequences(kind) : 1; }
+int shape_split(int cfg, int kind) { return cfg == 3 || cfg == 4 ? order_sequences(kind) : 1; }
 
 // The queue of the pass pipeline for L's tasks with passes of wb sweeps, built on first use;
 // null when the stream is capturing then (the upload synchronises) or on an allocation
@@ -1234,7 +1240,7 @@ cudaError_t launch_shape(int kind, bool hi2lo, int cfg, const RotLaunch & L, int
 // lane halves a step, at half the rotations per (sin, cos) load, until about 400 passes of 64
 // sweeps give every SM enough of them for throughput to count.
 int default_config(int kind, const RotLaunch & L, RotSchedule * sched, cudaStream_t st) {
-    if (L.nfields > 0 && L.fields[0].blk > 0) return 4;   // at most 31 sweeps a column: one pass of 4 x 8
+    if (L.nfields > 0 && L.fields[0].blk > 0) return 4;   // at most 31 sweeps a column: one pass
     const bool pair = order_sequences(kind) == 2;
     int len = 0;
     for (int f = 0; f < L.nfields; ++f) len = std::max(len, Geo::chain_len(kind, L.fields[f].N, 0));

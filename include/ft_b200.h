@@ -538,8 +538,8 @@ int ft_b200_profile_read(int family, double * ms, int * launches);
  * whose kernels have no launch shape).  cfg = s + 8 p forces shape s = 0 .. 5
  * and pass-pipeline mode p = 0 .. 2.  Shapes 0 .. 4 stream the columns through
  * warps x sweeps per warp x chunk: 8 x 8 x 16, 8 x 8 x 8, 4 x 8 x 8 on one CTA
- * per SM, 8 x 8 x 8 with one column (or part) a lane, and 4 x 8 x 8 with as many
- * CTAs per SM as fit; shape 5 keeps the columns of a task in shared memory (shape 0
+ * per SM, and with one column (or part) a lane 8 x 8 x 8 on one and 4 x 8 x 16 on
+ * two CTAs per SM; shape 5 keeps the columns of a task in shared memory (shape 0
  * where they do not fit).
  * p = 1: each pass of 32 or 64 sweeps of a task is its own work unit, queued
  * pass-major, and streams down the columns on another SM right behind the previous

@@ -16,7 +16,7 @@ import pytest
 SPH, TRI, DISK, SPIN, RECT = 0, 1, 2, 3, 4
 ROWS, LEN = 8, 8                    # Geo::kSkewRows, Geo::kSkewLen
 # W, B, E, one sequence a lane (launch shapes 0 .. 4)
-SHAPES = [(8, 8, 16, False), (8, 8, 8, False), (4, 8, 8, False), (8, 8, 8, True)]
+SHAPES = [(8, 8, 16, False), (8, 8, 8, False), (4, 8, 8, False), (8, 8, 8, True), (4, 8, 16, True)]
 
 
 def sphlike(k): return k in (SPH, SPIN, RECT)
@@ -328,7 +328,7 @@ def test_spin_columns(n, s):
 
 @pytest.mark.parametrize("k,n", [(SPH, 74), (DISK, 37), (TRI, 40)])
 def test_heads_of_the_blocked_paths(k, n):
-    check(k, n, default_M(k, n), blk=32, shapes=[(4, 8, 8, False), (8, 8, 16, False)])
+    check(k, n, default_M(k, n), blk=32, shapes=[(4, 8, 16, True), (8, 8, 16, False)])
 
 
 @pytest.mark.parametrize("k,n,M", [(SPH, 17, 9), (SPH, 9, 41), (DISK, 9, 7), (DISK, 6, 45), (TRI, 18, 18)])
