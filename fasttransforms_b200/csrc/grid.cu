@@ -485,15 +485,12 @@ __global__ void t3_post_c(const double2 * __restrict__ C, double * __restrict__ 
     }
 }
 
-// Multiplies the first (last = 0) or last (last = 1) entry of the columns
-// {c0} (c0 >= 0) and {start + 4t, start + 1 + 4t, t >= 0} by f.
-__global__ void scale_ends(double * X, int N, int M, bool last, int c0, int start, double f) {
+// Multiplies the first entry of the columns {0, 3, 4, 7, 8, ..} by f.
+__global__ void scale_first(double * X, int N, int M, double f) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = last ? N - 1 : 0;
-    if (t == 0 && c0 >= 0 && c0 < M) X[(long long) c0 * N + row] *= f;
-    const int j0 = start + 4 * t;
-    if (j0 < M) X[(long long) j0 * N + row] *= f;
-    if (j0 + 1 < M) X[(long long) (j0 + 1) * N + row] *= f;
+    const int j = t == 0 ? 0 : 4 * t - 1;
+    if (j < M) X[(long long) j * N] *= f;
+    if (t > 0 && j + 1 < M) X[(long long) (j + 1) * N] *= f;
 }
 
 // ---------------------------------------------------------------------------
@@ -828,11 +825,10 @@ bool sphere(SphereGridPlan * P, double * X, bool phi_last, Ends e, Phi h, cudaSt
     return ok(cudaGetLastError(), "theta") && (!phi_last || pairs_to_rows(P, X, st));
 }
 
-bool ends(SphereGridPlan * P, double * X, bool last, int c0, int start, double f, cudaStream_t st) {
-    const int t = (P->M - start + 3) / 4 + 1;
-    scale_ends<<<blocks(t > 0 ? t : 1), 256, 0, st>>>(X, P->N, P->M, last, c0, start, f);
+bool first_entries(SphereGridPlan * P, double * X, double f, cudaStream_t st) {
+    scale_first<<<blocks(P->M / 4 + 1), 256, 0, st>>>(X, P->N, P->M, f);
     count_launch();
-    return ok(cudaGetLastError(), "scale_ends");
+    return ok(cudaGetLastError(), "scale_first");
 }
 
 // The reference's execute sequences (src/fftw.c:131-277).  End-entry factors: first
@@ -883,7 +879,7 @@ bool run(SphereGridPlan * P, int op, char T, double * X, cudaStream_t st) {
     const double nm2 = 2.0 * N * M;
     if (op == SPIN_SYN || op == SPIN_ANA) return run_spin(P, op, T, X, st);
     if (op == DISK_SYN || op == DISK_ANA) {   // src/fftw.c:460-532: first entries of {0, 3, 4, 7, 8, ..} only
-        auto first = [&](double f) { return ends(P, X, false, 0, 3, f, st); };
+        auto first = [&](double f) { return first_entries(P, X, f, st); };
         if (op == DISK_SYN) {
             if (T == 'N') return first(2.0) && theta_disk(P, X, st) && phi_c2r(P, X, C_1_4_SQRT_PI, C_SQRT2, st);
             return phi_r2c(P, X, C_1_2_SQRT_PI, C_SQRT1_2, st) && theta_disk(P, X, st);

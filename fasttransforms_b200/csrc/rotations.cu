@@ -420,8 +420,7 @@ struct Shape {
     static constexpr int D = 2 * B / E;                  // chunks an element spends in a stage's window
     static constexpr int SL = 2;                         // slots of a ring
     static constexpr int SCS = E >= 16 ? 2 : 3;          // staged (sin, cos) chunks of a stage
-    static constexpr int NL = 1;                         // loading warps
-    static constexpr int WARPS = W + NL + 1;
+    static constexpr int WARPS = W + 2;                  // and a loading and a storing warp
     static constexpr int SLOT = E * T::ROWD;     // doubles of a ring slot
     static constexpr int SCLEN = B * E * T::CH;          // pairs of a stage's chunk
     static constexpr int IDLEN = (E / Geo::kSkewLen - 1) * Geo::kSkewRows * Geo::kSkewLen * T::CH + Geo::kSkewLen * T::CH;   // a row's span in one
@@ -431,8 +430,7 @@ struct Shape {
     static constexpr size_t bytes = (doubles * sizeof(double) + 15) / 16 * 16 + pairs * sizeof(double2);
     static_assert(D >= 1 && D * E == 2 * B, "a window must hold whole chunks");
     static_assert(E % Geo::kSkewLen == 0, "a chunk must be whole chunks of the skewed table");
-    static_assert(B == Geo::kSkewRows || (Geo::kSkewRows % B == 0 && E == Geo::kSkewLen && 2 * B % E == 0),
-                  "a stage's rows must lie one after the other in the skewed table");
+    static_assert(B == Geo::kSkewRows, "a stage's sweeps must be the rows of one block of the skewed table");
 };
 
 // Columns without sweeps, in to out (one CTA a field; nothing when in place).
@@ -452,7 +450,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     using SH = Shape<KIND, NC, W, B, E>;
     using MV = Mover<KIND, NC, HI2LO, E>;
     constexpr int SUBS = 2;   // 4 measured the same, 8 (more registers) 10 % slower
-    constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, D = SH::D, SL = SH::SL, SCS = SH::SCS, NL = SH::NL, SLOT = SH::SLOT,
+    constexpr int CH = T::CH, STEP = T::STEP, NCOL = T::NCOL, D = SH::D, SL = SH::SL, SCS = SH::SCS, SLOT = SH::SLOT,
                   SCLEN = SH::SCLEN, UR = SH::UR;
     extern __shared__ __align__(16) double smem[];
     double * const rings = smem;                                  // ring q: input of stage q; ring W: output of the last stage
@@ -486,7 +484,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     };
     unsigned nunit = 0;        // queue entries taken so far
     unsigned seq = 0;          // passes begun so far
-    // The first loading warp takes an entry from the queue and hands it to the other warps, which
+    // The loading warp takes an entry from the queue and hands it to the other warps, which
     // take it up as they finish the one before: nothing in the CTA stands still between entries.
     auto next_unit = [&]() -> int {
         const int slot = nunit % UR;
@@ -563,18 +561,16 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const int j = jpar + STEP * (HI2LO ? i0 + B - 1 - b : i0 + b);
                     if (j <= me_lane - STEP && j >= jcut) lane_mask |= 1u << b;
                 }
-                // The (sin, cos) pairs of chunk k: one bulk copy of the stage's rows (B = 4: one half
-                // of a block's) of the skewed table's chunk, whose entries are the identity where a
-                // sweep has no rotation, so every chunk runs the same straight-line code and those
+                // The (sin, cos) pairs of chunk k: one bulk copy of the skewed table's chunk of the stage's
+                // block, whose entries are the identity where a sweep has no rotation, so every chunk runs the same straight-line code and those
                 // rotations are exact no-ops.  Returns false, staging nothing, when no sweep of the
                 // stage rotates in the chunk.
                 const int K = P.nchunk + D;
-                const int beta = i0 / Geo::kSkewRows, half = (i0 % Geo::kSkewRows) / B;
+                const int beta = i0 / Geo::kSkewRows;
                 const int nk = beta < Geo::skew_blocks(KIND, N, jpar) ? Geo::skew_chunks(KIND, N, jpar, beta) : 0;
-                const double2 * const rows = F.sc + Geo::skew_at(KIND, N, jpar, beta) + half * B * Geo::kSkewLen * CH;
+                const double2 * const rows = F.sc + Geo::skew_at(KIND, N, jpar, beta);
                 auto stage_sc = [&](int k) -> bool {
-                    // a stage of rows half B .. runs 2 half B positions ahead of the block's own grid
-                    const int kappa = P.kappa(k) * (E / Geo::kSkewLen) + half * 2 * B / Geo::kSkewLen;
+                    const int kappa = P.kappa(k) * (E / Geo::kSkewLen);
                     if (k >= K || kappa >= nk) return false;
                     if (lane == 0) {
                         const int slot = sc_issued % SCS;
@@ -632,9 +628,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const long long t0 = clock64();
             while (!tc::mbar_try_wait(&scbar[q * SCS + sc_used % SCS], (sc_used / SCS) & 1) && clock64() - t0 < (1LL << 24)) {}
         }
-    } else if (warp < W + NL) {
-        // ---------------- loading warps: chunk i of a pass by warp i mod NL ----------------
-        const int w = warp - W;
+    } else if (warp == W) {
+        // ---------------- loading warp ----------------
         unsigned n0 = 0;           // chunks of earlier passes
         for (;;) {
             const int id = next_unit();
@@ -643,7 +638,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const RotTask task = group(chain.task);
             const RotField & F = L.fields[task.field];
             const TaskGeo<KIND, NC, W, B> G(F, task);
-            if (w == 0 && lane == 0 && G.nsw > 0 && (chain.first >= G.npass || chain.stride < 1))
+            if (lane == 0 && G.nsw > 0 && (chain.first >= G.npass || chain.stride < 1))
                 atomicCAS(&g_rot_status, 0, 4);   // a schedule that does not match this launch shape
             const MV mv(F, task, G.mlast, lane);
             for (int r = chain.first; r < G.npass; r += chain.stride) {
@@ -689,8 +684,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 wait_chunk(0);
                 // hi2lo: the positions above this pass's range are final once the predecessor has
                 // finished the first chunk's (they belong to earlier passes only)
-                if (HI2LO && pipe && w == 0 && lane == 0 && r + 1 < G.npass) publish_progress(L.prog + chain.prog0 + r, -(P.emax + 1));
-                for (int i = w; i < P.nchunk; i += NL) { wait_chunk(i); fetch(i); }
+                if (HI2LO && pipe && lane == 0 && r + 1 < G.npass) publish_progress(L.prog + chain.prog0 + r, -(P.emax + 1));
+                for (int i = 0; i < P.nchunk; ++i) { wait_chunk(i); fetch(i); }
                 n0 += P.nchunk;
             }
         }
