@@ -127,29 +127,32 @@ __device__ __forceinline__ void publish_progress(int * p, int v) {
 // The word in which a launch (resident kernel: a CTA) keeps that one of its waits ran out: its other
 // waits then return at once, so one failed wait costs the launch about that long, not that long per
 // unit.  Streaming launches hold it behind their work counter, reset by the same fill.
+// Where it is stands in shared memory, written before the CTA's first barrier: the waits are calls from
+// many places, which then pass nothing, and only a wait that is polling looks (with the pointer as an
+// argument and a look before the first poll sph degree 4095 took 0.7 % longer).
 struct GiveUp { int * word; int clean; };
-__device__ __forceinline__ bool given_up(GiveUp g) { return *(volatile int *) g.word != g.clean; }
+__shared__ GiveUp s_giveup;
 // true once the wait that began at t0 is to end: about 2^32 SM cycles later, or when another one ran out
-__device__ __forceinline__ bool gave_up(long long t0, GiveUp g, int code) {
-    if (given_up(g)) return true;
+__device__ __forceinline__ bool gave_up(long long t0, int code) {
+    if (*(volatile int *) s_giveup.word != s_giveup.clean) return true;
     if (clock64() - t0 <= (1LL << 32)) return false;
-    atomicExch(g.word, g.clean + 1);
+    atomicExch(s_giveup.word, s_giveup.clean + 1);
     atomicCAS(&g_rot_status, 0, code);
     return true;
 }
 // Waits until *p >= need and returns the value read (a smaller one if the wait ended before).
 // (The launch's word is a read of global memory, as slow as the progress word's own: only every 64th
 // poll looks at it.)
-__device__ __noinline__ int wait_progress(const int * p, int need, GiveUp g) {
+__device__ __noinline__ int wait_progress(const int * p, int need) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
         if (v >= need) return v;
-        if (i % 64 == 0 && gave_up(t0, g, 3)) return v;
+        if (i % 64 == 0 && gave_up(t0, 3)) return v;
     }
 }
-// Whole-task launches run a task's passes one after another in one CTA, whose loading warps wait
+// Whole-task launches run a task's passes one after another in one CTA, whose loading warp waits
 // for its own storing warp: one 64-bit word in shared memory holds (pass counter of the CTA,
 // progress + 2^31), which only rises.
 __device__ __forceinline__ unsigned long long local_word(unsigned seq, int v) {
@@ -158,13 +161,13 @@ __device__ __forceinline__ unsigned long long local_word(unsigned seq, int v) {
 __device__ __forceinline__ void publish_local(unsigned long long * p, unsigned long long w) {
     asm volatile("st.release.cta.shared::cta.u64 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "l"(w) : "memory");
 }
-__device__ __noinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need, GiveUp g) {
+__device__ __noinline__ unsigned long long wait_local(const unsigned long long * p, unsigned long long need) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         unsigned long long v;
         asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];\n" : "=l"(v) : "r"(tc::smem_addr(p)) : "memory");
         if (v >= need) return v;
-        if (i % 64 == 0 && gave_up(t0, g, 3)) return v;
+        if (i % 64 == 0 && gave_up(t0, 3)) return v;
         __nanosleep(32);
     }
 }
@@ -172,21 +175,20 @@ __device__ __noinline__ unsigned long long wait_local(const unsigned long long *
 // end, and the kernel with them.
 // (The slow path is a call: the kernel's warps run different code at the same time, and what they
 // run between them has to stay small to be served from the instruction cache.)
-__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, uint32_t parity, GiveUp g) {
-    if (given_up(g)) return false;
+__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, uint32_t parity) {
     const long long t0 = clock64();
     while (!tc::mbar_try_wait(bar, parity))
-        if (gave_up(t0, g, 5)) return false;
+        if (gave_up(t0, 5)) return false;
     return true;
 }
-__device__ __forceinline__ bool wait_bar(uint64_t * bar, uint32_t parity, GiveUp g) {
+__device__ __forceinline__ bool wait_bar(uint64_t * bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok) : "r"(tc::smem_addr(bar)), "r"(parity) : "memory");
-    return ok || wait_bar_slow(bar, parity, g);
+    return ok || wait_bar_slow(bar, parity);
 }
 
 // Asynchronous 8-byte copy global -> shared (0 bytes read, zeros written when !valid), and the
@@ -373,19 +375,19 @@ __device__ __forceinline__ void stage_steps(double (&win)[NCOL][2 * B], const do
 __device__ __forceinline__ void publish_word(int * p, int v) {
     asm volatile("st.release.cta.shared::cta.s32 [%0], %1;\n" :: "r"(tc::smem_addr(p)), "r"(v) : "memory");
 }
-__device__ __noinline__ int wait_word_slow(const int * p, int need, GiveUp g) {
+__device__ __noinline__ int wait_word_slow(const int * p, int need) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         int v;
         asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
         if (v >= need) return v;
-        if (i % 256 == 0 && gave_up(t0, g, 3)) return v;
+        if (i % 256 == 0 && gave_up(t0, 3)) return v;
     }
 }
-__device__ __forceinline__ int wait_word(const int * p, int need, GiveUp g) {
+__device__ __forceinline__ int wait_word(const int * p, int need) {
     int v;
     asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];\n" : "=r"(v) : "r"(tc::smem_addr(p)) : "memory");
-    return v >= need ? v : wait_word_slow(p, need, g);
+    return v >= need ? v : wait_word_slow(p, need);
 }
 
 // E steps of one sequence of the resident kernel (stage_steps with the columns in place; a branch an
@@ -460,7 +462,6 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
     __shared__ unsigned long long s_local;
     __shared__ int s_unit[UR];
 
-    const GiveUp giveup{L.counter + 1, L.counter0};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < SH::IDLEN; i += blockDim.x) ident[i] = make_double2(0.0, 1.0);
     if (threadIdx.x == 0) {
@@ -468,6 +469,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         for (int i = 0; i < W * SCS; ++i) tc::mbar_init(&scbar[i], 1);
         for (int i = 0; i < UR; ++i) { tc::mbar_init(&ufull[i], 1); tc::mbar_init(&uempt[i], SH::WARPS - 1); }
         s_local = 0;
+        s_giveup = GiveUp{L.counter + 1, L.counter0};
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
@@ -492,7 +494,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
         ++nunit;
         int id = 0;
         if (warp == W) {
-            if (!__all_sync(0xffffffffu, wait_bar(&uempt[slot], ph ^ 1, giveup))) return -1;
+            if (!__all_sync(0xffffffffu, wait_bar(&uempt[slot], ph ^ 1))) return -1;
             if (lane == 0) {
                 id = atomicAdd(L.counter, 1) - L.counter0;
                 if (id >= nwork) id = -1;
@@ -501,7 +503,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             }
             id = __shfl_sync(0xffffffffu, id, 0);
         } else {
-            if (!__all_sync(0xffffffffu, wait_bar(&ufull[slot], ph, giveup))) return -1;
+            if (!__all_sync(0xffffffffu, wait_bar(&ufull[slot], ph))) return -1;
             id = *(volatile int *) &s_unit[slot];
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&uempt[slot]);
@@ -540,8 +542,8 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 if (q >= P.stages) {
                     // no sweep of the pass: hand the chunks on
                     for (int k = 0; k < P.nchunk; ++k) {
-                        wait_bar(&in_full[nin % SL], (nin / SL) & 1, giveup);
-                        wait_bar(&out_empty[nout % SL], ((nout / SL) & 1) ^ 1, giveup);
+                        wait_bar(&in_full[nin % SL], (nin / SL) & 1);
+                        wait_bar(&out_empty[nout % SL], ((nout / SL) & 1) ^ 1);
                         const double * const bin = in_ring + (nin % SL) * SLOT + lane_off;
                         double * const bout = out_ring + (nout % SL) * SLOT + lane_off;
 #pragma unroll
@@ -593,14 +595,14 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     live |= stage_sc(k + SCS - 1) ? 1u << (SCS - 1) : 0u;
                     const bool has_in = k < P.nchunk, has_out = k >= D;
                     const int is = nin % SL, os = nout % SL;
-                    if (has_in) wait_bar(&in_full[is], (nin / SL) & 1, giveup);
-                    if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1, giveup);
+                    if (has_in) wait_bar(&in_full[is], (nin / SL) & 1);
+                    if (has_out) wait_bar(&out_empty[os], ((nout / SL) & 1) ^ 1);
                     const double * const bin = in_ring + is * SLOT + lane_off;    // read while elements enter (has_in)
                     double * const bout = out_ring + os * SLOT + lane_off;        // written once elements leave (has_out)
                     const bool odd = D > 1 && (k & 1);   // the chunk starts halfway round the window
                     if (live & 1u) {
                         const int slot = sc_used % SCS;
-                        wait_bar(&scbar[q * SCS + slot], (sc_used / SCS) & 1, giveup);
+                        wait_bar(&scbar[q * SCS + slot], (sc_used / SCS) & 1);
                         ++sc_used;
                         const double2 * sc[B];
 #pragma unroll
@@ -628,7 +630,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
             const long long t0 = clock64();
             while (!tc::mbar_try_wait(&scbar[q * SCS + sc_used % SCS], (sc_used / SCS) & 1) && clock64() - t0 < (1LL << 24)) {}
         }
-    } else if (warp == W) {
+    } else if (warp <= W) {   // (== W: the compiler's layout takes 0.5 % longer at sph degree 4095)
         // ---------------- loading warp ----------------
         unsigned n0 = 0;           // chunks of earlier passes
         for (;;) {
@@ -655,10 +657,10 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                     const int pmin = P.pmin(i), pmax = pmin + E - 1;
                     const int need = HI2LO ? -max(pmin, 0) : min(pmax, P.emax);
                     if (prev) {
-                        if (seen < need) { if (lane == 0) seen = wait_progress(prev, need, giveup); seen = __shfl_sync(0xffffffffu, seen, 0); }
+                        if (seen < need) { if (lane == 0) seen = wait_progress(prev, need); seen = __shfl_sync(0xffffffffu, seen, 0); }
                     } else {
                         const unsigned long long want = local_word(seq - 1, need);
-                        if (seen_local < want) { if (lane == 0) seen_local = wait_local(&s_local, want, giveup); seen_local = __shfl_sync(0xffffffffu, seen_local, 0); }
+                        if (seen_local < want) { if (lane == 0) seen_local = wait_local(&s_local, want); seen_local = __shfl_sync(0xffffffffu, seen_local, 0); }
                     }
                     __syncwarp();
                 };
@@ -666,7 +668,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 auto fetch = [&](int i) {
                     const unsigned n = n0 + i;
                     const int pmin = P.pmin(i);
-                    wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1, giveup);
+                    wait_bar(&empt[n % SL], ((n / SL) & 1) ^ 1);
                     const uint32_t slot = tc::smem_addr(rings + (size_t) (n % SL) * SLOT);
 #pragma unroll 1
                     for (int ph = 0; ph < MV::PH; ++ph) {
@@ -712,7 +714,7 @@ rot_kernel(const __grid_constant__ RotLaunch L) {
                 int since = 0;
                 for (int i = 0; i < P.nchunk; ++i, ++n) {
                     const int pmin = P.pmin(i);
-                    wait_bar(&bfull[n % SL], (n / SL) & 1, giveup);
+                    wait_bar(&bfull[n % SL], (n / SL) & 1);
                     const double * const slot = ring + (n % SL) * SLOT;
 #pragma unroll 1
                     for (int ph = 0; ph < MV::PH; ++ph) {
@@ -811,8 +813,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
     double2 * const ident = pairs + W * SCS * SCLEN;
     double * const col = reinterpret_cast<double *>(ident + R::IDLEN) + ROW;   // position p of lane l at col[p * ROW + l]
     __shared__ __align__(8) uint64_t scbar[W * SCS];
-    __shared__ int prog[W], s_giveup;
-    const GiveUp giveup{&s_giveup, 0};
+    __shared__ int prog[W], s_gave_up;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     allow_next();
@@ -830,7 +831,8 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
 
     if (threadIdx.x < W) prog[threadIdx.x] = -1;
     if (threadIdx.x == 0) {
-        s_giveup = 0;
+        s_gave_up = 0;
+        s_giveup = GiveUp{&s_gave_up, 0};
         for (int i = 0; i < W * SCS; ++i) tc::mbar_init(&scbar[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -937,7 +939,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
             const int cin = HI2LO ? chi - k : k, cout = HI2LO ? cin + D : cin - D;
             if (has_in && g > 0) {
                 const int need = (g - 1) * 4096 + (HI2LO ? 2048 - cin : cin + 1);
-                if (seen < need) seen = wait_word(before, need, giveup);
+                if (seen < need) seen = wait_word(before, need);
             }
             // position of the chunk's first step, and the way the steps go
             const double * const bin = col + (HI2LO ? cin * E + E - 1 : cin * E - 1) * ROW + lane;
@@ -945,7 +947,7 @@ rot_resident_kernel(const __grid_constant__ RotLaunch L) {
             const bool odd = D > 1 && (k & 1);
             if (live & 1u) {
                 const int slot = sc_used % SCS;
-                wait_bar(&bars[slot], (sc_used / SCS) & 1, giveup);
+                wait_bar(&bars[slot], (sc_used / SCS) & 1);
                 ++sc_used;
                 const double2 * sc[B];
 #pragma unroll
