@@ -198,13 +198,13 @@ int rotation_status(int value);   // returns the rotation kernels' report word (
 // dimension), or null.  With it, the first launch of a shape times every configuration
 // there and keeps the fastest for the shape (the autotuner; FT_B200_AUTOTUNE=0 turns it off).
 // sched: the task list's schedule (null: no pass pipeline).  prog_call: progress words of the
-// calling execute (prog_cap of them, its work counter kProgLead words before them) for the pass pipeline instead of the schedule's own, so
-// that concurrent calls on one plan do not share them; a queue needing more runs without the
-// pipeline.
+// calling execute (prog_cap of them, its work counter kProgLead words before them) for the pass
+// pipeline instead of the schedule's own, so that concurrent calls on one plan do not share them; a
+// queue needing more runs without the pipeline.
 cudaError_t launch_rotations(int kind, bool hi2lo, const RotLaunch & L, int max_ctas, cudaStream_t st,
                              double * const * dead = nullptr, RotSchedule * sched = nullptr,
                              int * prog_call = nullptr, int prog_cap = 0);
-void set_rotation_config(int cfg);   // 0 .. 3 forces a configuration, -1 chooses per shape
+void set_rotation_config(int cfg);   // shape 0 .. 5 + 8 x pipeline mode 0 .. 2 forces a configuration, -1 chooses per shape
 // (Re)builds RP->d_skew from RP->d_sc (call after every change of d_sc; synchronous)
 bool rotation_plan_skew(ft_rotation_plan * RP);
 

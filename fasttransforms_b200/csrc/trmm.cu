@@ -174,7 +174,7 @@ __device__ __forceinline__ void tri_tile(const GemmClass & C, const int n, const
         double * as = As + stage * ASZ;
         double * bs = Bs + stage * BSZ;
         if (VEC16) {
-            // A: BM*BK doubles = 1024 pairs
+            // A: BM * BK doubles, in pairs
 #pragma unroll
             for (int r = 0; r < (BM * BK / 2) / NTHREADS; ++r) {
                 const int p = r * NTHREADS + tid;

@@ -550,8 +550,12 @@ int ft_b200_profile_read(int family, double * ms, int * launches);
  * heads only, fields, tasks, N, M) times every configuration once on its
  * destination, whose contents are not needed yet, and keeps the fastest for that
  * shape.  That first launch synchronises with the stream, so make it before any
- * stream capture; a capturing stream or an in-place launch uses an untimed rule
- * (resident for short columns, else the pass pipeline).  FT_B200_AUTOTUNE=0
+ * stream capture; a capturing stream or an in-place launch (spin, annulus and
+ * Dunkl-Xu plans, rotation plans, some tri calls) uses an untimed rule (resident
+ * for short columns, else the pass pipeline).  The first in-place launch of a plan
+ * and M that takes the pipeline uploads its queue (an allocation and a synchronous
+ * copy), so make it before any capture too: a capturing stream without the queue
+ * runs whole tasks.  FT_B200_AUTOTUNE=0
  * turns the timing off.  Results are bit-identical for every configuration.
  * Process-wide. */
 void ft_b200_set_rotation_config(int cfg);
